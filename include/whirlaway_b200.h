@@ -272,7 +272,7 @@ wl_status wl_ctx_set_spin_sync(wl_ctx* ctx, int32_t spin);
 
 /* Autotuning of the commitment's launch plans (no reference counterpart; the reference has
  * no GPU kernels). The LDE's stage split and persistent-pass occupancy ("lde", 6 plans), the
- * leaf sponges' rows per block ("leaf", 3 plans) and the Merkle level schedule ("merkle",
+ * leaf sponges' tiles of 128 rows per block ("leaf", 3 plans) and the Merkle level schedule ("merkle",
  * 3 plans) each have plans that write the same result at different speeds. A context that
  * tunes (the default for wl_ctx_create; server workers do not) runs every plan the first time
  * it meets a table shape, timed with CUDA events, and keeps the fastest per device and shape

@@ -289,7 +289,6 @@ __global__ void k_twiddles(uint2* tw, uint32_t w24) {
   }
 }
 
-// Leaf rows per block: 64, 128 (default) or 256, the autotuner's pick (LEAF_PLANS).
 constexpr int TOP_LEVELS = 7;  // the last levels (<= 2^7 digests) run in one block
 constexpr int FLAT_LEVEL_MIN_LOG = 13;  // levels of at least 2^13 digests get their own launch
 
@@ -324,17 +323,16 @@ __device__ __forceinline__ void leaf_chunk(const uint32_t* __restrict__ lde, int
 }
 
 // The tree holds canonical digests: the permutations run in the canonical domain (see
-// p2_permute_fd), the absorbed LDE entries are converted from Montgomery form, and the host
+// p2_permute_tc), the absorbed LDE entries are converted from Montgomery form, and the host
 // converts the root and the opened digests back.
 //
-// Absorbs chunk ch of LDE row `row` into the sponge state st (the chunk overwrites the rate
-// st[0..15]; st[16..23] is the capacity): the Moebius transform over the position bits
-// [log_elem, 7) of the column index makes entry j the sum over i <= j (bitwise on those bits,
-// equal elsewhere) of (-1)^popcount(i ^ j) row[i]. Bits 4..6 select the 16-entry chunk, so
-// chunk ch is the signed sum of the chunks below it, and bits below 4 are transformed inside
-// the chunk. Then the permutation.
-__device__ __forceinline__ void leaf_absorb(const uint32_t* __restrict__ lde, int T, size_t row, int n_cols,
-                                            int log_elem, int ch, const kb::P2ConstsFd<24>& c, uint32_t* st) {
+// The rate words of chunk ch of LDE row `row`, in [1, p] (p for zero): the Moebius transform
+// over the position bits [log_elem, 7) of the column index makes entry j the sum over i <= j
+// (bitwise on those bits, equal elsewhere) of (-1)^popcount(i ^ j) row[i]. Bits 4..6 select the
+// 16-entry chunk, so chunk ch is the signed sum of the chunks below it, and bits below 4 are
+// transformed inside the chunk.
+__device__ __forceinline__ void leaf_rate(const uint32_t* __restrict__ lde, int T, size_t row, int n_cols,
+                                          int log_elem, int ch, uint32_t* st) {
   const int cmask = log_elem <= 4 ? 7 : (7 << (log_elem - 4)) & 7;  // chunk bits in the transform
   leaf_chunk(lde, T, row, n_cols, ch, 0, st);
   const int m = ch & cmask;
@@ -354,64 +352,84 @@ __device__ __forceinline__ void leaf_absorb(const uint32_t* __restrict__ lde, in
     for (int i = 0; i < 16; i++)
       if (!(i & h)) st[i + h] = kb::sub(st[i + h], st[i]);
   }
+  // x 2^-32 = -umulhi(x p^-1, p) (mod p)
 #pragma unroll
-  for (int i = 0; i < 16; i++) st[i] = kb::from_mont(st[i]);
-  kb::p2_permute_fd<24>(st, c);
+  for (int i = 0; i < 16; i++) st[i] = kb::P - __umulhi(st[i] * kb::PINV, kb::P);
 }
 
-// Leaf digests (level 0 of the tree), one row per thread: each thread hashes one row of 128
-// entries with the width-24 sponge (16 entries per absorption, 8 absorptions). Rows are read
-// straight from the tile-major LDE (no shared-memory staging, so occupancy is bounded by
-// registers).
-template <int ROWS>
-__global__ void __launch_bounds__(ROWS) k_leaf_hash(const uint32_t* __restrict__ lde, int T, int n_cols,
-                                                    int log_elem, const __grid_constant__ kb::P2ConstsFd<24> c,
-                                                    uint32_t* __restrict__ tree) {
-  const size_t row0 = size_t(blockIdx.x) * ROWS;
+// Leaf digests (level 0 of the tree): a tile of 128 rows at a time, one row per thread, each
+// hashed with the width-24 sponge (16 entries per absorption, 8 absorptions; only the 8 words
+// that an absorption hands on are formed). Rows are read straight from the tile-major LDE.
+// Threads past the last row work on it again without writing, since the whole block takes part
+// in the permutation's matrix products.
+__global__ void __launch_bounds__(kb::TC_ROWS, 4)
+    k_leaf_hash(const uint32_t* __restrict__ lde, int T, int n_cols, int log_elem,
+                const __grid_constant__ kb::P2ConstsTc<24> c, int tiles, uint32_t* __restrict__ tree,
+                unsigned* __restrict__ timeouts) {
+  extern __shared__ __align__(16) char leaf_smem[];
+  kb::P2TcShared<24>& sh = *reinterpret_cast<kb::P2TcShared<24>*>(leaf_smem);
+  kb::p2_tc_begin<24>(sh);
   const size_t rows = size_t(1) << T;
-  const int nrows = (rows - row0) < size_t(ROWS) ? int(rows - row0) : ROWS;
-  const int t = threadIdx.x;
-  uint32_t st[24];
-  if (t < nrows) {
-    const size_t row = row0 + t;
-#pragma unroll
-    for (int i = 0; i < 24; i++) st[i] = 0;
+  uint32_t parity = 0;
 #pragma unroll 1
-    for (int ch = 0; ch < 8; ch++) leaf_absorb(lde, T, row, n_cols, log_elem, ch, c, st);
-    uint4* o = reinterpret_cast<uint4*>(tree + (row0 + t) * 8);
-    o[0] = make_uint4(st[0], st[1], st[2], st[3]);
-    o[1] = make_uint4(st[4], st[5], st[6], st[7]);
+  for (int i = 0; i < tiles; i++) {
+    const size_t t = (size_t(blockIdx.x) * tiles + i) * kb::TC_ROWS + threadIdx.x;
+    const size_t row = t < rows ? t : rows - 1;
+    uint32_t st[24], o[8];
+#pragma unroll
+    for (int j = 16; j < 24; j++) st[j] = 0;
+#pragma unroll 1
+    for (int ch = 0; ch < 8; ch++) {
+      leaf_rate(lde, T, row, n_cols, log_elem, ch, st);
+      kb::p2_permute_tc<24>(st, c, sh, parity, ch == 7, o);
+#pragma unroll
+      for (int j = 0; j < 8; j++) st[16 + j] = kb::umin(o[j], o[j] - kb::P);
+    }
+    if (t < rows) {
+      uint4* out = reinterpret_cast<uint4*>(tree + row * 8);
+      out[0] = make_uint4(st[16], st[17], st[18], st[19]);
+      out[1] = make_uint4(st[20], st[21], st[22], st[23]);
+    }
   }
+  kb::p2_tc_end<24>(sh, timeouts);
 }
 
 // One absorption (chunk ch) for every row, the capacity carried between launches in cap
 // (8 words per row): the sponge of k_leaf_hash split by chunk, so that chunk ch can be hashed
 // as soon as the LDE tiles it reads exist. The last chunk writes the digests.
-template <int ROWS>
-__global__ void __launch_bounds__(ROWS) k_leaf_absorb(const uint32_t* __restrict__ lde, int T, int n_cols,
-                                                      int log_elem, const __grid_constant__ kb::P2ConstsFd<24> c,
-                                                      int ch, uint32_t* __restrict__ cap,
-                                                      uint32_t* __restrict__ tree) {
-  const size_t row = size_t(blockIdx.x) * ROWS + threadIdx.x;
-  if (row >= (size_t(1) << T)) return;
-  uint32_t st[24];
-  if (ch == 0) {
+__global__ void __launch_bounds__(kb::TC_ROWS, 4)
+    k_leaf_absorb(const uint32_t* __restrict__ lde, int T, int n_cols, int log_elem,
+                  const __grid_constant__ kb::P2ConstsTc<24> c, int tiles, int ch, uint32_t* __restrict__ cap,
+                  uint32_t* __restrict__ tree, unsigned* __restrict__ timeouts) {
+  extern __shared__ __align__(16) char leaf_smem[];
+  kb::P2TcShared<24>& sh = *reinterpret_cast<kb::P2TcShared<24>*>(leaf_smem);
+  kb::p2_tc_begin<24>(sh);
+  const size_t rows = size_t(1) << T;
+  uint32_t parity = 0;
+#pragma unroll 1
+  for (int i = 0; i < tiles; i++) {
+    const size_t t = (size_t(blockIdx.x) * tiles + i) * kb::TC_ROWS + threadIdx.x;
+    const size_t row = t < rows ? t : rows - 1;
+    uint32_t st[24], o[8];
+    if (ch == 0 || t >= rows) {
 #pragma unroll
-    for (int i = 16; i < 24; i++) st[i] = 0;
-  } else {
-    const uint4* in = reinterpret_cast<const uint4*>(cap + row * 8);
-    const uint4 a = in[0], b = in[1];
-    st[16] = a.x, st[17] = a.y, st[18] = a.z, st[19] = a.w, st[20] = b.x, st[21] = b.y, st[22] = b.z, st[23] = b.w;
+      for (int j = 16; j < 24; j++) st[j] = 0;
+    } else {
+      const uint4* in = reinterpret_cast<const uint4*>(cap + row * 8);
+      const uint4 a = in[0], b = in[1];
+      st[16] = a.x, st[17] = a.y, st[18] = a.z, st[19] = a.w, st[20] = b.x, st[21] = b.y, st[22] = b.z, st[23] = b.w;
+    }
+    leaf_rate(lde, T, row, n_cols, log_elem, ch, st);
+    kb::p2_permute_tc<24>(st, c, sh, parity, ch == 7, o);
+#pragma unroll
+    for (int j = 0; j < 8; j++) o[j] = kb::umin(o[j], o[j] - kb::P);
+    if (t < rows) {
+      uint4* out = reinterpret_cast<uint4*>(ch == 7 ? tree + row * 8 : cap + row * 8);
+      out[0] = make_uint4(o[0], o[1], o[2], o[3]);
+      out[1] = make_uint4(o[4], o[5], o[6], o[7]);
+    }
   }
-  leaf_absorb(lde, T, row, n_cols, log_elem, ch, c, st);
-  uint4* o = reinterpret_cast<uint4*>(ch == 7 ? tree + row * 8 : cap + row * 8);
-  if (ch == 7) {
-    o[0] = make_uint4(st[0], st[1], st[2], st[3]);
-    o[1] = make_uint4(st[4], st[5], st[6], st[7]);
-  } else {
-    o[0] = make_uint4(st[16], st[17], st[18], st[19]);
-    o[1] = make_uint4(st[20], st[21], st[22], st[23]);
-  }
+  kb::p2_tc_end<24>(sh, timeouts);
 }
 
 // Level l of the tree from level l - 1, one 2-to-1 compression per thread.
@@ -725,39 +743,51 @@ void launch_lde(const LdeSource& in, uint32_t* out, const uint2* tw, cudaStream_
   }
 }
 
-void launch_merkle_tree(const uint32_t* lde, size_t rows, int n_cols, int elem, const kb::P24Consts& p24,
-                        const kb::P16Consts& p16, uint32_t* tree, int LL, cudaStream_t s) {
-  const int log_elem = elem == 8 ? 3 : 0;
-  if (rows != (size_t(1) << LL) || n_cols % 8) throw std::runtime_error("Merkle leaves: 2^LL rows, columns in tiles of 8");
-  (void)log_elem;
-  launch_leaf_hash(lde, rows, n_cols, elem, p24, tree, LL, s, LEAF_PLAN_DEFAULT);
-  launch_merkle_levels(tree, LL, p16, s);
+namespace {
+// Opts a leaf kernel into its shared memory (above the default 48 KB), once per device.
+template <class K>
+void leaf_smem_limit(K kernel, size_t bytes) {
+  static std::mutex mu;
+  static std::map<std::pair<int, const void*>, bool> done;
+  int dev = 0;
+  WL_CUDA(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lk(mu);
+  bool& d = done[{dev, reinterpret_cast<const void*>(kernel)}];
+  if (d) return;
+  WL_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
+  d = true;
 }
+// Blocks for `rows` rows at `tiles` tiles of 128 rows a block.
+unsigned leaf_blocks(size_t rows, int tiles) {
+  const size_t per = size_t(tiles) * kb::TC_ROWS;
+  return unsigned((rows + per - 1) / per);
+}
+}  // namespace
 
-void launch_leaf_hash(const uint32_t* lde, size_t rows, int n_cols, int elem, const kb::P24Consts& p24,
-                      uint32_t* tree, int LL, cudaStream_t s, int rows_choice) {
+void launch_leaf_hash(const uint32_t* lde, size_t rows, int n_cols, int elem, const kb::P2ConstsTc<24>& p24,
+                      uint32_t* tree, int LL, unsigned* timeouts, cudaStream_t s, int plan) {
   const int log_elem = elem == 8 ? 3 : 0;
   if (rows != (size_t(1) << LL) || n_cols % 8) throw std::runtime_error("Merkle leaves: 2^LL rows, columns in tiles of 8");
-  const kb::P2ConstsFd<24> p24c = kb::p2_consts_fd(p24);
-  switch (rows_choice) {
-    case 0: k_leaf_hash<64><<<(unsigned)((rows + 63) / 64), 64, 0, s>>>(lde, LL, n_cols, log_elem, p24c, tree); break;
-    case 2: k_leaf_hash<256><<<(unsigned)((rows + 255) / 256), 256, 0, s>>>(lde, LL, n_cols, log_elem, p24c, tree); break;
-    default: k_leaf_hash<128><<<(unsigned)((rows + 127) / 128), 128, 0, s>>>(lde, LL, n_cols, log_elem, p24c, tree); break;
-  }
+  const int tiles = 1 << (plan < 0 || plan >= LEAF_PLANS ? LEAF_PLAN_DEFAULT : plan);
+  constexpr size_t smem = sizeof(kb::P2TcShared<24>);
+  leaf_smem_limit(k_leaf_hash, smem);
+  k_leaf_hash<<<leaf_blocks(rows, tiles), kb::TC_ROWS, smem, s>>>(lde, LL, n_cols, log_elem, p24, tiles, tree, timeouts);
   WL_LAUNCH_CHECK();
 }
 
-void launch_leaf_absorb(const uint32_t* lde, size_t rows, int n_cols, int elem, const kb::P24Consts& p24, int ch,
-                        uint32_t* cap, uint32_t* tree, int LL, cudaStream_t s, int rows_choice) {
+void launch_leaf_absorb(const uint32_t* lde, size_t rows, int n_cols, int elem, const kb::P2ConstsTc<24>& p24, int ch,
+                        uint32_t* cap, uint32_t* tree, int LL, unsigned* timeouts, cudaStream_t s) {
   const int log_elem = elem == 8 ? 3 : 0;
   if (rows != (size_t(1) << LL) || n_cols % 8) throw std::runtime_error("Merkle leaves: 2^LL rows, columns in tiles of 8");
   if (ch < 0 || ch > 7) throw std::invalid_argument("leaf chunk out of range");
-  const kb::P2ConstsFd<24> p24c = kb::p2_consts_fd(p24);
-  switch (rows_choice) {
-    case 0: k_leaf_absorb<64><<<(unsigned)((rows + 63) / 64), 64, 0, s>>>(lde, LL, n_cols, log_elem, p24c, ch, cap, tree); break;
-    case 2: k_leaf_absorb<256><<<(unsigned)((rows + 255) / 256), 256, 0, s>>>(lde, LL, n_cols, log_elem, p24c, ch, cap, tree); break;
-    default: k_leaf_absorb<128><<<(unsigned)((rows + 127) / 128), 128, 0, s>>>(lde, LL, n_cols, log_elem, p24c, ch, cap, tree); break;
-  }
+  // one absorption a launch: up to 8 tiles share a block's copy of the B operands, as long as
+  // four blocks an SM remain
+  const size_t all = (rows + kb::TC_ROWS - 1) / kb::TC_ROWS;
+  const int tiles = int(std::max<size_t>(1, std::min<size_t>(8, all / (4 * size_t(ntt_sm_count())))));
+  constexpr size_t smem = sizeof(kb::P2TcShared<24>);
+  leaf_smem_limit(k_leaf_absorb, smem);
+  k_leaf_absorb<<<leaf_blocks(rows, tiles), kb::TC_ROWS, smem, s>>>(lde, LL, n_cols, log_elem, p24, tiles, ch, cap, tree,
+                                                                    timeouts);
   WL_LAUNCH_CHECK();
 }
 

@@ -8,6 +8,7 @@
 
 #include "air.cuh"
 #include "common.cuh"
+#include "poseidon2_tc.cuh"
 
 namespace wl {
 
@@ -39,25 +40,24 @@ void launch_lde(const LdeSource& in, uint32_t* out, const uint2* twiddles, cudaS
 // floor(w 2^32 / p)) for w = w_{2^t}^x, x < 2^(t-1), at offset 2^(t-1) - 1.
 constexpr size_t TWIDDLE_ENTRIES = (size_t(1) << 24) - 1;
 void launch_twiddles(uint2* tw, cudaStream_t s);
-// Merkle tree over the rows of a tile-major LDE matrix (rows of 128 values, the first
-// `n_cols` stored): leaf digests (each row Moebius-transformed over the bits [log2(elem), 7) of the
-// column index, then PaddingFreeSponge over Poseidon2-24) and 2-to-1 compressions
-// (Poseidon2-16), written level by level into `tree` (level l at digest offset
-// 2^(LL+1) - 2^(LL+1-l), LL = log2(rows)).
-void launch_merkle_tree(const uint32_t* lde, size_t rows, int n_cols, int elem, const kb::P24Consts& p24,
-                        const kb::P16Consts& p16, uint32_t* tree, int LL, cudaStream_t s);
+// Leaf digests (level 0 of the Merkle tree) of the rows of a tile-major LDE matrix (rows of 128
+// values, the first `n_cols` stored): each row Moebius-transformed over the bits
+// [log2(elem), 7) of the column index, then PaddingFreeSponge over Poseidon2-24. The tree
+// holds level l at digest offset 2^(LL+1) - 2^(LL+1-l), LL = log2(rows).
+// plan: the autotuner's pick (leaf tiles of 128 rows per block 1 (default), 2 or 4; below, the
+// level width from which compressions run one per thread 2^11, 2^13 (default) or 2^15).
+// timeouts: a device counter of the tensor-core products' bounded waits that ran out (the
+// caller fails the proof when it is not zero).
+constexpr int LEAF_PLANS = 3, LEAF_PLAN_DEFAULT = 0, MERKLE_PLANS = 3, MERKLE_PLAN_DEFAULT = 1;
+void launch_leaf_hash(const uint32_t* lde, size_t rows, int n_cols, int elem, const kb::P2ConstsTc<24>& p24,
+                      uint32_t* tree, int LL, unsigned* timeouts, cudaStream_t s, int plan = LEAF_PLAN_DEFAULT);
 // The same leaves one absorption at a time: chunk ch (0..7) reads LDE tiles 2ch and 2ch + 1
 // (and, through the Moebius transform, those of the chunks below it); the 8 capacity words of
 // every row are carried in cap (8 * rows words) and chunk 7 writes the digests. Then
 // launch_merkle_levels builds the compressions.
-// rows_choice / plan: the autotuner's pick (leaf rows per block 64, 128 (default) or 256; the
-// level width from which compressions run one per thread 2^11, 2^13 (default) or 2^15).
-constexpr int LEAF_PLANS = 3, LEAF_PLAN_DEFAULT = 1, MERKLE_PLANS = 3, MERKLE_PLAN_DEFAULT = 1;
-void launch_leaf_absorb(const uint32_t* lde, size_t rows, int n_cols, int elem, const kb::P24Consts& p24, int ch,
-                        uint32_t* cap, uint32_t* tree, int LL, cudaStream_t s, int rows_choice = LEAF_PLAN_DEFAULT);
-// Level 0 of the tree (the leaf digests) only.
-void launch_leaf_hash(const uint32_t* lde, size_t rows, int n_cols, int elem, const kb::P24Consts& p24,
-                      uint32_t* tree, int LL, cudaStream_t s, int rows_choice = LEAF_PLAN_DEFAULT);
+void launch_leaf_absorb(const uint32_t* lde, size_t rows, int n_cols, int elem, const kb::P2ConstsTc<24>& p24, int ch,
+                        uint32_t* cap, uint32_t* tree, int LL, unsigned* timeouts, cudaStream_t s);
+// 2-to-1 compressions (Poseidon2-16), level by level.
 void launch_merkle_levels(uint32_t* tree, int LL, const kb::P16Consts& p16, cudaStream_t s,
                           int plan = MERKLE_PLAN_DEFAULT);
 // Gathers rows idx[q] of a tile-major LDE matrix (2^T rows, n_cols <= 128 stored columns) as

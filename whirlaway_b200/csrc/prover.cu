@@ -553,7 +553,7 @@ uint64_t lde_key(const LdeSource& src) {
   return uint64_t(src.L) | uint64_t(src.rho) << 8 | uint64_t(src.n_cols) << 16 | uint64_t(src.elem) << 32;
 }
 
-Commitment commit(Context& ctx, const LdeSource& src, int num_vars, int fold, const kb::P24Consts& p24,
+Commitment commit(Context& ctx, const LdeSource& src, int num_vars, int fold, const kb::P2ConstsTc<24>& p24,
                   const kb::P16Consts& p16, const std::vector<cudaEvent_t>* tile_ready = nullptr) {
   Commitment c;
   c.num_vars = num_vars;
@@ -574,7 +574,6 @@ Commitment commit(Context& ctx, const LdeSource& src, int num_vars, int fold, co
     DBuf cap(sizeof(uint32_t) * 8 * rows, ctx.stream);
     const int ntiles = c.n_cols / 8;
     const int lde_plan = tuned_plan(ctx, TUNE_LDE, lde_key(src));
-    const int leaf_plan = tuned_plan(ctx, TUNE_LEAF, lde_key(src));
     int next = 0;
     for (int ch = 0; ch < 8; ch++) {
       for (; next < std::min(ntiles, 2 * ch + 2); next++) {
@@ -583,8 +582,8 @@ Commitment commit(Context& ctx, const LdeSource& src, int num_vars, int fold, co
         launch_lde(src, c.lde.as<uint32_t>(), ctx.twiddles, ctx.stream, next, next + 1, lde_plan);
       }
       ProfScope _ps(ctx, "merkle_tree");
-      launch_leaf_absorb(c.lde.as<uint32_t>(), rows, c.n_cols, c.elem, p24, ch, cap.as<uint32_t>(), t, LL, ctx.stream,
-                         leaf_plan);
+      launch_leaf_absorb(c.lde.as<uint32_t>(), rows, c.n_cols, c.elem, p24, ch, cap.as<uint32_t>(), t, LL,
+                         ctx.pipe_timeouts, ctx.stream);
     }
     for (size_t e = ntiles; e < tile_ready->size(); e++) WL_CUDA(cudaStreamWaitEvent(ctx.stream, (*tile_ready)[e], 0));
     { ProfScope _ps(ctx, "merkle_tree"); launch_merkle_levels(t, LL, p16, ctx.stream, tuned_plan(ctx, TUNE_MERKLE, LL)); }
@@ -597,7 +596,7 @@ Commitment commit(Context& ctx, const LdeSource& src, int num_vars, int fold, co
     }
     ProfScope _ps(ctx, "merkle_tree");
     tuned(ctx, TUNE_LEAF, lde_key(src), [&](int plan) {
-      launch_leaf_hash(c.lde.as<uint32_t>(), rows, c.n_cols, c.elem, p24, t, LL, ctx.stream, plan);
+      launch_leaf_hash(c.lde.as<uint32_t>(), rows, c.n_cols, c.elem, p24, t, LL, ctx.pipe_timeouts, ctx.stream, plan);
     });
     tuned(ctx, TUNE_MERKLE, LL, [&](int plan) { launch_merkle_levels(t, LL, p16, ctx.stream, plan); });
   }
@@ -1027,7 +1026,8 @@ std::vector<uint32_t> prove_air(Context& ctx, const ProofJob& job, const uint32_
   split_vars(lv, lh_v, ll_v);
   LdeSource src0{wit, t_len, 1, lv, ws.c[0].log_inv_rate, 0};
   src0.n_cols = (int)(((t_len + (size_t(1) << lv) - 1) >> lv) + 7) / 8 * 8;
-  Commitment c0 = commit(ctx, src0, m0, ws.c[0].fold, job.p24, job.p16, tile_ready);
+  const kb::P2ConstsTc<24> p24 = kb::p2_consts_tc(job.p24);
+  Commitment c0 = commit(ctx, src0, m0, ws.c[0].fold, p24, job.p16, tile_ready);
   ts.add_base(c0.root, 8);
   // Commitment OOD: F_0[u] = sum_v T[u, v] eq(pt_v, v), answer = sum_u eq(pt_u, u) F_0[u].
   std::vector<std::vector<ef>> ood_pts;
@@ -1391,7 +1391,7 @@ std::vector<uint32_t> prove_air(Context& ctx, const ProofJob& job, const uint32_
       const WhirRound& cn = ws.c[i + 1];
       ts.phase(("whir_round_" + std::to_string(i + 1)).c_str());
       LdeSource src{g.as<uint32_t>(), size_t(8) << m, 8, m - cn.fold, cn.log_inv_rate, 128};
-      commits.push_back(commit(ctx, src, m, cn.fold, job.p24, job.p16));
+      commits.push_back(commit(ctx, src, m, cn.fold, p24, job.p16));
       const Commitment& cd = commits.back();
       ts.add_base(cd.root, 8);
       std::vector<std::vector<ef>> npts_ef;
@@ -1438,7 +1438,10 @@ std::vector<uint32_t> prove_air(Context& ctx, const ProofJob& job, const uint32_
     // final round
     ts.phase("whir_final");
     std::vector<ef> gf(size_t(1) << m), wf(size_t(1) << m);
-    ctx.to_host_many({{gf.data(), g.as<ef>(), sizeof(ef) << m}, {wf.data(), w.as<ef>(), sizeof(ef) << m}});
+    unsigned timeouts = 0;
+    ctx.to_host_many({{gf.data(), g.as<ef>(), sizeof(ef) << m}, {wf.data(), w.as<ef>(), sizeof(ef) << m},
+                      {&timeouts, ctx.pipe_timeouts, sizeof(unsigned)}});
+    if (timeouts) throw std::runtime_error("Merkle leaves: a bounded wait ran out on the device");
     ts.add_ext(gf.data(), gf.size());
     const WhirRound& cl = ws.c[ws.num_rounds];
     grind(ctx, ts, job.p16, cl.pow_bits);

@@ -5,13 +5,14 @@
 //
 // Warp 0 of the block runs a finish with its values spread over the lanes rather than
 // repeated in one: the challenger's 16-word state has word i in lanes i and i + 16, an
-// extension-field value has coordinate k in lanes k, k + 8, k + 16 and k + 24. A
-// Poseidon2-16 permutation then takes about a quarter of the cycles of the one-thread form
-// (each partial round's state sum is two warp reductions instead of fifteen modular
-// additions and sixteen diagonal products per lane), and an extension-field product about a
-// third (each lane forms one coordinate's eight-term dot product).
+// extension-field value has coordinate k in lanes k, k + 8, k + 16 and k + 24. The challenger's
+// words are canonical while a finish runs (the permutation's S-box works on canonical words;
+// proof words, sums and challenges stay in Montgomery form). An extension-field product takes
+// about a third of the cycles of the one-thread form (each lane forms one coordinate's
+// eight-term dot product).
 #pragma once
 #include "kernels.h"
+#include "poseidon2_warp.cuh"
 
 namespace wl {
 namespace {
@@ -21,14 +22,13 @@ constexpr unsigned FIN_FULL = 0xffffffffu;
 // Shared-memory part of a finish: the permutation's constants and the round's reduced sums.
 // One instance per block (fin_sm), so that the finish code addresses it as shared memory.
 struct FinSmem {
-  uint32_t rc[8][16];                             // full-round constants: rounds 0-3 initial, 4-7 terminal
-  uint32_t ci[kb::P16Consts::RP];                 // partial-round constants
-  uint32_t diag[16];                              // internal-layer diagonal V_i (Montgomery form)
+  kb::P2WarpConsts p16;                           // the permutation's constants
   uint32_t basis[2][4][4], one, two, inv2;        // FinishConsts' interpolation constants
   DevRound st;                                    // the phase state on entry
   ef r, rinv;                                     // eq-factor rounds: the round's eq challenge and inverse
   ef red[4];                                      // the round's sums, reduced over the partial rows
-  ef tmp[FIN_MAX_THREADS / 32];                   // per-warp partial sums of the reduction
+  ef tmp[3 * 512 / 32];                           // per-warp partial sums of the reduction
+  ef chal;                                        // the challenge the finish sampled
 };
 __shared__ FinSmem fin_sm;
 
@@ -45,20 +45,14 @@ __device__ __forceinline__ int fin_lane() { return threadIdx.x & 31; }
 // are independent, so their latencies overlap; warp 0 then reads shared memory only). A block
 // barrier must follow before warp 0 uses fin_sm.
 __device__ __forceinline__ void fin_load(int kind, const FinArgs& a) {
-  constexpr int RP = kb::P16Consts::RP;
   constexpr int NST = int(sizeof(DevRound) / 4);
-  constexpr int A = 128, B = A + RP, C = B + 16, D = C + 32, E = D + NST, F = E + 16;
+  constexpr int D = 32, E = D + NST, F = E + 16;
   const FinishConsts* __restrict__ fc = a.fc;
   const bool eq = kind == FIN_EQSC4 || kind == FIN_EQSC3;
+  kb::p2_warp_load(fin_sm.p16, &fc->p16);
   for (int t = threadIdx.x; t < F; t += blockDim.x) {
-    if (t < A) {
-      fin_sm.rc[t >> 4][t & 15] = (t >> 4) < 4 ? fc->p16.ext_init[t] : fc->p16.ext_term[t - 64];
-    } else if (t < B) {
-      fin_sm.ci[t - A] = fc->p16.internal[t - A];
-    } else if (t < C) {
-      fin_sm.diag[t - B] = kb::p2_diag<16>(t - B);
-    } else if (t < D) {
-      (&fin_sm.basis[0][0][0])[t - C] = (&fc->basis[0][0][0])[t - C];
+    if (t < D) {
+      (&fin_sm.basis[0][0][0])[t] = (&fc->basis[0][0][0])[t];
     } else if (t < E) {
       reinterpret_cast<uint32_t*>(&fin_sm.st)[t - D] = reinterpret_cast<const uint32_t*>(a.st)[t - D];
     } else if (eq) {
@@ -79,19 +73,20 @@ __device__ __forceinline__ void fin_load(int kind, const FinArgs& a) {
 __device__ __forceinline__ FinCh fin_ch_load(const DevChallenger& c) {
   const int l = fin_lane();
   FinCh f;
-  f.st = c.state[l & 15];
-  f.in = c.in[l & 7];
-  f.out = c.out[l & 7];
+  f.st = kb::from_mont(c.state[l & 15]);
+  f.in = kb::from_mont(c.in[l & 7]);
+  f.out = kb::from_mont(c.out[l & 7]);
   f.in_len = c.in_len;
   f.out_len = c.out_len;
   return f;
 }
 __device__ __forceinline__ void fin_ch_store(DevChallenger& c, const FinCh& f) {
   const int l = fin_lane();
-  if (l < 16) c.state[l] = f.st;
+  const uint32_t st = kb::mul(f.st, kb::R2_MOD_P), in = kb::mul(f.in, kb::R2_MOD_P), out = kb::mul(f.out, kb::R2_MOD_P);
+  if (l < 16) c.state[l] = st;
   if (l < 8) {
-    c.in[l] = f.in;
-    c.out[l] = f.out;
+    c.in[l] = in;
+    c.out[l] = out;
   }
   if (l == 0) {
     c.in_len = f.in_len;
@@ -99,57 +94,11 @@ __device__ __forceinline__ void fin_ch_store(DevChallenger& c, const FinCh& f) {
   }
 }
 
-// External layer across the 16 lanes of a half-warp: row i of circ(2, 3, 1, 1) within the
-// 4-word chunk, plus the sum of that position over the four chunks (gathered in one step).
-__device__ __forceinline__ uint32_t fin_m4(uint32_t a, int i) {
-  const int base = i & ~3;
-  const uint32_t b = __shfl_sync(FIN_FULL, a, base | ((i + 1) & 3), 16);
-  const uint32_t c = __shfl_sync(FIN_FULL, a, base | ((i + 2) & 3), 16);
-  const uint32_t d = __shfl_sync(FIN_FULL, a, base | ((i + 3) & 3), 16);
-  const uint32_t y = kb::add(kb::add(kb::add(a, b), kb::add(c, d)), kb::add(a, kb::dbl(b)));
-  const uint32_t y4 = __shfl_xor_sync(FIN_FULL, y, 4, 16), y8 = __shfl_xor_sync(FIN_FULL, y, 8, 16);
-  const uint32_t y12 = __shfl_xor_sync(FIN_FULL, y, 12, 16);
-  return kb::add(kb::add(kb::add(y, y4), kb::add(y8, y12)), y);
-}
-
-// Poseidon2-16 (Montgomery form; the values of kb::p2_permute<16>) of the state whose word
-// (lane & 15) is v. Partial rounds: word 0 is carried in every lane (a), the other words in
-// their lanes, kept below 2p between rounds (the diagonal product accepts them and the sum
-// below stays in range); the sum of words 1..15 is two warp reductions of their 16-bit halves
-// (each total below 2^20), recombined with 2^31 = 2^24 - 1 (mod p) to below 2p, and does not
-// wait for the S-box. Measured on the B200 in one warp: 5.2 K cycles per permutation, against
-// 23 K with the whole state in every lane and 7.3 K for a form whose partial rounds carry
-// only the S-box chain (more instructions per round than the warp hides).
-__device__ __noinline__ uint32_t fin_perm(uint32_t v) {
-  const int lane = fin_lane(), i = lane & 15;
-  const uint32_t d = fin_sm.diag[i];
-  v = fin_m4(v, i);
-#pragma unroll 1
-  for (int r = 0; r < 4; r++) v = fin_m4(kb::cube(kb::add(v, fin_sm.rc[r][i])), i);
-  uint32_t a = __shfl_sync(FIN_FULL, v, 0);
-  const bool contrib = lane >= 1 && lane < 16;
-#pragma unroll 1
-  for (int r = 0; r < kb::P16Consts::RP; r++) {
-    const uint32_t x0 = kb::cube(kb::add(a, fin_sm.ci[r]));
-    const uint32_t w = contrib ? v : 0u;
-    const uint32_t lo = __reduce_add_sync(FIN_FULL, w & 0xffffu), hi = __reduce_add_sync(FIN_FULL, w >> 16);
-    uint32_t t = ((hi & 0x7fffu) << 16) + (hi >> 15) * 0xffffffu + lo;  // below 2^31 + 2^29 + 2^20 < 2p
-    t = kb::umin(t, t - kb::P);
-    const uint32_t S = kb::add(t, x0);
-    a = kb::sub(S, kb::dbl(x0));  // V_0 = -2
-    v = kb::mul(v, d) + S;        // below 2p
-  }
-  v = i == 0 ? a : kb::umin(v, v - kb::P);
-#pragma unroll 1
-  for (int r = 4; r < 8; r++) v = fin_m4(kb::cube(kb::add(v, fin_sm.rc[r][i])), i);
-  return v;
-}
-
 // Duplexing: the pending inputs overwrite the first in_len words of the state, which is
 // permuted; the rate part becomes the output.
 __device__ __forceinline__ void fin_duplex(FinCh& c) {
   const int lane = fin_lane(), i = lane & 15;
-  c.st = fin_perm((i < 8 && i < c.in_len) ? c.in : c.st);
+  c.st = kb::p2_warp_permute((i < 8 && i < c.in_len) ? c.in : c.st, fin_sm.p16);
   c.out = __shfl_sync(FIN_FULL, c.st, lane & 7);
   c.in_len = 0;
   c.out_len = 8;
@@ -162,6 +111,7 @@ __device__ __forceinline__ void fin_duplex(FinCh& c) {
 __device__ __forceinline__ void fin_observe_ext(FinCh& c, uint32_t x, uint32_t* __restrict__ proof, uint32_t plen) {
   const int lane = fin_lane(), k = lane & 7;
   if (lane < 8) proof[plen + lane] = x;
+  x = kb::from_mont(x);
   const int L = c.in_len;
   const uint32_t first = __shfl_sync(FIN_FULL, x, (k - L) & 7);  // lane k >= L: word k - L
   c.in = k >= L ? first : c.in;
@@ -181,15 +131,16 @@ __device__ __forceinline__ uint32_t fin_sample_ext(FinCh& c) {
   const int k = fin_lane() & 7;
   if (c.in_len || !c.out_len) fin_duplex(c);
   const int O = c.out_len;
-  const uint32_t a = __shfl_sync(FIN_FULL, c.out, (O - 1 - k) & 7);  // sample k < O: out[O - 1 - k]
+  uint32_t a = __shfl_sync(FIN_FULL, c.out, (O - 1 - k) & 7);  // sample k < O: out[O - 1 - k]
   if (O == 8) {
     c.out_len = 0;
-    return a;
+  } else {
+    fin_duplex(c);  // the output ran out after O samples
+    const uint32_t b = __shfl_sync(FIN_FULL, c.out, (7 - (k - O)) & 7);  // sample k >= O: out[7 - (k - O)]
+    c.out_len = O;
+    a = k < O ? a : b;
   }
-  fin_duplex(c);  // the output ran out after O samples
-  const uint32_t b = __shfl_sync(FIN_FULL, c.out, (7 - (k - O)) & 7);  // sample k >= O: out[7 - (k - O)]
-  c.out_len = O;
-  return k < O ? a : b;
+  return kb::mul(a, kb::R2_MOD_P);
 }
 
 // Extension-field product in F[X]/(X^8 - 3), coordinate (lane & 7) of a * b within each group
@@ -250,9 +201,9 @@ __device__ void fin_reduce_rows(const ef* __restrict__ partial, int nb, int nsum
   }
 }
 
-// The round's finish proper (warp 0, every lane). The state st (challenger, claim, eq weight,
-// proof length, round) is read from and written back to a.st; the round polynomial goes to
-// a.proof, the challenge to a.ch_out[round].
+// The round's finish proper (warp 0, every lane). The state (challenger, claim, eq weight, proof
+// length, round) is read from and written back to fin_sm.st (fin_commit copies it to a.st); the
+// round polynomial goes to a.proof, the challenge to a.ch_out[round] and fin_sm.chal.
 //
 // Round of a sumcheck with an eq factor (the AIR zerocheck's rounds >= 1: NPTS = 4; the
 // a*b - c zerocheck: NPTS = 3): the sums are at z = 0, 2, .., NPTS - 1, weighted by the eq
@@ -263,7 +214,7 @@ __device__ void fin_reduce_rows(const ef* __restrict__ partial, int nb, int nsum
 template <int NPTS>
 __device__ __noinline__ void fin_round_eqsc(const FinArgs& a) {
   const int lane = fin_lane();
-  DevRound* stp = a.st;
+  DevRound* stp = &fin_sm.st;
   const int round = fin_sm.st.round;
   uint32_t plen = fin_sm.st.proof_len;
   FinCh c = fin_ch_load(fin_sm.st.ch);
@@ -306,6 +257,7 @@ __device__ __noinline__ void fin_round_eqsc(const FinArgs& a) {
     stp->sum.c[lane] = s;
     stp->mmf.c[lane] = m2;
     a.ch_out[round].c[lane] = ch;
+    fin_sm.chal.c[lane] = ch;
   }
   if (lane == 0) {
     stp->proof_len = plen;
@@ -317,7 +269,7 @@ __device__ __noinline__ void fin_round_eqsc(const FinArgs& a) {
 // claim; the round polynomial (3 coefficients) interpolates 0, 1, 2.
 __device__ __noinline__ void fin_round_prod(const FinArgs& a) {
   const int lane = fin_lane();
-  DevRound* stp = a.st;
+  DevRound* stp = &fin_sm.st;
   const int round = fin_sm.st.round;
   uint32_t plen = fin_sm.st.proof_len;
   FinCh c = fin_ch_load(fin_sm.st.ch);
@@ -340,6 +292,7 @@ __device__ __noinline__ void fin_round_prod(const FinArgs& a) {
   if (lane < 8) {
     stp->sum.c[lane] = s;
     a.ch_out[round].c[lane] = ch;
+    fin_sm.chal.c[lane] = ch;
   }
   if (lane == 0) {
     stp->proof_len = plen;
@@ -352,7 +305,7 @@ __device__ __noinline__ void fin_round_prod(const FinArgs& a) {
 // h(r) = h0 (r-1)(r-2)/2 - h1 r (r-2) + h2 r (r-1)/2.
 __device__ __noinline__ void fin_round_whir(const FinArgs& a) {
   const int lane = fin_lane();
-  DevRound* stp = a.st;
+  DevRound* stp = &fin_sm.st;
   const int round = fin_sm.st.round;
   uint32_t plen = fin_sm.st.proof_len;
   FinCh c = fin_ch_load(fin_sm.st.ch);
@@ -374,6 +327,7 @@ __device__ __noinline__ void fin_round_whir(const FinArgs& a) {
   if (lane < 8) {
     stp->sum.c[lane] = s;
     a.ch_out[round].c[lane] = r;
+    fin_sm.chal.c[lane] = r;
   }
   if (lane == 0) {
     stp->proof_len = plen;
@@ -395,6 +349,16 @@ __device__ __forceinline__ void fin_round(int kind, const FinArgs& a) {
     fin_round_whir(a);
 }
 
+// The phase state back to device memory, with the block count cleared for the next kernel (warp
+// 0, after its last finish).
+__device__ __forceinline__ void fin_commit(const FinArgs& a) {
+  __syncwarp();
+  if (fin_lane() == 0) fin_sm.st.arrived = 0;
+  __syncwarp();
+  for (int t = fin_lane(); t < int(sizeof(DevRound) / 4); t += 32)
+    reinterpret_cast<uint32_t*>(a.st)[t] = reinterpret_cast<const uint32_t*>(&fin_sm.st)[t];
+}
+
 // Epilogue of a kernel whose blocks each wrote one row of `nsum` partial sums (thread 0 of the
 // block, before the call): the block that arrives last reduces all gridDim.x rows and finishes
 // the round. Every thread of every block calls it, after its own stores.
@@ -413,7 +377,7 @@ __device__ __forceinline__ void fin_last_block(int kind, const FinArgs& a, const
   __syncthreads();
   if (threadIdx.x < 32) {
     fin_round(kind, a);
-    if (threadIdx.x == 0) a.st->arrived = 0;  // for the next round's grid
+    fin_commit(a);
   }
 }
 

@@ -9,6 +9,8 @@
 // row and repeat the last (crates/air/src/utils.rs:140-160); neither is materialised.
 // Folded columns are extension-field arrays, column c at cols + c * len.
 #include <algorithm>
+#include <map>
+#include <mutex>
 #include "finish.cuh"
 #include "kernels.h"
 #include "limb_mma.cuh"
@@ -1655,6 +1657,178 @@ __global__ void __launch_bounds__(FE_THREADS) k_abc_fold_eval(const ef* __restri
   if (fin.st) fin_last_block(FIN_EQSC3, fin, partial, 2);
 }
 
+// ------------------------------------------------------------------ the last rounds of a phase
+// Once a phase's tables fit one block's shared memory, all rounds that remain run in one
+// launch: fold at the last challenge, the round's sums, the finish, and again, with the tables
+// folded in place and the phase state kept in shared memory between the rounds. As a launch of
+// its own such a round also cost a kernel boundary, a count of blocks through device memory and
+// the reload of all it needs: 26.6 us a round of the a*b - c sumcheck, 16.4 us here on average
+// over its last nine (9.3 us of each the finish, which is one warp's serial work).
+//
+// Eight lanes form one extension product (fin_mul), here as in the finish. With one thread per
+// product the last rounds have one warp walk through a dozen products in turn, and their code, a
+// few hundred instructions each, does not stay in the instruction cache from round to round:
+// 20.3 us a round. For many points the other form needs half the instructions, so the tail
+// starts at TAIL_MAX_H = 256 points: from 512 on its first round would take longer (23 us a round
+// on average with 256 threads) than the several blocks of the separate launch.
+//
+// h is the number of points of the first round. With fold_in the tables come in at length 4h
+// (the eq table at 2h), to be folded at challenge *ch0; else at length 2h (h), to be evaluated as
+// they are.
+constexpr int TAIL_THREADS = 512;
+constexpr int TAIL_GROUPS = TAIL_THREADS / 8;
+
+// Adds the groups' sums acc[z] (coordinate lane & 7) over the block into fin_sm.red and finishes
+// the round on warp 0. fin_sm.chal is valid for every thread on return.
+template <int NS>
+__device__ __forceinline__ void tail_finish(int kind, const FinArgs& fin, const uint32_t* acc) {
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+  for (int z = 0; z < NS; z++) {
+    uint32_t v = kb::add(acc[z], __shfl_xor_sync(FIN_FULL, acc[z], 8));
+    v = kb::add(v, __shfl_xor_sync(FIN_FULL, v, 16));
+    if (lane < 8) fin_sm.tmp[z * (TAIL_THREADS / 32) + w].c[lane] = v;
+  }
+  __syncthreads();
+  if (w == 0) {
+    const int z = lane >> 3, k = lane & 7;
+    if (z < NS) {
+      uint32_t v = 0;
+#pragma unroll
+      for (int u = 0; u < TAIL_THREADS / 32; u++) v = kb::add(v, fin_sm.tmp[z * (TAIL_THREADS / 32) + u].c[k]);
+      fin_sm.red[z].c[k] = v;
+    }
+    __syncwarp();
+    fin_round(kind, fin);
+  }
+  __syncthreads();
+}
+// Entries [0, n) of each of NT tables (length 2n at src + q sstride) folded at r (coordinate
+// lane & 7) into dst + q dstride; dst may be src, as an entry that is written is read only by the
+// group that writes it.
+template <int NT>
+__device__ __forceinline__ void tail_fold(const ef* src, size_t sstride, ef* dst, size_t dstride, uint32_t n, uint32_t r) {
+  const uint32_t g = threadIdx.x >> 3, k = threadIdx.x & 7;
+#pragma unroll 1
+  for (uint32_t t0 = 0; t0 < NT * n; t0 += TAIL_GROUPS) {
+    const uint32_t t = t0 + g;
+    const bool on = t < NT * n;
+    const uint32_t q = on ? t / n : 0, x = on ? t - q * n : 0;
+    const ef* s = src + q * sstride + x;
+    const uint32_t lo = s[0].c[k], hi = s[n].c[k];
+    const uint32_t v = kb::add(lo, fin_mul(r, kb::sub(hi, lo)));
+    if (on) dst[q * dstride + x].c[k] = v;
+  }
+}
+// The same entries copied.
+template <int NT>
+__device__ __forceinline__ void tail_copy(const ef* src, size_t sstride, ef* dst, size_t dstride, uint32_t n) {
+  for (uint32_t t = threadIdx.x; t < NT * n * 8; t += TAIL_THREADS) {
+    const uint32_t e = t >> 3, q = e / n, x = e - q * n;
+    dst[q * dstride + x].c[t & 7] = src[q * sstride + x].c[t & 7];
+  }
+}
+
+// Product (NS = 2) and WHIR (NS = 3) rounds; the tables folded at the last challenge go to oa, ob.
+template <int NS>
+__global__ void __launch_bounds__(TAIL_THREADS, 1)
+    k_pair_tail(const ef* __restrict__ a, const ef* __restrict__ b, uint32_t h, bool fold_in,
+                const ef* __restrict__ ch0, int rounds, ef* __restrict__ oa, ef* __restrict__ ob, const FinArgs fin) {
+  extern __shared__ __align__(16) char tail_smem[];
+  ef* sa = reinterpret_cast<ef*>(tail_smem);
+  const uint32_t stride = 2 * h, g = threadIdx.x >> 3, k = threadIdx.x & 7;
+  ef* sb = sa + stride;
+  constexpr int kind = NS == 2 ? FIN_PROD : FIN_WHIR;
+  fin_load(kind, fin);
+  if (fold_in) {
+    const uint32_t r = ch0->c[k];
+    tail_fold<1>(a, 0, sa, 0, 2 * h, r);
+    tail_fold<1>(b, 0, sb, 0, 2 * h, r);
+  } else {
+    tail_copy<1>(a, 0, sa, 0, 2 * h);
+    tail_copy<1>(b, 0, sb, 0, 2 * h);
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (int t = 0;; t++, h >>= 1) {
+    uint32_t acc[NS];
+#pragma unroll
+    for (int z = 0; z < NS; z++) acc[z] = 0;
+#pragma unroll 1
+    for (uint32_t x0 = 0; x0 < h; x0 += TAIL_GROUPS) {
+      const uint32_t x = x0 + g;
+      const bool on = x < h;
+      const uint32_t al = on ? sa[x].c[k] : 0u, ah = on ? sa[x + h].c[k] : 0u;
+      const uint32_t bl = on ? sb[x].c[k] : 0u, bh = on ? sb[x + h].c[k] : 0u;
+      acc[0] = kb::add(acc[0], fin_mul(al, bl));
+      if (NS == 3) acc[1] = kb::add(acc[1], fin_mul(ah, bh));
+      acc[NS - 1] = kb::add(acc[NS - 1], fin_mul(kb::sub(kb::dbl(ah), al), kb::sub(kb::dbl(bh), bl)));
+    }
+    tail_finish<NS>(kind, fin, acc);
+    if (t == rounds - 1) break;
+    tail_fold<2>(sa, stride, sa, stride, h, fin_sm.chal.c[k]);
+    __syncthreads();
+  }
+  tail_fold<1>(sa, 0, oa, 0, h, fin_sm.chal.c[k]);
+  tail_fold<1>(sb, 0, ob, 0, h, fin_sm.chal.c[k]);
+  if (threadIdx.x < 32) fin_commit(fin);
+}
+
+// The a*b - c zerocheck's rounds, to the end; the three columns folded at the last challenge go
+// to oc (column q at q times the last round's points).
+__global__ void __launch_bounds__(TAIL_THREADS, 1)
+    k_abc_tail(const ef* __restrict__ cols, const ef* __restrict__ eq_in, uint32_t h, bool fold_in,
+               const ef* __restrict__ ch0, int rounds, ef* __restrict__ oc, const FinArgs fin) {
+  extern __shared__ __align__(16) char tail_smem[];
+  ef* sc = reinterpret_cast<ef*>(tail_smem);
+  const uint32_t stride = 2 * h, g = threadIdx.x >> 3, k = threadIdx.x & 7;
+  ef* se = sc + 3 * stride;
+  fin_load(FIN_EQSC3, fin);
+  if (fold_in) {
+    tail_fold<3>(cols, 2 * stride, sc, stride, stride, ch0->c[k]);
+    for (uint32_t i = threadIdx.x; i < 8 * h; i += TAIL_THREADS)
+      se[i >> 3].c[k] = kb::add(eq_in[i >> 3].c[k], eq_in[(i >> 3) + h].c[k]);
+  } else {
+    tail_copy<3>(cols, stride, sc, stride, stride);
+    tail_copy<1>(eq_in, 0, se, 0, h);
+  }
+  __syncthreads();
+  const int round0 = fin_sm.st.round;
+#pragma unroll 1
+  for (int t = 0;; t++, h >>= 1) {
+    // the eq challenge of a round after the first of the launch
+    if (t && threadIdx.x >= TAIL_THREADS - 16)
+      (threadIdx.x < TAIL_THREADS - 8 ? fin_sm.r : fin_sm.rinv).c[k] =
+          (threadIdx.x < TAIL_THREADS - 8 ? fin.req : fin.rinv)[round0 + t].c[k];
+    uint32_t acc[2] = {0, 0};
+#pragma unroll 1
+    for (uint32_t x0 = 0; x0 < h; x0 += TAIL_GROUPS) {
+      const uint32_t x = x0 + g;
+      const bool on = x < h;
+      uint32_t lo[3], d[3];
+#pragma unroll
+      for (int q = 0; q < 3; q++) {
+        lo[q] = on ? sc[q * stride + x].c[k] : 0u;
+        const uint32_t hi = on ? sc[q * stride + x + h].c[k] : 0u;
+        d[q] = kb::sub(kb::dbl(hi), lo[q]);
+      }
+      const uint32_t e = on ? se[x].c[k] : 0u;
+      acc[0] = kb::add(acc[0], fin_mul(kb::sub(fin_mul(lo[0], lo[1]), lo[2]), e));
+      acc[1] = kb::add(acc[1], fin_mul(kb::sub(fin_mul(d[0], d[1]), d[2]), e));
+    }
+    tail_finish<2>(FIN_EQSC3, fin, acc);
+    if (t == rounds - 1) break;
+    tail_fold<3>(sc, stride, sc, stride, h, fin_sm.chal.c[k]);
+    // the eq table without its leading variable (in place: an entry written is read by the same
+    // thread only)
+    for (uint32_t i = threadIdx.x; i < 4 * h; i += TAIL_THREADS)
+      se[i >> 3].c[k] = kb::add(se[i >> 3].c[k], se[(i >> 3) + h / 2].c[k]);
+    __syncthreads();
+  }
+  tail_fold<3>(sc, stride, oc, h, h, fin_sm.chal.c[k]);
+  if (threadIdx.x < 32) fin_commit(fin);
+}
+
 // ------------------------------------------------------------------ a*b - c
 
 // Round 0 of the a*b - c zerocheck: for every point z of the skipped variables' extension and
@@ -1986,6 +2160,46 @@ void launch_pair_fold_eval(int nsums, const ef* a, const ef* b, const ef* r_dev,
     throw std::invalid_argument("fold-evaluate: 2 or 3 sums");
   WL_LAUNCH_CHECK();
 }
+namespace {
+// Opts a kernel into `bytes` of dynamic shared memory, once per device.
+template <class K>
+void tail_smem_limit(K kernel, size_t bytes) {
+  if (bytes <= 32 * 1024) return;  // beside the static part, within the default 48 KB
+  static std::mutex mu;
+  static std::map<std::pair<int, const void*>, size_t> done;
+  int dev = 0;
+  WL_CUDA(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lk(mu);
+  size_t& d = done[{dev, reinterpret_cast<const void*>(kernel)}];
+  if (d >= bytes) return;
+  WL_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
+  d = bytes;
+}
+}  // namespace
+
+void launch_pair_tail(int nsums, const ef* a, const ef* b, size_t h, const ef* fold_ch, int rounds, ef* oa, ef* ob,
+                      const FinArgs& fin, cudaStream_t s) {
+  if (h < 1 || h > TAIL_MAX_H || rounds < 1 || (h >> (rounds - 1)) < 1) throw std::invalid_argument("sumcheck tail: size");
+  const size_t smem = sizeof(ef) * 4 * h;
+  if (nsums == 2) {
+    tail_smem_limit(k_pair_tail<2>, smem);
+    k_pair_tail<2><<<1, TAIL_THREADS, smem, s>>>(a, b, uint32_t(h), fold_ch != nullptr, fold_ch, rounds, oa, ob, fin);
+  } else {
+    tail_smem_limit(k_pair_tail<3>, smem);
+    k_pair_tail<3><<<1, TAIL_THREADS, smem, s>>>(a, b, uint32_t(h), fold_ch != nullptr, fold_ch, rounds, oa, ob, fin);
+  }
+  WL_LAUNCH_CHECK();
+}
+
+void launch_abc_tail(const ef* cols, const ef* eq, size_t h, const ef* fold_ch, int rounds, ef* oc, const FinArgs& fin,
+                     cudaStream_t s) {
+  if (h < 1 || h > TAIL_MAX_H || rounds < 1 || (h >> (rounds - 1)) < 1) throw std::invalid_argument("sumcheck tail: size");
+  const size_t smem = sizeof(ef) * 7 * h;
+  tail_smem_limit(k_abc_tail, smem);
+  k_abc_tail<<<1, TAIL_THREADS, smem, s>>>(cols, eq, uint32_t(h), fold_ch != nullptr, fold_ch, rounds, oc, fin);
+  WL_LAUNCH_CHECK();
+}
+
 void launch_abc_fold_eval(const ef* cols, const ef* r_dev, const ef* eq_prev, ef* nc, ef* eq_new, size_t h, ef* partial,
                           const FinArgs* fin, cudaStream_t s) {
   const FinArgs f = fin ? *fin : FinArgs{};

@@ -28,7 +28,10 @@ __global__ void __launch_bounds__(FIN_MAX_THREADS, 1) k_round_finish(int kind, c
   fin_load(kind, a);
   fin_reduce_rows(partial, nb, fin_kind_sums_dev(kind));
   __syncthreads();
-  if (threadIdx.x < 32) fin_round(kind, a);
+  if (threadIdx.x < 32) {
+    fin_round(kind, a);
+    fin_commit(a);
+  }
 }
 
 // First level of the reduction of nb interleaved rows of k partial sums (partial[row * k + z]):

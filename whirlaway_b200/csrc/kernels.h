@@ -9,6 +9,7 @@
 #include "air.cuh"
 #include "common.cuh"
 #include "poseidon2_tc.cuh"
+#include "poseidon2_warp.cuh"
 
 namespace wl {
 
@@ -163,6 +164,17 @@ void launch_pair_fold_eval(int nsums, const ef* a, const ef* b, const ef* r_dev,
 void launch_abc_fold_eval(const ef* cols, const ef* r_dev, const ef* eq_prev, ef* nc, ef* eq_new, size_t h, ef* partial,
                           const FinArgs* fin, cudaStream_t s);
 
+// The last `rounds` rounds of a phase in one launch of one block (k_pair_tail, k_abc_tail), the
+// first over h <= TAIL_MAX_H points: with fold_ch the tables have 4h entries (eq: 2h), folded
+// first at that challenge; without, 2h (eq: h), evaluated as they are. Each round is finished as
+// by launch_pair_fold_eval / launch_abc_fold_eval with fin; the tables folded at the last
+// challenge, (h >> (rounds - 1)) entries each, go to oa and ob (oc: three columns).
+constexpr size_t TAIL_MAX_H = 256;
+void launch_pair_tail(int nsums, const ef* a, const ef* b, size_t h, const ef* fold_ch, int rounds, ef* oa, ef* ob,
+                      const FinArgs& fin, cudaStream_t s);
+void launch_abc_tail(const ef* cols, const ef* eq, size_t h, const ef* fold_ch, int rounds, ef* oc, const FinArgs& fin,
+                     cudaStream_t s);
+
 // --------------------------------------------------------------- a*b - c zerocheck
 void launch_abc0_eval(const uint32_t* a, const uint32_t* b, const uint32_t* c, int log_n, int k, int nz,
                       const uint32_t* lw, const ef* eq, ef* partial, cudaStream_t s);
@@ -221,11 +233,11 @@ struct DevRound {
   int32_t round;
   uint32_t arrived;
 };
-// Constants of the round finish: Poseidon2-16 (Montgomery), the Lagrange bases on the nodes
+// Constants of the round finish: Poseidon2-16's, the Lagrange bases on the nodes
 // 0..2 and 0..3 (basis[0][i][k], basis[1][i][k]: coefficient k of basis polynomial i) and the
 // Montgomery forms of 1, 2 and 1/2.
-struct FinishConsts {
-  kb::P16Consts p16;
+struct alignas(16) FinishConsts {
+  kb::P2WarpConsts p16;
   uint32_t basis[2][4][4];
   uint32_t one, two, inv2;
 };

@@ -15,7 +15,8 @@
 //    exits) is shared by all calls and keeps the last call's contents; every buffer the prover
 //    reads is written earlier in the same call. Calls that overlap on the GPU (on different
 //    streams or from different threads) race on it and must be serialised by the caller.
-//  * The call copies to and from the host and waits for its stream between sumcheck rounds.
+//  * The call copies to and from the host and waits for its stream twice (after round 0 and at
+//    the end; the other rounds' transcript runs on the device).
 //    It must not be called from a stream callback or a host function (cudaLaunchHostFunc),
 //    where CUDA calls are not permitted, and it cannot run on a stream that is being captured
 //    into a graph: a capturing stream is rejected with WL_E_INVALID_ARG.
@@ -34,6 +35,10 @@ namespace {
 constexpr size_t NOALLOC_SCRATCH_BYTES = size_t(4) << 20;
 constexpr int NOALLOC_MAX_LOG_N = 14;
 constexpr int MAX_DEVICES = 64;
+// Points from which the rounds run in one launch: its shared memory stays within the default
+// limit, so that no function attribute has to be set (and remembered on the heap).
+constexpr size_t NOALLOC_TAIL_H = 128;
+static_assert(NOALLOC_TAIL_H <= TAIL_MAX_H, "a tail of this size exists");
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NOALLOC_SCRATCH_BYTES];
 
@@ -233,7 +238,6 @@ void prove_abc_fixed(const kb::P16Consts& p16, int n, int k, const uint32_t* a, 
   ef* red = ar.take<ef>(32);
   uint32_t* d_lw = ar.take<uint32_t>(size_t(nz) * nsk);
   ef* d_sel = ar.take<ef>(16);
-  ef* d_ch = ar.take<ef>(1);
   // round 0
   uint32_t lw[16 * 16];
   for (int zi = 0; zi < nz; zi++)
@@ -268,44 +272,68 @@ void prove_abc_fixed(const kb::P16Consts& p16, int n, int k, const uint32_t* a, 
   h2d(d_sel, selr, sizeof(ef) * nsk, st);
   k_abc0_fold_canon<<<dim3((unsigned)((S + 255) / 256), 3), 256, 0, st>>>(a, b, c, n, k, d_sel, cols);
   WL_LAUNCH_CHECK();
-  // rounds >= 1
-  for (int round = 1; round <= n - k; round++) {
-    const int m = n - k - round + 1;
-    const size_t half = size_t(1) << (m - 1);
-    launch_eq_table(d_r + 1 + round, m - 1, eq, st);
-    if (m - 1 == 0) {
-      const ef one = kb::ef_one();
-      h2d(eq, &one, sizeof(ef), st);
-    }
-    const int nb = (int)((half + 31) / 32);
-    launch_abc_eval_ef(cols, m, eq, part, st);
-    launch_reduce_partials(part, nb, 2, red, st);
-    ef s2[2];
-    d2h(s2, red, sizeof(s2), st);
-    const ef& rr = r[round];
-    ef v[3];
-    v[0] = kb::ef_mul(s2[0], mmf);
-    v[2] = kb::ef_mul(s2[1], mmf);
-    v[1] = kb::ef_mul(kb::ef_sub(sum, kb::ef_mul(v[0], kb::ef_sub(kb::ef_one(), rr))), kb::ef_inv(rr));
-    ef p3[3], lin[2], p4[4];
-    interpolate_fixed(v, 3, p3);
-    lin[0] = kb::ef_sub(kb::ef_one(), rr);
-    lin[1] = kb::ef_sub(kb::ef_add(rr, rr), kb::ef_one());
-    poly_mul_fixed(p3, 3, lin, 2, p4);
-    ts.add_ext(p4, 4);
-    ef cc = ts.sample_ext();
-    sum = poly_eval_fixed(p4, 4, cc);
-    mmf = kb::ef_mul(
-        kb::ef_add(kb::ef_mul(kb::ef_sub(kb::ef_one(), rr), kb::ef_sub(kb::ef_one(), cc)), kb::ef_mul(rr, cc)), mmf);
-    h2d(d_ch, &cc, sizeof(ef), st);
-    launch_fold_cols(cols, cols2, 3, half, d_ch, st);
-    ef* t = cols;
-    cols = cols2;
-    cols2 = t;
+  // rounds >= 1: the transcript on the device (finish.cuh), one upload and one read-back
+  const int R = n - k;
+  struct Phase {
+    DevRound st;
+    FinishConsts fc;
+    ef req[NOALLOC_MAX_LOG_N], rinv[NOALLOC_MAX_LOG_N], ch[NOALLOC_MAX_LOG_N], fin[3];
+    uint32_t words[32 * NOALLOC_MAX_LOG_N];
+  } ph;
+  memset(&ph, 0, sizeof(ph));
+  memcpy(ph.st.ch.state, ts.ch.state, sizeof(ph.st.ch.state));
+  memcpy(ph.st.ch.in, ts.ch.in, sizeof(ph.st.ch.in));
+  memcpy(ph.st.ch.out, ts.ch.out, sizeof(ph.st.ch.out));
+  ph.st.ch.in_len = ts.ch.in_len;
+  ph.st.ch.out_len = ts.ch.out_len;
+  ph.st.sum = sum;
+  ph.st.mmf = mmf;
+  ph.fc.p16 = kb::p2_warp_consts(p16);
+  for (int i = 0; i < 3; i++) {
+    ef unit[3] = {kb::ef_zero(), kb::ef_zero(), kb::ef_zero()}, co[3];
+    unit[i] = kb::ef_one();
+    interpolate_fixed(unit, 3, co);
+    for (int j = 0; j < 3; j++) ph.fc.basis[0][i][j] = co[j].c[0];
   }
-  ef fin[3];
-  d2h(fin, cols, sizeof(fin), st);
-  ts.add_ext(fin, 3);
+  ph.fc.one = fm(1);
+  ph.fc.two = fm(2);
+  ph.fc.inv2 = kb::inv_m(fm(2));
+  for (int i = 0; i < R; i++) ph.req[i] = r[1 + i], ph.rinv[i] = kb::ef_inv(r[1 + i]);
+  Phase* d_ph = ar.take<Phase>(1);
+  h2d(d_ph, &ph, sizeof(ph), st);
+  const FinArgs fa{&d_ph->st, d_ph->words, d_ph->ch, &d_ph->fc, d_ph->req, d_ph->rinv};
+  ef *eq1 = eq, *eq2 = ar.take<ef>(S / 4 + 1);
+  launch_eq_table(d_r + 2, R - 1, eq1, st);
+  if (R == 1) {
+    const ef one = kb::ef_one();
+    h2d(eq1, &one, sizeof(ef), st);
+  }
+  for (int round = 1; round <= R; round++) {
+    const int m = R - round + 1;
+    const size_t half = size_t(1) << (m - 1);
+    const ef* ch_prev = round > 1 ? d_ph->ch + (round - 2) : nullptr;
+    if (half <= NOALLOC_TAIL_H) {
+      launch_abc_tail(cols, eq1, half, ch_prev, m, d_ph->fin, fa, st);
+      break;
+    }
+    if (round == 1) {
+      launch_abc_eval_ef(cols, m, eq1, part, st);
+      launch_round_finish(FIN_EQSC3, part, (int)((half + 31) / 32), fa, st);
+    } else {
+      launch_abc_fold_eval(cols, ch_prev, eq1, cols2, eq2, half, part, &fa, st);
+      ef* t = cols;
+      cols = cols2;
+      cols2 = t;
+      t = eq1;
+      eq1 = eq2;
+      eq2 = t;
+    }
+  }
+  d2h(&ph, d_ph, sizeof(ph), st);
+  if (ph.st.round != R || ph.st.proof_len != uint32_t(32 * R)) throw std::runtime_error("device rounds: count mismatch");
+  if (ts.len + size_t(32) * R > ts.cap) throw std::length_error("proof buffer too small");
+  for (int i = 0; i < 32 * R; i++) ts.out[ts.len++] = kb::from_mont(ph.words[i]);
+  ts.add_ext(ph.fin, 3);
 }
 
 }  // namespace

@@ -367,7 +367,7 @@ DBuf scalar_dev(Context& ctx, const ef& v) { return upload(ctx, std::vector<ef>{
 // Constants of the round-finishing kernels for one proof.
 FinishConsts finish_consts(const kb::P16Consts& p16) {
   FinishConsts fc;
-  fc.p16 = p16;
+  fc.p16 = kb::p2_warp_consts(p16);
   for (int b = 0; b < 2; b++) {
     const auto& basis = lagrange_basis_cached(3 + b);
     for (int i = 0; i < 4; i++)
@@ -745,9 +745,22 @@ void whir_sumcheck_dev(Context& ctx, Transcript& ts, DBuf& g, DBuf& w, int& m, e
     // round 0 evaluates the tables as they are (the finish its own kernel); round t >= 1 folds
     // at challenge t - 1, evaluates and finishes in one kernel; the last challenge's fold
     // closes the block
-    for (int t = 0; t < rounds; t++) {
+    // (tables that fit one block run all their rounds in one launch, the last fold included)
+    bool folded = false;
+    for (int t = 0; t < rounds && !folded; t++) {
       const size_t half = size_t(1) << (m - 1 - t);
-      if (t == 0) {
+      if (half <= TAIL_MAX_H) {
+        const size_t left = size_t(1) << (m - rounds);
+        DBuf ng(sizeof(ef) * left, ctx.stream), nw(sizeof(ef) * left, ctx.stream);
+        {
+          ProfScope _ps(ctx, "sumcheck_tail");
+          launch_pair_tail(3, g.as<ef>(), w.as<ef>(), half, t ? ph.chs + (t - 1) : nullptr, rounds - t, ng.as<ef>(),
+                           nw.as<ef>(), ph.fin, ctx.stream);
+        }
+        g = std::move(ng);
+        w = std::move(nw);
+        folded = true;
+      } else if (t == 0) {
         const int nb = whir_sc_blocks(half);
         ef* part = ctx.partials(size_t(3) * nb);
         {
@@ -767,14 +780,14 @@ void whir_sumcheck_dev(Context& ctx, Transcript& ts, DBuf& g, DBuf& w, int& m, e
         w = std::move(nw);
       }
     }
-    {
+    if (!folded) {
       const size_t half = size_t(1) << (m - rounds);
       DBuf ng(sizeof(ef) * half, ctx.stream), nw(sizeof(ef) * half, ctx.stream);
       { ProfScope _ps(ctx, "fold"); launch_fold2_dev(g.as<ef>(), w.as<ef>(), ng.as<ef>(), nw.as<ef>(), half, ph.chs + (rounds - 1), ctx.stream); }
       g = std::move(ng);
       w = std::move(nw);
-      m -= rounds;
     }
+    m -= rounds;
     const std::vector<ef> r = ph.finish(&sigma, nullptr);
     rnd.insert(rnd.end(), r.begin(), r.end());
     return;
@@ -1286,11 +1299,22 @@ std::vector<uint32_t> prove_air(Context& ctx, const ProofJob& job, const uint32_
   if (inner_on_device) {
     DevPhase ph(ctx, ts, n, 24, inner_sum, kb::ef_one(), job.p16);
     // round 0 evaluates A and B as they are (the finish its own kernel); round r >= 1 folds
-    // them at challenge r - 1, evaluates and finishes in one kernel; the last challenge's fold
-    // leaves the final values
-    for (int round = 0; round < n; round++) {
+    // them at challenge r - 1, evaluates and finishes in one kernel
+    bool folded = false;
+    for (int round = 0; round < n && !folded; round++) {
       const size_t half = N >> (round + 1);
-      if (round == 0) {
+      if (half <= TAIL_MAX_H) {
+        // the rounds that remain, and the last fold, in one launch
+        DBuf na(sizeof(ef), st), nbuf(sizeof(ef), st);
+        {
+          ProfScope _ps(ctx, "sumcheck_tail");
+          launch_pair_tail(2, A.as<ef>(), B.as<ef>(), half, round ? ph.chs + (round - 1) : nullptr, n - round,
+                           na.as<ef>(), nbuf.as<ef>(), ph.fin, st);
+        }
+        A = std::move(na);
+        B = std::move(nbuf);
+        folded = true;
+      } else if (round == 0) {
         const int nb = prod_blocks(half);
         ef* part = ctx.partials(size_t(nb) * 2);
         {
@@ -1309,12 +1333,6 @@ std::vector<uint32_t> prove_air(Context& ctx, const ProofJob& job, const uint32_
         A = std::move(na);
         B = std::move(nbuf);
       }
-    }
-    {
-      DBuf na(sizeof(ef), st), nbuf(sizeof(ef), st);
-      { ProfScope _ps(ctx, "fold"); launch_fold2_dev(A.as<ef>(), B.as<ef>(), na.as<ef>(), nbuf.as<ef>(), 1, ph.chs + (n - 1), st); }
-      A = std::move(na);
-      B = std::move(nbuf);
     }
     inner_ch = ph.finish(&inner_sum, nullptr);
   }
@@ -1592,12 +1610,26 @@ std::vector<uint32_t> prove_abc(Context& ctx, const kb::P16Consts& p16, int n, i
     std::vector<cudaEvent_t> ev(n - k + 1);
     for (auto& e : ev) WL_CUDA(cudaEventCreate(&e));
     WL_CUDA(cudaEventRecord(ev[0], st));
+    int tail = 0;  // rounds of the last launch
     // round 1 evaluates the round-0 fold as it is; round r >= 2 folds the columns (and sums the
     // eq table's leading variable out) at challenge r - 1 and evaluates in one pass; the last
-    // challenge's fold leaves the three final values
+    // launch runs all rounds that fit one block and leaves the three final values
     for (int round = 1; round <= n - k; round++) {
       const int m = n - k - round + 1;
       const size_t half = size_t(1) << (m - 1);
+      if (half <= TAIL_MAX_H) {
+        // the rounds that remain, and the last fold, in one launch: they share its time evenly
+        DBuf nc(sizeof(ef) * 3, st);
+        {
+          ProfScope _ps(ctx, "sumcheck_tail");
+          launch_abc_tail(cols.as<ef>(), eqr.as<ef>(), half, round > 1 ? ph.chs + (round - 2) : nullptr, m, nc.as<ef>(),
+                          ph.fin, st);
+        }
+        cols = std::move(nc);
+        tail = m;
+        WL_CUDA(cudaEventRecord(ev[n - k], st));
+        break;
+      }
       if (round == 1) {
         const int nb = (int)((half + 31) / 32);
         ef* part = ctx.partials(size_t(nb) * 2);
@@ -1617,18 +1649,18 @@ std::vector<uint32_t> prove_abc(Context& ctx, const kb::P16Consts& p16, int n, i
         cols = std::move(nc);
         eqr = std::move(eqn);
       }
-      if (round == n - k) {
-        DBuf nc(sizeof(ef) * 3, st);
-        { ProfScope _ps(ctx, "fold"); launch_fold_cols_dev(cols.as<ef>(), nc.as<ef>(), 3, 1, ph.chs + (round - 1), st); }
-        cols = std::move(nc);
-      }
       WL_CUDA(cudaEventRecord(ev[round], st));
     }
     ph.finish(&sum, &mmf);
-    for (int round = 1; round <= n - k; round++) {
+    for (int round = 1; round <= n - k - tail; round++) {
       float ms = 0;
       WL_CUDA(cudaEventElapsedTime(&ms, ev[round - 1], ev[round]));
       if (round_ms) round_ms->push_back(ms);
+    }
+    if (tail) {
+      float ms = 0;
+      WL_CUDA(cudaEventElapsedTime(&ms, ev[n - k - tail], ev[n - k]));
+      for (int i = 0; round_ms && i < tail; i++) round_ms->push_back(ms / float(tail));
     }
     for (auto e : ev) cudaEventDestroy(e);
   }

@@ -506,11 +506,14 @@ wl_status wl_verify_batch_device(wl_ctx* ctx, const wl_air_settings* s, const ui
     {
       wl::ProfScope _ps(c, "check_openings");
       wl::launch_check_openings(words.as<uint32_t>(), dops.as<wl::OpeningCheck>(), int(ops.size()), job.p24, job.p16,
-                                dok.as<uint8_t>(), c.stream);
+                                dok.as<uint8_t>(), c.pipe_timeouts, c.stream);
     }
     std::vector<uint8_t> ok(ops.size());
+    unsigned timeouts = 0;
     WL_CUDA(cudaMemcpyAsync(ok.data(), dok.as<void>(), ok.size(), cudaMemcpyDeviceToHost, c.stream));
+    WL_CUDA(cudaMemcpyAsync(&timeouts, c.pipe_timeouts, sizeof timeouts, cudaMemcpyDeviceToHost, c.stream));
     c.wait_stream();
+    if (timeouts) throw std::runtime_error("Merkle openings: a bounded wait ran out on the device");
     // 3) a failed opening comes before whatever ended the replay: an opening error
     for (size_t j = 0; j < ok.size(); j++)
       if (!ok[j]) statuses[owner[j]] = WL_E_INVALID_PCS_OPENING;

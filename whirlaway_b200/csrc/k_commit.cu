@@ -289,9 +289,6 @@ __global__ void k_twiddles(uint2* tw, uint32_t w24) {
   }
 }
 
-constexpr int TOP_LEVELS = 7;  // the last levels (<= 2^7 digests) run in one block
-constexpr int FLAT_LEVEL_MIN_LOG = 13;  // levels of at least 2^13 digests get their own launch
-
 // Tree layout: level l (2^(LL-l) digests of 8 words) starts at digest offset
 // 2^(LL+1) - 2^(LL+1-l).
 __device__ __forceinline__ size_t tree_off(int LL, int l) {
@@ -432,96 +429,66 @@ __global__ void __launch_bounds__(kb::TC_ROWS, 4)
   kb::p2_tc_end<24>(sh, timeouts);
 }
 
-// Level l of the tree from level l - 1, one 2-to-1 compression per thread.
-__global__ void k_merkle_level(uint32_t* __restrict__ tree, int LL, int l, const __grid_constant__ kb::P2ConstsFd<16> c) {
-  const size_t m = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (m >= (size_t(1) << (LL - l))) return;
-  const uint4* src = reinterpret_cast<const uint4*>(tree + (tree_off(LL, l - 1) + 2 * m) * 8);
-  uint32_t st[16];
+// `levels` levels of the tree above level l0 (level l0 + i has 2^(LL-l0-i) digests), 128
+// compressions at a time on the tensor-core permutation. A block owns 2^(levels-1) tiles of the
+// first of these levels and everything above them, so its later levels read what it wrote. The
+// digests are read with plain loads: they were written in this launch.
+__global__ void __launch_bounds__(kb::TC_ROWS, 4)
+    k_merkle_tiles(uint32_t* tree, int LL, int l0, int levels, const __grid_constant__ kb::P2ConstsTc<16> c,
+                   unsigned* __restrict__ timeouts) {
+  extern __shared__ __align__(16) char merkle_smem[];
+  kb::P2TcShared<16>& sh = *reinterpret_cast<kb::P2TcShared<16>*>(merkle_smem);
+  kb::p2_tc_begin<16>(sh);
+  uint32_t parity = 0;
+#pragma unroll 1
+  for (int i = 1; i <= levels; i++) {
+    const int l = l0 + i, tiles = 1 << (levels - i);
+#pragma unroll 1
+    for (int t = 0; t < tiles; t++) {
+      const size_t m = (size_t(blockIdx.x) * tiles + t) * kb::TC_ROWS + threadIdx.x;
+      const uint4* src = reinterpret_cast<const uint4*>(tree + (tree_off(LL, l - 1) + 2 * m) * 8);
+      uint32_t st[16], o[8];
 #pragma unroll
-  for (int q = 0; q < 4; q++) {
-    const uint4 u = src[q];
-    st[4 * q] = u.x, st[4 * q + 1] = u.y, st[4 * q + 2] = u.z, st[4 * q + 3] = u.w;
-  }
-  kb::p2_permute_fd<16>(st, c);
-  uint4* o = reinterpret_cast<uint4*>(tree + (tree_off(LL, l) + m) * 8);
-  o[0] = make_uint4(st[0], st[1], st[2], st[3]);
-  o[1] = make_uint4(st[4], st[5], st[6], st[7]);
-}
-
-// Poseidon2-16 (canonical domain, canonical constants; the internal diagonal is applied by
-// Montgomery products with its Montgomery form, which is the same linear map) with the state
-// spread over the 16 lanes of a half-warp (lane i holds word i),
-// for the narrow top of a Merkle tree where one thread per permutation leaves the device
-// idle and a single permutation's latency is the cost. Every lane of the warp calls it.
-// External layer: lane i's M4 row is 2 x_i + 3 x_(i+1) + x_(i+2) + x_(i+3) within its chunk
-// of 4, then the sum over the 4 chunks at the same position. Internal layer: lane 0 takes the
-// S-box, the sum is a 16-lane reduction, and each lane scales by its own diagonal entry.
-__device__ __forceinline__ uint32_t mds16_lanes(uint32_t a, int i) {
-  const int base = i & ~3;
-  const uint32_t b = __shfl_sync(0xffffffffu, a, base | ((i + 1) & 3), 16);
-  const uint32_t c = __shfl_sync(0xffffffffu, a, base | ((i + 2) & 3), 16);
-  const uint32_t d = __shfl_sync(0xffffffffu, a, base | ((i + 3) & 3), 16);
-  const uint32_t y = kb::add(kb::add(kb::add(a, b), kb::add(c, d)), kb::add(a, kb::dbl(b)));
-  uint32_t t = kb::add(y, __shfl_xor_sync(0xffffffffu, y, 4, 16));
-  t = kb::add(t, __shfl_xor_sync(0xffffffffu, t, 8, 16));
-  return kb::add(y, t);
-}
-// rc_s: the full-round constants in shared memory (initial rounds at 0, terminal at 64): each
-// lane reads its own word, which from the constant bank would serialise across the warp.
-__device__ __forceinline__ void stage_p16_full_rounds(uint32_t* rc_s, const kb::P16Consts& c) {
-  for (int q = threadIdx.x; q < 128; q += blockDim.x) rc_s[q] = q < 64 ? c.ext_init[q] : c.ext_term[q - 64];
-}
-__device__ uint32_t p2_permute16_lanes(uint32_t v, const uint32_t* rc_s, const kb::P16Consts& c) {
-  const int i = threadIdx.x & 15;
-  const uint32_t dg = kb::p2_diag<16>(i);
-  v = mds16_lanes(v, i);
-#pragma unroll 1
-  for (int r = 0; r < 4; r++) v = mds16_lanes(kb::cube_fq(v + rc_s[r * 16 + i]), i);
-#pragma unroll 1
-  for (int r = 0; r < 20; r++) {
-    if (i == 0) v = kb::cube_fq(v + c.internal[r]);
-    uint32_t sum = v;
+      for (int q = 0; q < 4; q++) {
+        const uint4 u = src[q];
+        st[4 * q] = u.x, st[4 * q + 1] = u.y, st[4 * q + 2] = u.z, st[4 * q + 3] = u.w;
+      }
+      kb::p2_permute_tc<16>(st, c, sh, parity, true, o);
 #pragma unroll
-    for (int d = 8; d > 0; d >>= 1) sum = kb::add(sum, __shfl_xor_sync(0xffffffffu, sum, d, 16));
-    v = kb::add(kb::mul(v, dg), sum);
+      for (int j = 0; j < 8; j++) o[j] = kb::umin(o[j], o[j] - kb::P);
+      uint4* out = reinterpret_cast<uint4*>(tree + (tree_off(LL, l) + m) * 8);
+      out[0] = make_uint4(o[0], o[1], o[2], o[3]);
+      out[1] = make_uint4(o[4], o[5], o[6], o[7]);
+    }
+    __syncthreads();  // the level's digests before the next one reads them
   }
+  kb::p2_tc_end<16>(sh, timeouts);
+}
+
+// `levels` <= SUB_LEVELS levels above level l0, one warp per compression: each block turns
+// 2^levels digests into one, its digests kept in shared memory between the levels. For the
+// narrow part of a tree, where a single permutation's latency is a level's time: a tree of 2^8
+// leaves takes 38 us, against 54 us with 16 lanes per compression (Montgomery diagonal, five
+// shuffles a partial round) and a launch per level.
+constexpr int SUB_LEVELS = 6, SUB_WARPS = 1 << (SUB_LEVELS - 1);
+__global__ void __launch_bounds__(SUB_WARPS * 32)
+    k_merkle_sub(uint32_t* tree, int LL, int l0, int levels, const __grid_constant__ kb::P2WarpConsts c) {
+  __shared__ kb::P2WarpConsts sc;
+  __shared__ uint32_t dg[2][SUB_WARPS * 8];
+  for (int i = threadIdx.x; i < int(sizeof(sc) / 4); i += blockDim.x)
+    reinterpret_cast<uint32_t*>(&sc)[i] = reinterpret_cast<const uint32_t*>(&c)[i];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  __syncthreads();
 #pragma unroll 1
-  for (int r = 0; r < 4; r++) v = mds16_lanes(kb::cube_fq(v + rc_s[64 + r * 16 + i]), i);
-  return v;
-}
-
-// One level l of the tree, 16 lanes per compression (grid covers 16 * 2^(LL-l) threads).
-__global__ void k_merkle_level_lanes(uint32_t* __restrict__ tree, int LL, int l, const __grid_constant__ kb::P16Consts c) {
-  __shared__ uint32_t rc_s[128];
-  stage_p16_full_rounds(rc_s, c);
-  __syncthreads();
-  const size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  const size_t m = t >> 4;
-  const int i = threadIdx.x & 15;
-  const size_t cnt = size_t(1) << (LL - l);
-  const bool act = m < cnt;
-  const size_t warp_first = (t & ~size_t(31)) >> 4;
-  if (warp_first >= cnt) return;  // whole warp idle (uniform per warp)
-  uint32_t v = act ? tree[(tree_off(LL, l - 1) + 2 * m) * 8 + i] : 0u;
-  v = p2_permute16_lanes(v, rc_s, c);
-  if (act && i < 8) tree[(tree_off(LL, l) + m) * 8 + i] = v;
-}
-
-// Levels l0+1 .. LL in one block of 1024 threads (at most 64 compressions per level).
-__global__ void __launch_bounds__(1024) k_merkle_top(uint32_t* __restrict__ tree, int LL, int l0,
-                                                     const __grid_constant__ kb::P16Consts c) {
-  __shared__ uint32_t rc_s[128];
-  stage_p16_full_rounds(rc_s, c);
-  __syncthreads();
-  const int g = threadIdx.x >> 4, i = threadIdx.x & 15;
-  for (int l = l0 + 1; l <= LL; l++) {
-    const int cnt = 1 << (LL - l);
-    if ((threadIdx.x >> 5) * 2 < cnt) {  // warps holding at least one live compression
-      const bool act = g < cnt;
-      uint32_t v = act ? tree[(tree_off(LL, l - 1) + 2 * size_t(g)) * 8 + i] : 0u;
-      v = p2_permute16_lanes(v, rc_s, c);
-      if (act && i < 8) tree[(tree_off(LL, l) + g) * 8 + i] = v;
+  for (int i = 1; i <= levels; i++) {
+    if (w < (1 << (levels - i))) {
+      const size_t m = (size_t(blockIdx.x) << (levels - i)) + w;
+      const uint32_t v = i == 1 ? tree[(tree_off(LL, l0) + 2 * m) * 8 + (lane & 15)] : dg[(i - 1) & 1][w * 16 + (lane & 15)];
+      const uint32_t o = kb::p2_warp_permute(v, sc);
+      if (lane < 8) {
+        tree[(tree_off(LL, l0 + i) + m) * 8 + lane] = o;
+        dg[i & 1][w * 8 + lane] = o;
+      }
     }
     __syncthreads();
   }
@@ -578,30 +545,41 @@ struct GrindState {
 
 // Grinding: the smallest w in [base, base + count), below p, for which the challenger (state
 // st, input buffer in[0..inlen)) samples `bits` zero bits after observing w. The words are
-// canonical, the permutation runs in the canonical domain. Thread t tries base + t, then
-// base + t + G, ... (G threads in the grid) and stops at the first candidate above a witness
+// canonical. A block tries 128 candidates at a time on the tensor-core permutation: base + t,
+// then base + t + G, ... (G threads in the grid), and stops at the first tile above a witness
 // already found: every candidate below the smallest witness is tried, so the result does not
-// depend on the order in which the threads run, and the search ends soon after the first hit
-// instead of covering the whole batch.
-__global__ void __launch_bounds__(256) k_grind(const __grid_constant__ kb::P2ConstsFd<16> c,
-                                               const __grid_constant__ GrindState g, int inlen, int bits,
-                                               uint32_t base, uint32_t count, uint32_t* result) {
-  const uint32_t G = gridDim.x * blockDim.x;
-  const uint32_t mask = (1u << bits) - 1;
-  for (uint32_t off = blockIdx.x * blockDim.x + threadIdx.x; off < count; off += G) {
-    const uint32_t w = base + off;
-    if (w >= kb::P) return;
-    if (*reinterpret_cast<volatile const uint32_t*>(result) < w) return;  // a smaller witness is known
-    uint32_t st[16];
+// depend on the order in which the blocks run, and the search ends soon after the first hit
+// instead of covering the whole batch. At 16 bits 41 us with one candidate per thread and
+// p2_permute_fd in 2^17 threads, 21 us here; the grid is at most the blocks that are resident.
+__global__ void __launch_bounds__(kb::TC_ROWS, 4)
+    k_grind(const __grid_constant__ kb::P2ConstsTc<16> c, const __grid_constant__ GrindState g, int inlen, int bits,
+            uint32_t base, uint32_t count, uint32_t* result, unsigned* __restrict__ timeouts) {
+  extern __shared__ __align__(16) char grind_smem[];
+  kb::P2TcShared<16>& sh = *reinterpret_cast<kb::P2TcShared<16>*>(grind_smem);
+  __shared__ uint32_t known;
+  kb::p2_tc_begin<16>(sh);
+  const uint32_t G = gridDim.x * kb::TC_ROWS, mask = (1u << bits) - 1;
+  uint32_t parity = 0;
+#pragma unroll 1
+  for (uint32_t off = blockIdx.x * kb::TC_ROWS; off < count && base + off < kb::P; off += G) {
+    if (threadIdx.x == 0) known = *reinterpret_cast<volatile const uint32_t*>(result);
+    __syncthreads();
+    if (known < base + off) break;  // a smaller witness is known (the same for the whole block)
+    const uint32_t w = base + off + threadIdx.x;
+    uint32_t st[16], o[8];
 #pragma unroll
     for (int i = 0; i < 16; i++) st[i] = g.st[i];
-    for (int i = 0; i < inlen; i++) st[i] = g.in[i];
 #pragma unroll
     for (int i = 0; i < 8; i++)
-      if (i == inlen) st[i] = w;
-    kb::p2_permute_fd<16>(st, c);
-    if ((st[7] & mask) == 0) atomicMin(result, w);
+      if (i < inlen) st[i] = g.in[i];
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+      if (i == inlen) st[i] = w < kb::P ? w : 0u;
+    kb::p2_permute_tc<16>(st, c, sh, parity, true, o);  // its barriers order the next write of known
+    const uint32_t s = kb::umin(o[7], o[7] - kb::P);
+    if ((s & mask) == 0 && w < kb::P && off + threadIdx.x < count) atomicMin(result, w);
   }
+  kb::p2_tc_end<16>(sh, timeouts);
 }
 
 __global__ void k_to_mont(uint32_t* x, size_t n) {
@@ -791,29 +769,36 @@ void launch_leaf_absorb(const uint32_t* lde, size_t rows, int n_cols, int elem, 
   WL_LAUNCH_CHECK();
 }
 
-void launch_merkle_levels(uint32_t* tree, int LL, const kb::P16Consts& p16, cudaStream_t s, int plan) {
-  const kb::P16Consts p16c = kb::p2_consts_canonical(p16);
-  const kb::P2ConstsFd<16> p16d = kb::p2_consts_fd(p16);
-  // Wide levels: one launch each, one compression per thread. Narrower levels: 16 lanes per
-  // compression. The last levels (at most 128 digests) in one block. The plan sets the width
-  // from which a level runs one compression per thread: 2^11, 2^13 (default) or 2^15 digests.
-  const int flat_min = plan == 0 ? 11 : plan == 2 ? 15 : FLAT_LEVEL_MIN_LOG;
+void launch_merkle_levels(uint32_t* tree, int LL, const kb::P16Consts& p16, unsigned* timeouts, cudaStream_t s,
+                          int plan) {
+  // Wide levels on tiles of 128 compressions: up to three levels a launch while that leaves four
+  // blocks an SM, else one. Below, subtrees of 2^6 digests a block, one warp per compression.
+  // The plan sets the width from which a level runs on tiles: 2^10, 2^12 (default) or 2^14
+  // digests.
+  const int wide = plan == 0 ? 10 : plan == 2 ? 14 : 12;
   int l0 = 0;
-  while (l0 < LL && LL - l0 - 1 >= flat_min) {
-    const size_t cnt = size_t(1) << (LL - l0 - 1);
-    k_merkle_level<<<(unsigned)((cnt + 127) / 128), 128, 0, s>>>(tree, LL, l0 + 1, p16d);
-    WL_LAUNCH_CHECK();
-    l0++;
-  }
-  while (l0 < LL && LL - l0 > TOP_LEVELS) {
-    const size_t threads = size_t(16) << (LL - l0 - 1);
-    k_merkle_level_lanes<<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(tree, LL, l0 + 1, p16c);
-    WL_LAUNCH_CHECK();
-    l0++;
+  if (LL - 1 >= wide) {
+    const kb::P2ConstsTc<16> c = kb::p2_consts_tc(p16);
+    constexpr size_t smem = sizeof(kb::P2TcShared<16>);
+    leaf_smem_limit(k_merkle_tiles, smem);
+    const size_t full = 4 * size_t(ntt_sm_count());
+    while (LL - l0 - 1 >= wide) {
+      const size_t tiles = (size_t(1) << (LL - l0 - 1)) / kb::TC_ROWS;
+      int levels = 1;
+      while (levels < 3 && LL - l0 - 1 - levels >= wide && (tiles >> levels) >= full) levels++;
+      k_merkle_tiles<<<(unsigned)(tiles >> (levels - 1)), kb::TC_ROWS, smem, s>>>(tree, LL, l0, levels, c, timeouts);
+      WL_LAUNCH_CHECK();
+      l0 += levels;
+    }
   }
   if (l0 < LL) {
-    k_merkle_top<<<1, 1024, 0, s>>>(tree, LL, l0, p16c);
-    WL_LAUNCH_CHECK();
+    const kb::P2WarpConsts c = kb::p2_warp_consts(p16);
+    while (l0 < LL) {
+      const int levels = std::min(SUB_LEVELS, LL - l0);
+      k_merkle_sub<<<1u << (LL - l0 - levels), 16 << levels, 0, s>>>(tree, LL, l0, levels, c);
+      WL_LAUNCH_CHECK();
+      l0 += levels;
+    }
   }
 }
 
@@ -832,13 +817,17 @@ void launch_gather_u32(const uint32_t* src, const uint64_t* idx, int width, int 
 }
 
 void launch_grind(const kb::P16Consts& p16, const uint32_t* state16, const uint32_t* inbuf, int inlen, int bits,
-                  uint32_t base, uint32_t count, uint32_t threads, uint32_t* result, cudaStream_t s) {
+                  uint32_t base, uint32_t count, uint32_t threads, uint32_t* result, unsigned* timeouts,
+                  cudaStream_t s) {
   if (bits < 1 || bits > 31 || inlen < 0 || inlen > 7) throw std::invalid_argument("grinding: bits 1..31, inlen 0..7");
   GrindState g;
   for (int i = 0; i < 16; i++) g.st[i] = kb::from_mont(state16[i]);
   for (int i = 0; i < 8; i++) g.in[i] = i < inlen ? kb::from_mont(inbuf[i]) : 0;
-  threads = std::max<uint32_t>(256, std::min<uint32_t>(count, threads));
-  k_grind<<<(threads + 255) / 256, 256, 0, s>>>(kb::p2_consts_fd(p16), g, inlen, bits, base, count, result);
+  const uint32_t blocks = (std::max<uint32_t>(256, std::min<uint32_t>(count, threads)) + kb::TC_ROWS - 1) / kb::TC_ROWS;
+  constexpr size_t smem = sizeof(kb::P2TcShared<16>);
+  leaf_smem_limit(k_grind, smem);
+  k_grind<<<std::min(blocks, 4 * uint32_t(ntt_sm_count())), kb::TC_ROWS, smem, s>>>(kb::p2_consts_tc(p16), g, inlen, bits,
+                                                                                    base, count, result, timeouts);
   WL_LAUNCH_CHECK();
 }
 

@@ -46,7 +46,7 @@ void launch_twiddles(uint2* tw, cudaStream_t s);
 // [log2(elem), 7) of the column index, then PaddingFreeSponge over Poseidon2-24. The tree
 // holds level l at digest offset 2^(LL+1) - 2^(LL+1-l), LL = log2(rows).
 // plan: the autotuner's pick (leaf tiles of 128 rows per block 1 (default), 2 or 4; below, the
-// level width from which compressions run one per thread 2^11, 2^13 (default) or 2^15).
+// level width from which compressions run on tiles of 128, 2^10, 2^12 (default) or 2^14).
 // timeouts: a device counter of the tensor-core products' bounded waits that ran out (the
 // caller fails the proof when it is not zero).
 constexpr int LEAF_PLANS = 3, LEAF_PLAN_DEFAULT = 0, MERKLE_PLANS = 3, MERKLE_PLAN_DEFAULT = 1;
@@ -59,7 +59,7 @@ void launch_leaf_hash(const uint32_t* lde, size_t rows, int n_cols, int elem, co
 void launch_leaf_absorb(const uint32_t* lde, size_t rows, int n_cols, int elem, const kb::P2ConstsTc<24>& p24, int ch,
                         uint32_t* cap, uint32_t* tree, int LL, unsigned* timeouts, cudaStream_t s);
 // 2-to-1 compressions (Poseidon2-16), level by level.
-void launch_merkle_levels(uint32_t* tree, int LL, const kb::P16Consts& p16, cudaStream_t s,
+void launch_merkle_levels(uint32_t* tree, int LL, const kb::P16Consts& p16, unsigned* timeouts, cudaStream_t s,
                           int plan = MERKLE_PLAN_DEFAULT);
 // Gathers rows idx[q] of a tile-major LDE matrix (2^T rows, n_cols <= 128 stored columns) as
 // the leaves hash them: 128 values per row (zero beyond n_cols), Moebius-transformed over the
@@ -77,7 +77,7 @@ void launch_gather_u32(const uint32_t* src, const uint64_t* idx, int width, int 
 // `threads` threads in increasing order with an early stop (any thread count gives the same
 // result).
 void launch_grind(const kb::P16Consts& p16, const uint32_t* state16, const uint32_t* inbuf, int inlen, int bits,
-                  uint32_t base, uint32_t count, uint32_t threads, uint32_t* result, cudaStream_t s);
+                  uint32_t base, uint32_t count, uint32_t threads, uint32_t* result, unsigned* timeouts, cudaStream_t s);
 
 // --------------------------------------------------------------- eq tables / reductions
 void launch_eq_table(const ef* point, int nvars, ef* out, cudaStream_t s);
@@ -295,8 +295,8 @@ struct OpeningCheck {
   int32_t ll;
 };
 // ok[i] = 1 when opening i's row hashes, through its path, to its root (p24, p16: Montgomery
-// constants as in a constants blob).
+// constants as in a constants blob). timeouts as for launch_leaf_hash.
 void launch_check_openings(const uint32_t* words, const OpeningCheck* ops, int n, const kb::P24Consts& p24,
-                           const kb::P16Consts& p16, uint8_t* ok, cudaStream_t s);
+                           const kb::P16Consts& p16, uint8_t* ok, unsigned* timeouts, cudaStream_t s);
 
 }  // namespace wl

@@ -391,11 +391,11 @@ template <int W>
 struct P2TcShared {
   using T = P2TcTab<W>;
   static constexpr int EA = 2 * (T::KS + T::KX) * TC_ROWS;  // 16-byte entries of A
-  uint4 b[T::E1 + T::E2 + T::E3];
-  uint4 a[EA];
   uint64_t bar;
   uint32_t tmem;
   uint32_t dead;  // a bounded wait ran out
+  uint4 b[T::E1 + T::E2 + T::E3];
+  uint4 a[EA];
 };
 template <int W>
 __device__ const P2TcTab<W> g_p2_tc_tab = p2lin::make_tab<W>();
@@ -405,12 +405,20 @@ constexpr long long TC_WAIT_CLOCKS = 4000000000ll;
 
 __device__ __forceinline__ uint32_t tc_smem(const void* p) { return uint32_t(__cvta_generic_to_shared(p)); }
 
-// Loads the B operands, sets the mbarrier up and allocates the tile's accumulators. All threads.
+// Loads the B operands. All threads; ends with a barrier. A block that has begun with one width
+// may go on with the other on the same bytes (the mbarrier and the accumulators stay).
 template <int W>
-__device__ __forceinline__ void p2_tc_begin(P2TcShared<W>& sh) {
+__device__ __forceinline__ void p2_tc_load(P2TcShared<W>& sh) {
   using T = P2TcTab<W>;
   const uint4* src = reinterpret_cast<const uint4*>(g_p2_tc_tab<W>.w);
   for (int i = threadIdx.x; i < T::E1 + T::E2 + T::E3; i += TC_ROWS) sh.b[i] = src[i];
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+}
+// Sets the mbarrier up, allocates the tile's accumulators and loads the B operands.
+template <int W>
+__device__ __forceinline__ void p2_tc_begin(P2TcShared<W>& sh) {
   if (threadIdx.x < 32) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem(&sh.tmem)),
                  "r"(TC_COLS)
@@ -422,9 +430,7 @@ __device__ __forceinline__ void p2_tc_begin(P2TcShared<W>& sh) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem(&sh.bar)) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  p2_tc_load(sh);
 }
 // Frees the accumulators; every thread has passed its last wait. Counts a wait that ran out.
 template <int W>

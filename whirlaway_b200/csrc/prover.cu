@@ -487,7 +487,7 @@ void grind(Context& ctx, Transcript& ts, const kb::P16Consts& p16, int bits) {
     uint32_t init = UINT32_MAX;
     ctx.to_device(res.as<void>(), &init, 4);
     { ProfScope _ps(ctx, "grind"); launch_grind(p16, ts.ch.state, ts.ch.in, ts.ch.in_len, bits, (uint32_t)base, batch, threads, res.as<uint32_t>(),
-                 ctx.stream); }
+                 ctx.pipe_timeouts, ctx.stream); }
     uint32_t r;
     ctx.to_host(&r, res.as<uint32_t>(), 4);
     if (r != UINT32_MAX) {
@@ -586,7 +586,7 @@ Commitment commit(Context& ctx, const LdeSource& src, int num_vars, int fold, co
                          ctx.pipe_timeouts, ctx.stream);
     }
     for (size_t e = ntiles; e < tile_ready->size(); e++) WL_CUDA(cudaStreamWaitEvent(ctx.stream, (*tile_ready)[e], 0));
-    { ProfScope _ps(ctx, "merkle_tree"); launch_merkle_levels(t, LL, p16, ctx.stream, tuned_plan(ctx, TUNE_MERKLE, LL)); }
+    { ProfScope _ps(ctx, "merkle_tree"); launch_merkle_levels(t, LL, p16, ctx.pipe_timeouts, ctx.stream, tuned_plan(ctx, TUNE_MERKLE, LL)); }
   } else {
     {
       ProfScope _ps(ctx, "lde");
@@ -598,7 +598,7 @@ Commitment commit(Context& ctx, const LdeSource& src, int num_vars, int fold, co
     tuned(ctx, TUNE_LEAF, lde_key(src), [&](int plan) {
       launch_leaf_hash(c.lde.as<uint32_t>(), rows, c.n_cols, c.elem, p24, t, LL, ctx.pipe_timeouts, ctx.stream, plan);
     });
-    tuned(ctx, TUNE_MERKLE, LL, [&](int plan) { launch_merkle_levels(t, LL, p16, ctx.stream, plan); });
+    tuned(ctx, TUNE_MERKLE, LL, [&](int plan) { launch_merkle_levels(t, LL, p16, ctx.pipe_timeouts, ctx.stream, plan); });
   }
   ctx.to_host(c.root, t + level_offset(LL, LL) * 8, 32);
   for (uint32_t& w : c.root) w = kb::to_mont(w);  // the tree holds canonical digests

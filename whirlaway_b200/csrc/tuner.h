@@ -1,7 +1,7 @@
 // Autotuner of kernel launch plans. Several kernels of the commitment have launch plans that
 // compute the same result with different shapes: the LDE's split of its stages into passes and
-// the persistent passes' blocks per SM, the leaf sponges' rows per block, and the width from
-// which a Merkle level runs one compression per thread; and the inner sums' staging of the
+// the persistent passes' blocks per SM, the leaf sponges' tiles of rows per block, and the
+// width from which a Merkle level runs on tiles of compressions; and the inner sums' staging of the
 // witness (cp.async per thread, or bulk copies by the TMA engine on an mbarrier pipeline).
 // Which plan is fastest depends on the
 // table's shape (rows, columns, element size). The first time a tuning context meets a shape it

@@ -310,14 +310,17 @@ __global__ void __launch_bounds__(AEQ_WARPS * 32) k_add_eq_terms_f_mma(ef* __res
 }
 
 // w[v] += sum_t coefs[t] * hi_t[v_hi] * lo_t[v_lo]   (extension-field points)
+struct AddEqCoefs {
+  ef c[ADD_EQ_MAX];
+};
 __global__ void k_add_eq_terms_ef(ef* __restrict__ w, int lh, int ll, int npts, const ef* __restrict__ hi,
-                                  const ef* __restrict__ lo, const ef* __restrict__ coefs) {
+                                  const ef* __restrict__ lo, const __grid_constant__ AddEqCoefs coefs) {
   const size_t v = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (v >= (size_t(1) << (lh + ll))) return;
   const size_t vh = v >> ll, vl = v & ((size_t(1) << ll) - 1);
   const size_t nhi = size_t(1) << lh, nlo = size_t(1) << ll;
   ef acc = w[v];
-  for (int t = 0; t < npts; t++) acc = ef_add(acc, ef_mul(ef_mul(coefs[t], hi[t * nhi + vh]), lo[t * nlo + vl]));
+  for (int t = 0; t < npts; t++) acc = ef_add(acc, ef_mul(ef_mul(coefs.c[t], hi[t * nhi + vh]), lo[t * nlo + vl]));
   w[v] = acc;
 }
 
@@ -419,7 +422,10 @@ void launch_add_eq_terms_ef(ef* w, int lh, int ll, int npts, const ef* hi, const
                             cudaStream_t s) {
   if (!npts) return;
   size_t n = size_t(1) << (lh + ll);
-  k_add_eq_terms_ef<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(w, lh, ll, npts, hi, lo, coefs);
+  if (npts > ADD_EQ_MAX) throw std::invalid_argument("add_eq_terms_ef: too many points");
+  AddEqCoefs c{};
+  for (int t = 0; t < npts; t++) c.c[t] = coefs[t];
+  k_add_eq_terms_ef<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(w, lh, ll, npts, hi, lo, c);
   WL_LAUNCH_CHECK();
 }
 int whir_sc_blocks(size_t half) {

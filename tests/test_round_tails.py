@@ -36,3 +36,24 @@ def test_inner_tail_matches_oracle(oracle, wl, ctx, log_n):
     wit = oracle.trace(log_n, consts, inputs)
     ref, _ = oracle.prove(log_n, consts, wit)
     assert np.array_equal(wl.AirTable(ctx, consts, log_n).prove(wit), ref)
+
+
+@pytest.mark.parametrize("log_n,skips", [(5, 1), (12, 2), (14, 3), (13, 4)])
+def test_abc_takes_any_word_for_its_residue(oracle, wl, ctx, log_n, skips):
+    """The device columns are read as they are: words x and x + p are the same value, and the
+    caller's columns are left as they were."""
+    import torch
+    cols = _abc(log_n, 90 + skips)
+    consts, _ = oracle.workload(2)
+    p16 = consts[148:296]
+    ref = oracle.prove_abc(p16, log_n, skips, *cols)
+    for every in (1, 3):
+        shifted = [c.copy() for c in cols]
+        for c in shifted:
+            c[::every] += np.uint32(P)
+        dev = [torch.from_numpy(c.view(np.int32)).cuda() for c in shifted]
+        torch.cuda.synchronize()
+        got, _ = wl.sumcheck_abc_prove(ctx, p16, log_n, skips, *dev, device=True)
+        assert np.array_equal(got, ref)
+        for d, c in zip(dev, shifted):
+            assert np.array_equal(d.cpu().numpy().view(np.uint32), c)

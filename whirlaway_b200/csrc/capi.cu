@@ -345,16 +345,17 @@ static wl_status abc_common(wl_ctx* ctx, const uint32_t* p16c, int32_t log_n, in
   return guarded(ctx, [&] {
     cudaStream_t st = ctx->c->stream;
     const size_t N = size_t(1) << log_n;
-    wl::DBuf d(N * 12, st);
-    uint32_t* da = d.as<uint32_t>();
-    auto kind = device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-    WL_CUDA(cudaMemcpyAsync(da, a, N * 4, kind, st));
-    WL_CUDA(cudaMemcpyAsync(da + N, b, N * 4, kind, st));
-    WL_CUDA(cudaMemcpyAsync(da + 2 * N, c, N * 4, kind, st));
-    wl::launch_to_mont(da, 3 * N, st);
+    wl::DBuf d(device ? 0 : N * 12, st);
+    if (!device) {
+      uint32_t* da = d.as<uint32_t>();
+      WL_CUDA(cudaMemcpyAsync(da, a, N * 4, cudaMemcpyHostToDevice, st));
+      WL_CUDA(cudaMemcpyAsync(da + N, b, N * 4, cudaMemcpyHostToDevice, st));
+      WL_CUDA(cudaMemcpyAsync(da + 2 * N, c, N * 4, cudaMemcpyHostToDevice, st));
+      a = da, b = da + N, c = da + 2 * N;
+    }
     kb::P16Consts p16 = wl::perm_consts_from<16>(p16c);
     std::vector<float> ms;
-    std::vector<uint32_t> pr = wl::prove_abc(*ctx->c, p16, log_n, skips, da, da + N, da + 2 * N, &ms);
+    std::vector<uint32_t> pr = wl::prove_abc(*ctx->c, p16, log_n, skips, a, b, c, &ms);
     if (round_ms) std::copy(ms.begin(), ms.end(), round_ms);
     return emit_proof(ctx, pr, proof_out, proof_len);
   });

@@ -63,10 +63,12 @@ __device__ __forceinline__ void eq_table_block(const ef* __restrict__ pt, int nv
     __syncthreads();
     len = m;
   }
-  if (tid < (1 << nbits)) {
-    const ef h = nhi ? fac[0] : ef_one();
-    out[(xhi << nbits) + tid] = ef_mul(ef_mul(h, A[tid >> nb]), B[tid & ((1 << nb) - 1)]);
+  // the block's factor joins A first: one product per entry
+  if (nhi) {
+    if (tid < (1 << na)) A[tid] = ef_mul(fac[0], A[tid]);
+    __syncthreads();
   }
+  if (tid < (1 << nbits)) out[(xhi << nbits) + tid] = ef_mul(A[tid >> nb], B[tid & ((1 << nb) - 1)]);
 }
 
 __global__ void __launch_bounds__(EQ_THREADS) k_eq_table(const ef* __restrict__ pt, int nvars, ef* __restrict__ out) {
@@ -1849,49 +1851,55 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1)
 // thread: each value is read once (a, b, c and eq(x) coalesced), the points' products stay in
 // registers, and each thread keeps nz extension accumulators that one block reduction sums at
 // the end (one partial per block and point).
+// The inputs are the caller's canonical words, read as they are: lw and sel come multiplied by
+// 2^32 once more than Montgomery form, which makes the weighted sums Montgomery values (a pass
+// that copied and converted the three columns took 0.13 ms of a 2^24 proof). Any 32-bit word is
+// taken for its residue.
+__device__ __forceinline__ uint32_t abc_in(uint32_t x) {
+  x = kb::umin(x, x - P);
+  return kb::umin(x, x - P);  // 2^32 < 3 p
+}
 constexpr int ABC_X = 32;
 constexpr int ABC0_THREADS = 256;
 constexpr int ABC0_MAX_Z = 7;  // 2 (2^k - 1) - 2^k + 1 points for k <= 3
+template <int K>
 __global__ void __launch_bounds__(ABC0_THREADS, 2) k_abc0_eval(const uint32_t* __restrict__ a,
                                                            const uint32_t* __restrict__ b,
-                                                           const uint32_t* __restrict__ c, int log_n, int k, int nz,
+                                                           const uint32_t* __restrict__ c, size_t S,
                                                            const uint32_t* __restrict__ lw,
                                                            const ef* __restrict__ eq, ef* __restrict__ partial) {
-  __shared__ uint32_t w_s[ABC0_MAX_Z * 8];
+  constexpr int NSK = 1 << K, NZ = NSK - 1;
+  __shared__ uint32_t w_s[NZ * NSK];
   __shared__ ef scratch[32];
-  const int nsk = 1 << k;
-  for (int i = threadIdx.x; i < nz * nsk; i += blockDim.x) w_s[i] = lw[i];
+  for (int i = threadIdx.x; i < NZ * NSK; i += blockDim.x) w_s[i] = lw[i];
   __syncthreads();
-  const size_t N = size_t(1) << log_n, S = N >> k;
-  ef acc[ABC0_MAX_Z];
+  ef acc[NZ];
 #pragma unroll
-  for (int z = 0; z < ABC0_MAX_Z; z++) acc[z] = ef_zero();
+  for (int z = 0; z < NZ; z++) acc[z] = ef_zero();
   for (size_t x = size_t(blockIdx.x) * blockDim.x + threadIdx.x; x < S; x += size_t(gridDim.x) * blockDim.x) {
-    uint32_t va[8], vb[8], vc[8];
+    uint32_t va[NSK], vb[NSK], vc[NSK];
 #pragma unroll
-    for (int j = 0; j < 8; j++)
-      if (j < nsk) va[j] = a[size_t(j) * S + x], vb[j] = b[size_t(j) * S + x], vc[j] = c[size_t(j) * S + x];
+    for (int j = 0; j < NSK; j++) {
+      va[j] = abc_in(a[size_t(j) * S + x]);
+      vb[j] = abc_in(b[size_t(j) * S + x]);
+      vc[j] = abc_in(c[size_t(j) * S + x]);
+    }
     const ef e = eq[x];
 #pragma unroll
-    for (int z = 0; z < ABC0_MAX_Z; z++) {
-      if (z >= nz) break;
-      const uint32_t* wz = w_s + z * nsk;
-      uint64_t sa = 0, sb = 0, sc = 0, ta = 0, tb = 0, tc = 0;
+    for (int z = 0; z < NZ; z++) {
+      const uint32_t* wz = w_s + z * NSK;
+      uint64_t sa[2] = {0, 0}, sb[2] = {0, 0}, sc[2] = {0, 0};
 #pragma unroll
-      for (int j = 0; j < 8; j++) {
-        if (j >= nsk) break;
-        if (j < 4) sa += wmul(wz[j], va[j]), sb += wmul(wz[j], vb[j]), sc += wmul(wz[j], vc[j]);
-        else ta += wmul(wz[j], va[j]), tb += wmul(wz[j], vb[j]), tc += wmul(wz[j], vc[j]);
-      }
-      const uint32_t A = add(redc(sa), redc(ta)), B = add(redc(sb), redc(tb)), C = add(redc(sc), redc(tc));
-      acc[z] = ef_add(acc[z], ef_mul_f(e, sub(mul(A, B), C)));
+      for (int j = 0; j < NSK; j++)
+        sa[j >> 2] += wmul(wz[j], va[j]), sb[j >> 2] += wmul(wz[j], vb[j]), sc[j >> 2] += wmul(wz[j], vc[j]);
+      auto fin = [](const uint64_t* s) { return NSK > 4 ? add(redc(s[0]), redc(s[1])) : redc(s[0]); };
+      acc[z] = ef_add(acc[z], ef_mul_f(e, sub(mul(fin(sa), fin(sb)), fin(sc))));
     }
   }
 #pragma unroll
-  for (int z = 0; z < ABC0_MAX_Z; z++) {
-    if (z >= nz) break;
+  for (int z = 0; z < NZ; z++) {
     const ef t = block_reduce_ef(acc[z], scratch);
-    if (threadIdx.x == 0) partial[size_t(blockIdx.x) * nz + z] = t;
+    if (threadIdx.x == 0) partial[size_t(blockIdx.x) * NZ + z] = t;
     __syncthreads();  // scratch is reused by the next point
   }
 }
@@ -1899,14 +1907,12 @@ __global__ void __launch_bounds__(ABC0_THREADS, 2) k_abc0_eval(const uint32_t* _
 // One thread per (x, point) with the block spanning the points: the form for 4 skipped
 // variables (15 points, too many to keep per thread).
 __global__ void k_abc0_eval_points(const uint32_t* __restrict__ a, const uint32_t* __restrict__ b,
-                            const uint32_t* __restrict__ c, int log_n, int k, int nz, const uint32_t* __restrict__ lw,
+                            const uint32_t* __restrict__ c, size_t S, int nsk, int nz, const uint32_t* __restrict__ lw,
                             const ef* __restrict__ eq, ef* __restrict__ partial) {
   __shared__ uint32_t w_s[32 * 16];
-  const int nsk = 1 << k;
   const int tid = threadIdx.y * ABC_X + threadIdx.x;
   for (int i = tid; i < nz * nsk; i += ABC_X * blockDim.y) w_s[i] = lw[i];
   __syncthreads();
-  const size_t N = size_t(1) << log_n, S = N >> k;
   const size_t x = size_t(blockIdx.x) * ABC_X + threadIdx.x;
   const int zi = threadIdx.y;
   ef res = ef_zero();
@@ -1915,9 +1921,9 @@ __global__ void k_abc0_eval_points(const uint32_t* __restrict__ a, const uint32_
     uint64_t sa[4] = {0, 0, 0, 0}, sb[4] = {0, 0, 0, 0}, sc[4] = {0, 0, 0, 0};
     for (int j = 0; j < nsk; j++) {
       size_t i = size_t(j) * S + x;
-      sa[j & 3] += wmul(wz[j], a[i]);
-      sb[j & 3] += wmul(wz[j], b[i]);
-      sc[j & 3] += wmul(wz[j], c[i]);
+      sa[j & 3] += wmul(wz[j], abc_in(a[i]));
+      sb[j & 3] += wmul(wz[j], abc_in(b[i]));
+      sc[j & 3] += wmul(wz[j], abc_in(c[i]));
     }
     auto fin = [](uint64_t* s) { return add(add(redc(s[0]), redc(s[1])), add(redc(s[2]), redc(s[3]))); };
     uint32_t v = sub(mul(fin(sa), fin(sb)), fin(sc));
@@ -1927,24 +1933,75 @@ __global__ void k_abc0_eval_points(const uint32_t* __restrict__ a, const uint32_
   if (threadIdx.x == 0 && zi < nz) partial[size_t(blockIdx.x) * nz + zi] = res;
 }
 
+// sum_j sel[j] src[j S + x], the loads first.
+template <int NSK>
+__device__ __forceinline__ ef abc_fold0(const uint32_t* __restrict__ src, size_t S, size_t x, const ef* sel) {
+  uint32_t v[NSK];
+#pragma unroll
+  for (int j = 0; j < NSK; j++) v[j] = src[size_t(j) * S + x];
+  EfMacF m;
+  m.init();
+#pragma unroll
+  for (int j = 0; j < NSK; j++) {
+    m.mac(sel[j], abc_in(v[j]));
+    if ((j & 3) == 3 && j + 1 < NSK) m.flush();
+  }
+  return m.value();
+}
+template <int NSK>
 __global__ void k_abc0_fold(const uint32_t* __restrict__ a, const uint32_t* __restrict__ b,
-                            const uint32_t* __restrict__ c, int log_n, int k, const ef* __restrict__ sel_g,
+                            const uint32_t* __restrict__ c, size_t S, const ef* __restrict__ sel_g,
                             ef* __restrict__ out) {
-  __shared__ ef sel[16];
-  const int nsk = 1 << k;
-  if (threadIdx.x < nsk) sel[threadIdx.x] = sel_g[threadIdx.x];
+  __shared__ ef sel[NSK];
+  if (threadIdx.x < NSK) sel[threadIdx.x] = sel_g[threadIdx.x];
   __syncthreads();
-  const size_t N = size_t(1) << log_n, S = N >> k;
   const size_t x = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (x >= S) return;
   const uint32_t* src = blockIdx.y == 0 ? a : blockIdx.y == 1 ? b : c;
-  EfMacF m;
-  m.init();
-  for (int j = 0; j < nsk; j++) {
-    m.mac(sel[j], src[size_t(j) * S + x]);
-    if ((j & 3) == 3 || j == nsk - 1) m.flush();
+  out[size_t(blockIdx.y) * S + x] = abc_fold0<NSK>(src, S, x, sel);
+}
+// The same with round 1 in one pass: thread x folds entries x and x + h of every column (h = S/2),
+// sums the eq table's leading variable out and adds round 1's values at 0 and 2; the last block
+// finishes the round. The folded columns are then written once and not read again before round
+// 2's fold. For 2^24 values and three skips: 0.24 ms, against 0.33 ms in four launches (fold, eq
+// table, sums, finish).
+template <int NSK>
+__global__ void __launch_bounds__(FE_THREADS, 2)
+    k_abc0_fold_eval(const uint32_t* __restrict__ a, const uint32_t* __restrict__ b, const uint32_t* __restrict__ c,
+                     size_t S, const ef* __restrict__ sel_g, const ef* __restrict__ eq, ef* __restrict__ out,
+                     ef* __restrict__ eq_new, ef* __restrict__ partial, const FinArgs fin) {
+  __shared__ ef scratch[32];
+  __shared__ ef sel[NSK];
+  if (threadIdx.x < NSK) sel[threadIdx.x] = sel_g[threadIdx.x];
+  __syncthreads();
+  const size_t h = S / 2;
+  ef s0 = ef_zero(), s2 = ef_zero();
+  for (size_t x = size_t(blockIdx.x) * blockDim.x + threadIdx.x; x < h; x += size_t(gridDim.x) * blockDim.x) {
+    // column q's entry x, and its value at 2 of the leading variable
+    auto column = [&](const uint32_t* src, int q, ef& lo, ef& at2) {
+      lo = abc_fold0<NSK>(src, S, x, sel);
+      out[size_t(q) * S + x] = lo;
+      const ef hi = abc_fold0<NSK>(src, S, x + h, sel);
+      out[size_t(q) * S + x + h] = hi;
+      at2 = ef_sub(ef_add(hi, hi), lo);
+    };
+    ef p0, p2, lo, at2;
+    column(a, 0, p0, p2);
+    column(b, 1, lo, at2);
+    p0 = ef_mul(p0, lo);
+    p2 = ef_mul(p2, at2);
+    column(c, 2, lo, at2);
+    const ef e = ef_add(eq[x], eq[x + h]);
+    eq_new[x] = e;
+    s0 = ef_add(s0, ef_mul(ef_sub(p0, lo), e));
+    s2 = ef_add(s2, ef_mul(ef_sub(p2, at2), e));
   }
-  out[size_t(blockIdx.y) * S + x] = m.value();
+  s0 = block_reduce_ef(s0, scratch);
+  if (threadIdx.x == 0) partial[size_t(blockIdx.x) * 2] = s0;
+  __syncthreads();
+  s2 = block_reduce_ef(s2, scratch);
+  if (threadIdx.x == 0) partial[size_t(blockIdx.x) * 2 + 1] = s2;
+  fin_last_block(FIN_EQSC3, fin, partial, 2);
 }
 
 __global__ void k_abc_eval_ef(const ef* __restrict__ cols, int m, const ef* __restrict__ eq, ef* __restrict__ partial) {
@@ -2248,19 +2305,42 @@ int abc0_blocks(int log_n, int k) {
 }
 void launch_abc0_eval(const uint32_t* a, const uint32_t* b, const uint32_t* c, int log_n, int k, int nz,
                       const uint32_t* lw, const ef* eq, ef* partial, cudaStream_t s) {
-  if (k > 3) {
-    if (nz > 32 || k > 4) throw std::runtime_error("abc round 0: too many points");
-    k_abc0_eval_points<<<abc0_blocks(log_n, k), dim3(ABC_X, nz), 0, s>>>(a, b, c, log_n, k, nz, lw, eq, partial);
-  } else {
-    if (nz > ABC0_MAX_Z) throw std::runtime_error("abc round 0: too many points");
-    k_abc0_eval<<<abc0_blocks(log_n, k), ABC0_THREADS, 0, s>>>(a, b, c, log_n, k, nz, lw, eq, partial);
-  }
+  const size_t S = size_t(1) << (log_n - k);
+  const int nb = abc0_blocks(log_n, k);
+  if (k < 1 || k > 4 || nz != (1 << k) - 1) throw std::invalid_argument("abc round 0: skips 1..4");
+  if (k == 1) k_abc0_eval<1><<<nb, ABC0_THREADS, 0, s>>>(a, b, c, S, lw, eq, partial);
+  if (k == 2) k_abc0_eval<2><<<nb, ABC0_THREADS, 0, s>>>(a, b, c, S, lw, eq, partial);
+  if (k == 3) k_abc0_eval<3><<<nb, ABC0_THREADS, 0, s>>>(a, b, c, S, lw, eq, partial);
+  if (k == 4) k_abc0_eval_points<<<nb, dim3(ABC_X, nz), 0, s>>>(a, b, c, S, 1 << k, nz, lw, eq, partial);
   WL_LAUNCH_CHECK();
 }
 void launch_abc0_fold(const uint32_t* a, const uint32_t* b, const uint32_t* c, int log_n, int k, const ef* sel,
                       ef* out, cudaStream_t s) {
-  size_t S = size_t(1) << (log_n - k);
-  k_abc0_fold<<<dim3((unsigned)((S + 255) / 256), 3), 256, 0, s>>>(a, b, c, log_n, k, sel, out);
+  const size_t S = size_t(1) << (log_n - k);
+  const dim3 grid((unsigned)((S + 255) / 256), 3);
+  if (k < 1 || k > 4) throw std::invalid_argument("abc round 0: skips 1..4");
+  if (k == 1) k_abc0_fold<2><<<grid, 256, 0, s>>>(a, b, c, S, sel, out);
+  if (k == 2) k_abc0_fold<4><<<grid, 256, 0, s>>>(a, b, c, S, sel, out);
+  if (k == 3) k_abc0_fold<8><<<grid, 256, 0, s>>>(a, b, c, S, sel, out);
+  if (k == 4) k_abc0_fold<16><<<grid, 256, 0, s>>>(a, b, c, S, sel, out);
+  WL_LAUNCH_CHECK();
+}
+int abc0_fold_eval_blocks(int log_n, int k) {
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const size_t h = size_t(1) << (log_n - k - 1);
+  return (int)std::max<size_t>(1, std::min<size_t>((h + FE_THREADS - 1) / FE_THREADS, size_t(sms) * 2));
+}
+void launch_abc0_fold_eval(const uint32_t* a, const uint32_t* b, const uint32_t* c, int log_n, int k, const ef* sel,
+                           const ef* eq, ef* out, ef* eq_new, ef* partial, const FinArgs& fin, cudaStream_t s) {
+  const size_t S = size_t(1) << (log_n - k);
+  const int nb = abc0_fold_eval_blocks(log_n, k);
+  if (k < 1 || k > 4 || S < 2) throw std::invalid_argument("abc round 0: skips 1..4");
+  if (k == 1) k_abc0_fold_eval<2><<<nb, FE_THREADS, 0, s>>>(a, b, c, S, sel, eq, out, eq_new, partial, fin);
+  if (k == 2) k_abc0_fold_eval<4><<<nb, FE_THREADS, 0, s>>>(a, b, c, S, sel, eq, out, eq_new, partial, fin);
+  if (k == 3) k_abc0_fold_eval<8><<<nb, FE_THREADS, 0, s>>>(a, b, c, S, sel, eq, out, eq_new, partial, fin);
+  if (k == 4) k_abc0_fold_eval<16><<<nb, FE_THREADS, 0, s>>>(a, b, c, S, sel, eq, out, eq_new, partial, fin);
   WL_LAUNCH_CHECK();
 }
 void launch_abc_eval_ef(const ef* cols, int m, const ef* eq, ef* partial, cudaStream_t s) {

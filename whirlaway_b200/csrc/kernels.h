@@ -187,11 +187,18 @@ void launch_abc_tail(const ef* cols, const ef* eq, size_t h, const ef* fold_ch, 
                      cudaStream_t s);
 
 // --------------------------------------------------------------- a*b - c zerocheck
+// Round 0 on the caller's columns (any 32-bit words, read as they are): lw and sel are the
+// Lagrange weights times 2^64 mod p.
 void launch_abc0_eval(const uint32_t* a, const uint32_t* b, const uint32_t* c, int log_n, int k, int nz,
                       const uint32_t* lw, const ef* eq, ef* partial, cudaStream_t s);
 int abc0_blocks(int log_n, int k);
 void launch_abc0_fold(const uint32_t* a, const uint32_t* b, const uint32_t* c, int log_n, int k, const ef* sel,
                       ef* out, cudaStream_t s);
+// The fold and round 1 in one launch: eq the table over S = 2^(log_n - k) entries, out the three
+// folded columns, eq_new round 1's table (S / 2), abc0_fold_eval_blocks partial rows.
+int abc0_fold_eval_blocks(int log_n, int k);
+void launch_abc0_fold_eval(const uint32_t* a, const uint32_t* b, const uint32_t* c, int log_n, int k, const ef* sel,
+                           const ef* eq, ef* out, ef* eq_new, ef* partial, const FinArgs& fin, cudaStream_t s);
 void launch_abc_eval_ef(const ef* cols, int m, const ef* eq, ef* partial, cudaStream_t s);
 
 // --------------------------------------------------------------- WHIR

@@ -1589,11 +1589,15 @@ std::vector<uint32_t> prove_abc(Context& ctx, const kb::P16Consts& p16, int n, i
     WL_CUDA(cudaEventElapsedTime(&ms, e0, e1));
     if (round_ms) round_ms->push_back(ms);
   };
-  DBuf cols;
+  DBuf cols, d_sel;
   DBuf eq0;
+  // round 0's fold joins round 1 (whose time it then counts to) when that is not in the last launch
+  const bool fold_round1 = S / 2 > TAIL_MAX_H && sumcheck_pow_bits(128, 3) == 0;
   {
     tick();
-    DBuf d_lw = upload(ctx, point_weights_cached(nsk, nz));
+    std::vector<uint32_t> lw = point_weights_cached(nsk, nz);
+    for (uint32_t& w : lw) w = kb::to_mont(w);  // the columns are canonical (launch_abc0_eval)
+    DBuf d_lw = upload(ctx, lw);
     eq0 = eq_table_dev(ctx, std::vector<ef>(r.begin() + 1, r.end()));
     const int nb = abc0_blocks(n, k);
     ef* part = ctx.partials(size_t(nb) * nz);
@@ -1611,18 +1615,25 @@ std::vector<uint32_t> prove_abc(Context& ctx, const kb::P16Consts& p16, int n, i
     ch.push_back(c0);
     sum = poly_eval(p, c0);
     grind(ctx, ts, p16, sumcheck_pow_bits(128, deg));
-    const std::vector<ef> selr = upoly_eval_all(sel, c0);
+    std::vector<ef> selr = upoly_eval_all(sel, c0);
     mmf = hv_dot(qv.data(), selr.data(), selr.size());
-    DBuf d_sel = upload(ctx, selr);
+    for (ef& e : selr) e = kb::ef_mul_f(e, kb::R2_MOD_P);
+    d_sel = upload(ctx, selr);
     cols = DBuf(sizeof(ef) * 3 * S, st);
-    { ProfScope _ps(ctx, "abc0_fold"); launch_abc0_fold(a, b, c, n, k, d_sel.as<ef>(), cols.as<ef>(), st); }
+    if (!fold_round1) {
+      ProfScope _ps(ctx, "abc0_fold");
+      launch_abc0_fold(a, b, c, n, k, d_sel.as<ef>(), cols.as<ef>(), st);
+    }
     tock();
   }
   const auto basis3 = lagrange_basis_cached(3);
   DBuf eqr;  // eq table of the current round, carried by the folds (see prove_air)
   if (n - k >= 1) {
     eqr = DBuf(sizeof(ef) * (S / 2), st);
-    { ProfScope _ps(ctx, "fold"); launch_fold_cols(nullptr, nullptr, 0, 0, nullptr, st, eq0.as<ef>(), eqr.as<ef>(), S / 2); }
+    if (!fold_round1) {
+      ProfScope _ps(ctx, "fold");
+      launch_fold_cols(nullptr, nullptr, 0, 0, nullptr, st, eq0.as<ef>(), eqr.as<ef>(), S / 2);
+    }
   }
   if (n - k >= 1 && sumcheck_pow_bits(128, 3) == 0) {
     // rounds >= 1 with the transcript on the device; per-round times from events recorded at
@@ -1632,7 +1643,7 @@ std::vector<uint32_t> prove_abc(Context& ctx, const kb::P16Consts& p16, int n, i
     for (auto& e : ev) e = event();
     WL_CUDA(cudaEventRecord(ev[0], st));
     int tail = 0;  // rounds of the last launch
-    // round 1 evaluates the round-0 fold as it is; round r >= 2 folds the columns (and sums the
+    // round 1 makes the round-0 fold and evaluates it; round r >= 2 folds the columns (and sums the
     // eq table's leading variable out) at challenge r - 1 and evaluates in one pass; the last
     // launch runs all rounds that fit one block and leaves the three final values
     for (int round = 1; round <= n - k; round++) {
@@ -1652,13 +1663,9 @@ std::vector<uint32_t> prove_abc(Context& ctx, const kb::P16Consts& p16, int n, i
         break;
       }
       if (round == 1) {
-        const int nb = (int)((half + 31) / 32);
-        ef* part = ctx.partials(size_t(nb) * 2);
-        {
-          ProfScope _ps(ctx, "abc_eval_ef");
-          launch_abc_eval_ef(cols.as<ef>(), m, eqr.as<ef>(), part, st);
-        }
-        ph.finish_round(FIN_EQSC3, part, nb);
+        ef* part = ctx.partials(size_t(2) * abc0_fold_eval_blocks(n, k));
+        ProfScope _ps(ctx, "abc0_fold_eval");
+        launch_abc0_fold_eval(a, b, c, n, k, d_sel.as<ef>(), eq0.as<ef>(), cols.as<ef>(), eqr.as<ef>(), part, ph.fin, st);
       } else {
         ef* part = ctx.partials(size_t(2) * fold_eval_blocks(half));
         DBuf nc(sizeof(ef) * 3 * 2 * half, st), eqn(sizeof(ef) * half, st);

@@ -156,7 +156,13 @@ __device__ __forceinline__ uint32_t zc0_rc(const AirConsts& K, int i) {
 // and the committed-column term -L_j(z) sum_r eq[x] sum_i alpha_i col_(17+i) of the block's
 // rows as partial[blockIdx.x * nz + z]; arow[r] = sum_i alpha_i col_(17+i) (the later rounds
 // carry its fold as one more column).
+// A thread's row is one chain: 37 steps of four column products, then 20 partial rounds, each
+// waiting for its loads. The loads run ZC0R_AHEAD words (4 in the rounds) ahead of their use:
+// 2^12 rows 38 us before, 25 after; 2^20 rows 424 us both ways (other warps hid the waits).
+// A table whose rows in blocks of 256 leave SMs idle runs in blocks of 64.
 constexpr int ZC0R_THREADS = 256;
+constexpr int ZC0R_SMALL = 64;
+constexpr int ZC0R_AHEAD = 12;  // a multiple of 4
 __global__ void __launch_bounds__(ZC0R_THREADS) k_zc0_rows(const uint32_t* __restrict__ wit, int log_n, int k,
                                                            int nz, const uint32_t* __restrict__ lw,
                                                            const ef* __restrict__ eq,
@@ -167,24 +173,35 @@ __global__ void __launch_bounds__(ZC0R_THREADS) k_zc0_rows(const uint32_t* __res
   __shared__ ef alphas[AIR_NC];
   __shared__ ef scratch[32];
   __shared__ ef total;
+  __shared__ ef rows[ZC0R_THREADS], sums[16];
   for (int i = threadIdx.x; i < AIR_NC; i += blockDim.x) alphas[i] = alphas_g[i];
   __syncthreads();
   const int lS = log_n - k;
   const size_t N = size_t(1) << log_n;
-  const size_t rb = size_t(blockIdx.x) * ZC0R_THREADS;
+  const size_t rb = size_t(blockIdx.x) * blockDim.x;
   const size_t r = rb + threadIdx.x;
   ef c = ef_zero();
   if (r < N) {
     const uint32_t* row = wit + up_row(r, N);
     EfMacF m;
     m.init();
+    // ZC0R_AHEAD column loads in flight ahead of the products that use them
+    uint32_t v[ZC0R_AHEAD];
+#pragma unroll
+    for (int e = 0; e < ZC0R_AHEAD; e++) v[e] = __ldg(row + size_t(17 + e) * N);
 #pragma unroll 1
     for (int i = 0; i < AIR_NC; i += 4) {
-      uint32_t v[4];
+      uint32_t u[4];
 #pragma unroll
-      for (int e = 0; e < 4; e++) v[e] = __ldg(row + size_t(17 + i + e) * N);
+      for (int e = 0; e < 4; e++) u[e] = v[e];
 #pragma unroll
-      for (int e = 0; e < 4; e++) m.mac(alphas[i + e], v[e]);
+      for (int e = 0; e + 4 < ZC0R_AHEAD; e++) v[e] = v[e + 4];
+      if (i + ZC0R_AHEAD < AIR_NC) {
+#pragma unroll
+        for (int e = 0; e < 4; e++) v[ZC0R_AHEAD - 4 + e] = __ldg(row + size_t(17 + i + ZC0R_AHEAD + e) * N);
+      }
+#pragma unroll
+      for (int e = 0; e < 4; e++) m.mac(alphas[i + e], u[e]);
       m.flush();
     }
     uint32_t s[16];
@@ -196,10 +213,17 @@ __global__ void __launch_bounds__(ZC0R_THREADS) k_zc0_rows(const uint32_t* __res
     for (int t = 0; t < 16; t++) qr[size_t(t) * N] = add(s[t], K.begin[0][t]);
 #pragma unroll
     for (int t = 0; t < 16; t++) s[t] = __ldg(row + size_t(65 + t) * N);
+    uint32_t post[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) post[e] = __ldg(row + size_t(81 + e) * N);
 #pragma unroll 1
     for (int pr = 0; pr < 20; pr++) {
+      const uint32_t p0 = post[0];
+#pragma unroll
+      for (int e = 0; e < 3; e++) post[e] = post[e + 1];
+      if (pr + 4 < 20) post[3] = __ldg(row + size_t(81 + pr + 4) * N);
       qr[size_t(16 + pr) * N] = add(s[0], K.partial[pr]);
-      internal_layer_with0<16>(s, __ldg(row + size_t(81 + pr) * N));
+      internal_layer_with0<16>(s, p0);
     }
 #pragma unroll
     for (int t = 0; t < 16; t++) qr[size_t(36 + t) * N] = add(s[t], K.end[0][t]);
@@ -207,20 +231,29 @@ __global__ void __launch_bounds__(ZC0R_THREADS) k_zc0_rows(const uint32_t* __res
     arow[r] = a;
     c = ef_mul(a, eq[r & ((size_t(1) << lS) - 1)]);
   }
-  const size_t last = (rb + ZC0R_THREADS <= N ? rb + ZC0R_THREADS : N) - 1;
   const int nsk = 1 << k;
-  if ((rb >> lS) == (last >> lS)) {  // one skip index j in the block: reduce, then weight
+  const int S = lS < 16 ? 1 << lS : 1 << 16;  // only compared with the block
+  if (S >= int(blockDim.x)) {  // one skip index j in the block: reduce, then weight
     const ef tot = block_reduce_ef(c, scratch);
     if (threadIdx.x == 0) total = tot;
     __syncthreads();
     const int j = int(rb >> lS);
     for (int z = threadIdx.x; z < nz; z += blockDim.x)
       partial[size_t(blockIdx.x) * nz + z] = ef_sub(ef_zero(), ef_mul_f(total, lw[size_t(z) * nsk + j]));
-  } else {  // small tables: weight per row, reduce per point
-    const int j = r < N ? int(r >> lS) : 0;
-    for (int z = 0; z < nz; z++) {
-      const ef v = block_reduce_ef(ef_mul_f(c, lw[size_t(z) * nsk + j]), scratch);
-      if (threadIdx.x == 0) partial[size_t(blockIdx.x) * nz + z] = ef_sub(ef_zero(), v);
+  } else {  // S divides the block: sum the rows of each j, then weight the sums per point
+    rows[threadIdx.x] = c;
+    __syncthreads();
+    const int j0 = int(rb >> lS), nj = min(int(blockDim.x), int(N - rb)) >> lS;
+    for (int e = threadIdx.x; e < nj * 8; e += blockDim.x) {
+      uint32_t v = 0;
+      for (int i = 0; i < S; i++) v = add(v, rows[((e >> 3) << lS) + i].c[e & 7]);
+      sums[e >> 3].c[e & 7] = v;
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < nz * 8; e += blockDim.x) {
+      uint32_t v = 0;
+      for (int j = 0; j < nj; j++) v = add(v, kb::mul(sums[j].c[e & 7], lw[size_t(e >> 3) * nsk + j0 + j]));
+      partial[size_t(blockIdx.x) * nz + (e >> 3)].c[e & 7] = kb::neg(v);
     }
   }
 }
@@ -240,6 +273,11 @@ __global__ void __launch_bounds__(ZC0R_THREADS) k_zc0_rows(const uint32_t* __res
 // sums, and the B fragments (16 words per lane) depend on z only. The 16 x 32 values of each
 // input are staged in shared memory by a cp.async pipeline, ZC0_GROUP inputs per stage; the
 // weights of j >= 2^k are zero, so unstaged entries contribute nothing.
+// A block walks 19 groups of inputs one after the other, ~5.5 us each; with too few x blocks to
+// fill the chip (2 an SM) the groups are split over blockIdx.y, each block with its own partial
+// sums: 2^12 rows (8 x blocks) 110 us before, 17 after (19 splits). From 256 x blocks on
+// (2^17 rows) one block keeps all groups.
+constexpr int ZC0_FILL = 2 * 148;
 constexpr int ZC0M_WARPS = 8;  // 2 x-tiles x 4 z-octets (30 points)
 __global__ void __launch_bounds__(ZC0M_WARPS * 32, 2) k_zc0_eval_mma(const uint32_t* __restrict__ wit,
                                                                     const uint32_t* __restrict__ q, int log_n,
@@ -303,11 +341,13 @@ __global__ void __launch_bounds__(ZC0M_WARPS * 32, 2) k_zc0_eval_mma(const uint3
     slast[e] = size_t(j) * S + xx == N - 1;
     sdst[e] = uint32_t(xl * ZC0_PAD + j);
   }
+  constexpr int NG = (AIR_NC + ZC0_GROUP - 1) / ZC0_GROUP;
+  const int per = (NG + gridDim.y - 1) / gridDim.y, g0 = blockIdx.y * per, g1 = min(g0 + per, NG);
   auto issue = [&](int grp) {
 #pragma unroll
     for (int cc = 0; cc < ZC0_GROUP; cc++) {
       const int i = ZC0_GROUP * grp + cc;
-      if (i < AIR_NC) {
+      if (i < AIR_NC && grp < g1) {
         const int qc = zc0_qcol(i);
         const uint32_t* col = qc >= 0 ? q + size_t(qc) * N : wit + size_t(1 + i) * N;
         uint32_t* dst = tile[grp % ZC0_STAGES][cc];
@@ -318,14 +358,13 @@ __global__ void __launch_bounds__(ZC0M_WARPS * 32, 2) k_zc0_eval_mma(const uint3
     }
     cp_async_commit();
   };
-  for (int grp = 0; grp < ZC0_STAGES - 1; grp++) issue(grp);
+  for (int grp = g0; grp < g0 + ZC0_STAGES - 1; grp++) issue(grp);
   EfMacF m[4];  // (x, z) = (g, 2t), (g, 2t + 1), (g + 8, 2t), (g + 8, 2t + 1) of the warp's tile
 #pragma unroll
   for (int o = 0; o < 4; o++) m[o].init();
-  constexpr int NG = (AIR_NC + ZC0_GROUP - 1) / ZC0_GROUP;
   static_assert(ZC0_GROUP % 4 == 0 && AIR_NC % 4 == 0, "flushes after every 4 products");
 #pragma unroll 1
-  for (int grp = 0; grp < NG; grp++) {
+  for (int grp = g0; grp < g1; grp++) {
     cp_async_wait<ZC0_STAGES - 2>();
     __syncthreads();  // group grp landed for every thread; the slot of group grp - 1 is free
     issue(grp + ZC0_STAGES - 1);
@@ -393,9 +432,31 @@ __global__ void __launch_bounds__(ZC0M_WARPS * 32, 2) k_zc0_eval_mma(const uint3
 #pragma unroll
     for (int c = 0; c < 2; c++) {
       const int z = zo * 8 + 2 * t + c;
-      if (z < nz) partial[size_t(blockIdx.x) * nz + z] = ef_add(sz[c], red[zo][2 * t + c]);
+      if (z < nz)
+        partial[(size_t(blockIdx.y) * gridDim.x + blockIdx.x) * nz + z] = ef_add(sz[c], red[zo][2 * t + c]);
     }
   }
+}
+
+// out[x] = sum_j sel[j] * a[j S + x] for the block's 32 x of an extension-field table a that is
+// already read at up rows (the committed-column combination of k_zc0_rows). Warp w takes j = w,
+// w + 8 of all 32 x; the eight sums of an x are added through shared memory, one coefficient of
+// one x per thread.
+__device__ void zc0_fold_arow(const ef* __restrict__ a, int log_n, int k, const ef* __restrict__ sel,
+                              ef* __restrict__ out, ef* sums) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const size_t S = size_t(1) << (log_n - k), x0 = size_t(blockIdx.x) * ZC0_X, x = x0 + lane;
+  EfMacE m;
+  m.init();
+  if (x < S)
+    for (int j = warp; j < (1 << k); j += ZC0M_WARPS) m.mac(sel[j], a[size_t(j) * S + x]);
+  sums[warp * ZC0_X + lane] = m.value();
+  __syncthreads();
+  const int xl = threadIdx.x >> 3, c = threadIdx.x & 7;
+  uint32_t v = 0;
+#pragma unroll
+  for (int w = 0; w < ZC0M_WARPS; w++) v = add(v, sums[w * ZC0_X + xl].c[c]);
+  if (x0 + xl < S) out[x0 + xl].c[c] = v;
 }
 
 // out[c * S + x] = sum_j sel[j] * up_c[j * S + x] for every column c, on the tensor cores as
@@ -404,12 +465,19 @@ __global__ void __launch_bounds__(ZC0M_WARPS * 32, 2) k_zc0_eval_mma(const uint3
 // of sel[j] and the 4 bytes b of the Montgomery form of sel[j]_n 2^(8a). Each lane ends with
 // all limbs of coefficients 2t, 2t + 1 of rows g, g + 8; one Montgomery reduction each. A
 // block holds 32 x and walks the columns in staged groups of ZC0_GROUP; warp (tile, slot)
-// takes columns slot and slot + 4 of each group. The up row of row N - 1 is N - 2.
+// takes columns slot and slot + 4 of each group. The up row of row N - 1 is N - 2. The groups are
+// split over blockIdx.y as in k_zc0_eval_mma (no sum to join here); the last blockIdx.y folds
+// the extension column: 2^12 rows 24 + 17 us as two launches of 8 and 1 blocks, 5 us in one.
 __global__ void __launch_bounds__(ZC0M_WARPS * 32) k_zc0_fold_mma(const uint32_t* __restrict__ wit, int log_n,
                                                                  int k, const ef* __restrict__ sel,
+                                                                 const ef* __restrict__ arow,
                                                                  ef* __restrict__ out) {
   __shared__ __align__(16) uint32_t tile[ZC0_STAGES][ZC0_GROUP][ZC0_X * ZC0_PAD];
   constexpr int NT = ZC0M_WARPS * 32;
+  if (blockIdx.y == gridDim.y - 1) {
+    zc0_fold_arow(arow, log_n, k, sel, out + (size_t(AIR_W) << (log_n - k)), reinterpret_cast<ef*>(tile));
+    return;
+  }
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3, mt = warp & 1, slot = warp >> 1;
   const int nsk = 1 << k;
@@ -447,11 +515,14 @@ __global__ void __launch_bounds__(ZC0M_WARPS * 32) k_zc0_fold_mma(const uint32_t
     srow[e] = uint32_t(row == N - 1 ? N - 2 : row);
     sdst[e] = uint32_t(xl * ZC0_PAD + j);
   }
+  constexpr int NG = (AIR_W + ZC0_GROUP - 1) / ZC0_GROUP;
+  const int splits = gridDim.y - 1, per = (NG + splits - 1) / splits;
+  const int g0 = blockIdx.y * per, g1 = min(g0 + per, NG);
   auto issue = [&](int grp) {
 #pragma unroll
     for (int cc = 0; cc < ZC0_GROUP; cc++) {
       const int c = ZC0_GROUP * grp + cc;
-      if (c < AIR_W) {
+      if (c < AIR_W && grp < g1) {
         const uint32_t* col = wit + size_t(c) * N;
         uint32_t* dst = tile[grp % ZC0_STAGES][cc];
 #pragma unroll
@@ -461,11 +532,10 @@ __global__ void __launch_bounds__(ZC0M_WARPS * 32) k_zc0_fold_mma(const uint32_t
     }
     cp_async_commit();
   };
-  for (int grp = 0; grp < ZC0_STAGES - 1; grp++) issue(grp);
-  constexpr int NG = (AIR_W + ZC0_GROUP - 1) / ZC0_GROUP;
+  for (int grp = g0; grp < g0 + ZC0_STAGES - 1; grp++) issue(grp);
   const size_t xa = x0 + 16 * mt + g, xb = xa + 8;
 #pragma unroll 1
-  for (int grp = 0; grp < NG; grp++) {
+  for (int grp = g0; grp < g1; grp++) {
     cp_async_wait<ZC0_STAGES - 2>();
     __syncthreads();  // group grp landed for every thread; the slot of group grp - 1 is free
     issue(grp + ZC0_STAGES - 1);
@@ -499,19 +569,6 @@ __global__ void __launch_bounds__(ZC0M_WARPS * 32) k_zc0_fold_mma(const uint32_t
     }
   }
   cp_async_wait<0>();
-}
-
-// out[x] = sum_j sel[j] * a[j * S + x] for an extension-field table a that is already read at
-// up rows (the committed-column combination of k_zc0_rows).
-__global__ void k_zc0_fold_ef(const ef* __restrict__ a, int log_n, int k, const ef* __restrict__ sel,
-                              ef* __restrict__ out) {
-  const size_t N = size_t(1) << log_n, S = N >> k;
-  const size_t x = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (x >= S) return;
-  EfMacE m;
-  m.init();
-  for (int j = 0; j < (1 << k); j++) m.mac(sel[j], a[size_t(j) * S + x]);
-  out[x] = m.value();
 }
 
 // ------------------------------------------------------------------ zerocheck rounds >= 1
@@ -1300,6 +1357,8 @@ __global__ void __launch_bounds__(ISM_WARPS * 32) k_inner_sums_bulk(const uint32
 // lo (limbs[(b * 8 + n) * nlo + x]). Each warp owns a 16-row tile (16 consecutive v_hi of one
 // u) and all 4 x 4 limb pairs, so every segment value is loaded and split into limbs once;
 // its rows' dot products times hi[v_hi], summed, are partial[(v_hi / 16) * 2^lu + u].
+// Short tables give v_hi 6 variables so that this form runs: 2^12 rows 41 + 12 us on
+// k_mle_partial_base and its sum (fewer than 16 v_hi), 7 + 4 + 3 us here.
 __global__ void __launch_bounds__(CS_WARPS * 32) k_mle_partial_mma(const uint32_t* __restrict__ T, size_t t_len,
                                                                   int lu, int lh, int ll,
                                                                   const ef* __restrict__ hi,
@@ -2058,34 +2117,46 @@ void launch_reduce_partials(const ef* partial, int nblk, int k, ef* out, cudaStr
   WL_LAUNCH_CHECK();
 }
 
-int zc0_blocks(int log_n, int k) {
+static int zc0_tiles(int log_n, int k) {  // blocks of 32 x
   size_t S = size_t(1) << (log_n - k);
   return (int)((S + ZC0_X - 1) / ZC0_X);
 }
-int zc0_row_blocks(int log_n) { return (int)(((size_t(1) << log_n) + ZC0R_THREADS - 1) / ZC0R_THREADS); }
+static int zc0_splits(int tiles, int groups) {
+  const int want = std::min(std::max(ZC0_FILL / tiles, 1), groups);
+  const int per = (groups + want - 1) / want;
+  return (groups + per - 1) / per;  // no empty range
+}
+static int zc0_eval_splits(int tiles) { return zc0_splits(tiles, (AIR_NC + ZC0_GROUP - 1) / ZC0_GROUP); }
+int zc0_blocks(int log_n, int k) {
+  const int tiles = zc0_tiles(log_n, k);
+  return tiles * zc0_eval_splits(tiles);
+}
+static int zc0_row_threads(int log_n) { return (size_t(1) << log_n) < size_t(148) * ZC0R_THREADS ? ZC0R_SMALL : ZC0R_THREADS; }
+int zc0_row_blocks(int log_n) {
+  const int t = zc0_row_threads(log_n);
+  return (int)(((size_t(1) << log_n) + t - 1) / t);
+}
 void launch_zc0_rows(const uint32_t* wit, int log_n, int k, int nz, const uint32_t* lw, const ef* eq,
                      const ef* alphas, const AirConsts& K, uint32_t* q, ef* partial, ef* arow, cudaStream_t s) {
-  k_zc0_rows<<<zc0_row_blocks(log_n), ZC0R_THREADS, 0, s>>>(wit, log_n, k, nz, lw, eq, alphas, K, q, partial,
-                                                            arow);
-  WL_LAUNCH_CHECK();
-}
-void launch_zc0_fold_ef(const ef* a, int log_n, int k, const ef* sel, ef* out, cudaStream_t s) {
-  const size_t S = size_t(1) << (log_n - k);
-  k_zc0_fold_ef<<<(unsigned)((S + 255) / 256), 256, 0, s>>>(a, log_n, k, sel, out);
+  k_zc0_rows<<<zc0_row_blocks(log_n), zc0_row_threads(log_n), 0, s>>>(wit, log_n, k, nz, lw, eq, alphas, K, q,
+                                                                      partial, arow);
   WL_LAUNCH_CHECK();
 }
 void launch_zc0_eval(const uint32_t* wit, const uint32_t* q, int log_n, int k, int nz, const uint32_t* lw,
                      const ef* eq, const ef* alphas, const ef* betas, const AirConsts& K, ef* partial,
                      cudaStream_t s) {
   if (nz > 32) throw std::invalid_argument("zc0_eval: at most 32 points");
-  k_zc0_eval_mma<<<zc0_blocks(log_n, k), ZC0M_WARPS * 32, 0, s>>>(wit, q, log_n, k, nz, lw, eq, alphas, betas, K,
-                                                                  partial);
+  const int tiles = zc0_tiles(log_n, k);
+  k_zc0_eval_mma<<<dim3(tiles, zc0_eval_splits(tiles)), ZC0M_WARPS * 32, 0, s>>>(wit, q, log_n, k, nz, lw, eq,
+                                                                                 alphas, betas, K, partial);
   WL_LAUNCH_CHECK();
 }
-void launch_zc0_fold(const uint32_t* wit, int log_n, int k, const ef* sel, ef* out, cudaStream_t s) {
+void launch_zc0_fold(const uint32_t* wit, const ef* arow, int log_n, int k, const ef* sel, ef* out,
+                     cudaStream_t s) {
   size_t S = size_t(1) << (log_n - k);
   if (S < 2) throw std::invalid_argument("zc0_fold: at least 2 points per skip block");
-  k_zc0_fold_mma<<<zc0_blocks(log_n, k), ZC0M_WARPS * 32, 0, s>>>(wit, log_n, k, sel, out);
+  const int tiles = zc0_tiles(log_n, k), splits = zc0_splits(tiles, (AIR_W + ZC0_GROUP - 1) / ZC0_GROUP);
+  k_zc0_fold_mma<<<dim3(tiles, splits + 1), ZC0M_WARPS * 32, 0, s>>>(wit, log_n, k, sel, arow, out);
   WL_LAUNCH_CHECK();
 }
 // Rounds with at least ZC_DENSE_MIN_HALF points per z use the dense kernels.

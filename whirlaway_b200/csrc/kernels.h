@@ -107,14 +107,13 @@ int zc0_blocks(int log_n, int k);
 int zc0_row_blocks(int log_n);
 void launch_zc0_rows(const uint32_t* wit, int log_n, int k, int nz, const uint32_t* lw, const ef* eq,
                      const ef* alphas, const AirConsts& K, uint32_t* q, ef* partial, ef* arow, cudaStream_t s);
-// Round-0 fold of the committed-column combination arow (2^log_n EF, one per row): out[x] =
-// sum_j sel[j] arow[j 2^(log_n-k) + x]. The rounds >= 1 carry it as column AIR_W of their
-// folded columns: the committed-post terms of every constraint, summed once per point.
-void launch_zc0_fold_ef(const ef* arow, int log_n, int k, const ef* sel, ef* out, cudaStream_t s);
 void launch_zc0_eval(const uint32_t* wit, const uint32_t* q, int log_n, int k, int nz, const uint32_t* lw,
                      const ef* eq, const ef* alphas, const ef* betas, const AirConsts& K, ef* partial,
                      cudaStream_t s);
-void launch_zc0_fold(const uint32_t* wit, int log_n, int k, const ef* sel, ef* out, cudaStream_t s);
+// Round-0 fold: out[c 2^(log_n-k) + x] = sum_j sel[j] up_c[j 2^(log_n-k) + x] for the AIR_W
+// columns and, as column AIR_W, the committed-column combination arow (2^log_n EF, one per
+// row): the committed-post terms of every constraint, summed once per point.
+void launch_zc0_fold(const uint32_t* wit, const ef* arow, int log_n, int k, const ef* sel, ef* out, cudaStream_t s);
 int zc_ef_blocks(int m);
 // True when the round over m variables runs on the dense kernels (k_zc_full_dense,
 // k_zc_partial_dense) rather than one block per point (k_zc_ef).

@@ -1072,6 +1072,12 @@ std::vector<uint32_t> prove_air(Context& ctx, const ProofJob& job, const uint32_
   const int lu = ws.c[0].fold, lv = m0 - lu;
   int lh_v, ll_v;
   split_vars(lv, lh_v, ll_v);
+  // The partial evaluation's tiles are 16 v_hi: a short table gives them 6 variables (down to
+  // INNER_MMA_MIN_LL left in the segments), so that 2^(lu + 2) warps share it.
+  if (lh_v < 6 && lv >= 4 + INNER_MMA_MIN_LL) {
+    lh_v = std::min(6, lv - INNER_MMA_MIN_LL);
+    ll_v = lv - lh_v;
+  }
   LdeSource src0{wit, t_len, 1, lv, ws.c[0].log_inv_rate, 0};
   src0.n_cols = (int)(((t_len + (size_t(1) << lv) - 1) >> lv) + 7) / 8 * 8;
   const kb::P2ConstsTc<24> p24 = kb::p2_consts_tc(job.p24);
@@ -1189,8 +1195,7 @@ std::vector<uint32_t> prove_air(Context& ctx, const ProofJob& job, const uint32_
       mmf = hv_dot(qv.data(), selr.data(), selr.size());
       DBuf d_sel = upload(ctx, selr);
       cols = DBuf(sizeof(ef) * size_t(W + 1) * S, st);
-      { ProfScope _ps(ctx, "zc0_fold"); launch_zc0_fold(wit, n, k, d_sel.as<ef>(), cols.as<ef>(), st); }
-      { ProfScope _ps(ctx, "zc0_fold"); launch_zc0_fold_ef(arow.as<ef>(), n, k, d_sel.as<ef>(), cols.as<ef>() + size_t(W) * S, st); }
+      { ProfScope _ps(ctx, "zc0_fold"); launch_zc0_fold(wit, arow.as<ef>(), n, k, d_sel.as<ef>(), cols.as<ef>(), st); }
       arow.reset();
     }
     const auto basis4 = lagrange_basis_cached(4);

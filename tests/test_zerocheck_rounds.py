@@ -1,5 +1,6 @@
-"""The zerocheck's round 0 over tables whose input groups are split over blocks, and the partial
-evaluation of short tables: proofs at the edges of the splits against the oracle."""
+"""The zerocheck's round 0 over tables whose input groups are split over blocks, its later rounds on
+the carried cube inputs, and the partial evaluation of short tables: proofs at the edges of the
+splits against the oracle."""
 import numpy as np
 import pytest
 

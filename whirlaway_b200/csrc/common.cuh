@@ -115,17 +115,21 @@ struct EfMacE {
     return uint64_t(uint32_t(v >> 32)) * EfMacF::C32 + uint32_t(v);
   }
   __device__ __forceinline__ void mac(const ef& a, const ef& b) {
-    uint32_t b3[8];
+    ef b3;
 #pragma unroll
-    for (int j = 0; j < 8; j++) b3[j] = kb::add(kb::dbl(b.c[j]), b.c[j]);
+    for (int j = 0; j < 8; j++) b3.c[j] = kb::add(kb::dbl(b.c[j]), b.c[j]);
+    mac3(a, b, b3);
+  }
+  // with b3 = 3 b from the caller
+  __device__ __forceinline__ void mac3(const ef& a, const ef& b, const ef& b3) {
 #pragma unroll
     for (int k = 0; k < 8; k++) {
       uint64_t v = s[k];
 #pragma unroll
-      for (int t = 0; t < 4; t++) v += kb::wmul(a.c[t], t <= k ? b.c[k - t] : b3[k + 8 - t]);
+      for (int t = 0; t < 4; t++) v += kb::wmul(a.c[t], t <= k ? b.c[k - t] : b3.c[k + 8 - t]);
       v = fold(v);
 #pragma unroll
-      for (int t = 4; t < 8; t++) v += kb::wmul(a.c[t], t <= k ? b.c[k - t] : b3[k + 8 - t]);
+      for (int t = 4; t < 8; t++) v += kb::wmul(a.c[t], t <= k ? b.c[k - t] : b3.c[k + 8 - t]);
       s[k] = fold(v);
     }
   }

@@ -459,25 +459,34 @@ __device__ void zc0_fold_arow(const ef* __restrict__ a, int log_n, int k, const 
   if (x0 + xl < S) out[x0 + xl].c[c] = v;
 }
 
-// out[c * S + x] = sum_j sel[j] * up_c[j * S + x] for every column c, on the tensor cores as
+// The columns the rounds >= 1 carry: the 148 cube inputs, first the ZC0_NQ computed ones in
+// q's order, then the committed ones in constraint order (zc_wit_col), and last the
+// committed-column combination.
+__device__ __forceinline__ int zc_wit_col(int c) { return c < 100 ? c - 35 : c + 1; }
+
+// out[(c - cb) * S + x] = sum_j sel[j] * v_c[j * S + x] for the cube inputs cb <= c < ce (either
+// all computed, src = q, or all committed, src = the witness at up rows), on the tensor cores as
 // in k_zc0_eval_mma: rows x, reduction index (j, a) over the 16 points and the 4 bytes of
-// up_c[j S + x] (the staged [x][j] words as they lie), columns (n, b) for the 8 coefficients n
+// v_c[j S + x] (the staged [x][j] words as they lie), columns (n, b) for the 8 coefficients n
 // of sel[j] and the 4 bytes b of the Montgomery form of sel[j]_n 2^(8a). Each lane ends with
 // all limbs of coefficients 2t, 2t + 1 of rows g, g + 8; one Montgomery reduction each. A
 // block holds 32 x and walks the columns in staged groups of ZC0_GROUP; warp (tile, slot)
 // takes columns slot and slot + 4 of each group. The up row of row N - 1 is N - 2. The groups are
-// split over blockIdx.y as in k_zc0_eval_mma (no sum to join here); the last blockIdx.y folds
-// the extension column: 2^12 rows 24 + 17 us as two launches of 8 and 1 blocks, 5 us in one.
-__global__ void __launch_bounds__(ZC0M_WARPS * 32) k_zc0_fold_mma(const uint32_t* __restrict__ wit, int log_n,
-                                                                 int k, const ef* __restrict__ sel,
+// split over blockIdx.y as in k_zc0_eval_mma (no sum to join here); with arow, the last
+// blockIdx.y folds it as column ce: 2^12 rows 24 + 17 us as two launches of 8 and 1 blocks over
+// all 166 columns, 5 us in one.
+__global__ void __launch_bounds__(ZC0M_WARPS * 32) k_zc0_fold_mma(const uint32_t* __restrict__ src, int log_n,
+                                                                 int k, int cb, int ce,
+                                                                 const ef* __restrict__ sel,
                                                                  const ef* __restrict__ arow,
                                                                  ef* __restrict__ out) {
   __shared__ __align__(16) uint32_t tile[ZC0_STAGES][ZC0_GROUP][ZC0_X * ZC0_PAD];
   constexpr int NT = ZC0M_WARPS * 32;
-  if (blockIdx.y == gridDim.y - 1) {
-    zc0_fold_arow(arow, log_n, k, sel, out + (size_t(AIR_W) << (log_n - k)), reinterpret_cast<ef*>(tile));
+  if (arow && blockIdx.y == gridDim.y - 1) {
+    zc0_fold_arow(arow, log_n, k, sel, out + (size_t(ce - cb) << (log_n - k)), reinterpret_cast<ef*>(tile));
     return;
   }
+  const bool comp = ce <= ZC0_NQ;  // computed inputs: the columns of src, already read at up rows
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3, mt = warp & 1, slot = warp >> 1;
   const int nsk = 1 << k;
@@ -512,18 +521,18 @@ __global__ void __launch_bounds__(ZC0M_WARPS * 32) k_zc0_fold_mma(const uint32_t
     if (xx >= S) xx = 0;
     sval[e] = idx < 16 * ZC0_X && j < nsk;
     const size_t row = size_t(j) * S + xx;
-    srow[e] = uint32_t(row == N - 1 ? N - 2 : row);
+    srow[e] = uint32_t(row == N - 1 && !comp ? N - 2 : row);
     sdst[e] = uint32_t(xl * ZC0_PAD + j);
   }
-  constexpr int NG = (AIR_W + ZC0_GROUP - 1) / ZC0_GROUP;
-  const int splits = gridDim.y - 1, per = (NG + splits - 1) / splits;
-  const int g0 = blockIdx.y * per, g1 = min(g0 + per, NG);
+  const int ng = (ce - cb + ZC0_GROUP - 1) / ZC0_GROUP;
+  const int splits = gridDim.y - (arow ? 1 : 0), per = (ng + splits - 1) / splits;
+  const int g0 = blockIdx.y * per, g1 = min(g0 + per, ng);
   auto issue = [&](int grp) {
 #pragma unroll
     for (int cc = 0; cc < ZC0_GROUP; cc++) {
-      const int c = ZC0_GROUP * grp + cc;
-      if (c < AIR_W && grp < g1) {
-        const uint32_t* col = wit + size_t(c) * N;
+      const int c = cb + ZC0_GROUP * grp + cc;
+      if (c < ce && grp < g1) {
+        const uint32_t* col = src + size_t(comp ? c : zc_wit_col(c)) * N;
         uint32_t* dst = tile[grp % ZC0_STAGES][cc];
 #pragma unroll
         for (int e = 0; e < NE; e++)
@@ -542,8 +551,8 @@ __global__ void __launch_bounds__(ZC0M_WARPS * 32) k_zc0_fold_mma(const uint32_t
 #pragma unroll
     for (int r = 0; r < 2; r++) {
       const int cc = slot + 4 * r;
-      const int c = ZC0_GROUP * grp + cc;
-      if (c >= AIR_W) break;
+      const int c = cb + ZC0_GROUP * grp + cc;
+      if (c >= ce) break;
       const uint32_t* r0 = tile[grp % ZC0_STAGES][cc] + (16 * mt + g) * ZC0_PAD;
       const uint32_t* r1 = r0 + 8 * ZC0_PAD;
       int acc[4][4];
@@ -564,284 +573,79 @@ __global__ void __launch_bounds__(ZC0M_WARPS * 32) k_zc0_fold_mma(const uint32_t
         const uint32_t hi = uint32_t(acc[2][o]) + (uint32_t(acc[3][o]) << 8);  // < 2^31
         res[o] = kb::redc(uint64_t(lo) + (uint64_t(hi) << 16));
       }
-      if (xa < S) reinterpret_cast<uint2*>(out + size_t(c) * S + xa)[t] = make_uint2(res[0], res[1]);
-      if (xb < S) reinterpret_cast<uint2*>(out + size_t(c) * S + xb)[t] = make_uint2(res[2], res[3]);
+      if (xa < S) reinterpret_cast<uint2*>(out + size_t(c - cb) * S + xa)[t] = make_uint2(res[0], res[1]);
+      if (xb < S) reinterpret_cast<uint2*>(out + size_t(c - cb) * S + xb)[t] = make_uint2(res[2], res[3]);
     }
   }
   cp_async_wait<0>();
 }
 
 // ------------------------------------------------------------------ zerocheck rounds >= 1
-// One block per (x, z), x < 2^(m-1), z in {0, 2, 3}: the 148 batched constraints at the
-// point whose columns are lo + z (hi - lo) (lo, hi = the column at x and 2^(m-1) + x).
-//  * Warps 0-3: thread (seg, j), seg < 7, j < 16, one full-round constraint without state.
-//    For full round f with weights alpha_(c0+i), sum_i alpha_(c0+i) (MDS(cubes)_i - post_i)
-//    = sum_j beta_(f,j) cube_j - sum_i alpha_(c0+i) post_i with beta_f = MDS^T alpha (from
-//    the host); each round's input is committed: the previous round's post columns, or
-//    MDS(inputs) for the first round. seg 0..3 = beginning rounds, 4..6 = ending rounds 1..3.
-//  * Warp 4: the 20 partial rounds and ending round 0, whose input is the state after the
-//    partial rounds. Lane i < 16 holds state word i; the internal layer's sum is a shuffle
-//    reduction over the 16 lanes. The state continues from the committed partial post p_r,
-//    so the S-box of round r is off the chain: lane r keeps state word 0 of round r and the
-//    20 S-box constraints are evaluated in parallel after the loop.
-constexpr int ZCE_THREADS = 160;
-
-__device__ __forceinline__ void m4_ef(ef& x0, ef& x1, ef& x2, ef& x3) {
-  ef t01 = ef_add(x0, x1), t23 = ef_add(x2, x3), t0123 = ef_add(t01, t23);
-  ef t01123 = ef_add(t0123, x1), t01233 = ef_add(t0123, x3);
-  ef y3 = ef_add(t01233, ef_add(x0, x0));
-  ef y1 = ef_add(t01123, ef_add(x2, x2));
-  ef y0 = ef_add(t01123, t01);
-  ef y2 = ef_add(t01233, t23);
-  x0 = y0;
-  x1 = y1;
-  x2 = y2;
-  x3 = y3;
+// The batched constraint at the points z = 0, 2, 3 of every x < 2^(m-1), weighted by eq[x]: the
+// 148 cube inputs and the committed-column combination are the carried columns (each an affine
+// function of the row, so their values at z are lo + z (hi - lo) of the folded columns, lo, hi
+// at x and 2^(m-1) + x), and the constraint is sum_c gamma_c cube(u_c + rc_c) minus the
+// combination: no linear layer is left in these rounds, and 149 columns are folded, not 166.
+// (Carrying the 165 witness columns instead needs the MDS of the inputs and the chain of the 20
+// partial rounds at every point: for 2^20 rows the six rounds of 2^10 points and more took 1.73 ms
+// and the ten smaller ones 0.21 ms; here 1.09 and 0.11 ms. 2^12 rows: 8 rounds 135, here 74 us.)
+// A warp holds 32 x, one z and every fourth column of its block's share; the three z of a block
+// read the same lines (L1 hit rate 95%). Bound by the wide multiplies: about 240 per column and
+// point (square, product, weight, reductions) keep the multiply pipe 85% busy. Columns are split
+// over blockIdx.y until the grid is two waves of 2 blocks an SM (six waves measured 1.16 ms: more
+// epilogues, and their partial sums need a second reduction), so a round of few x has one column
+// per warp and takes the latency of one term.
+constexpr int ZCS_COLS = 4;                          // columns at a time in a block
+constexpr int ZCS_THREADS = 3 * ZCS_COLS * 32;
+struct ZcCols {  // columns [0, split) at a, the rest at b
+  const ef *a, *b;
+  int split;
+  __device__ __forceinline__ const ef* col(int c, size_t len) const {
+    return c < split ? a + size_t(c) * len : b + size_t(c - split) * len;
+  }
+};
+__device__ __forceinline__ uint32_t zc_const(int c, const AirConsts& K) {
+  if (c < 52) return 0u;  // the computed inputs include theirs
+  return c < 100 ? K.begin[(c - 52) / 16 + 1][(c - 52) & 15] : K.end[(c - 100) / 16 + 1][(c - 100) & 15];
 }
-
-__device__ __forceinline__ ef shfl_xor_ef(const ef& v, int d) {
-  ef r;
-#pragma unroll
-  for (int i = 0; i < 8; i++) r.c[i] = __shfl_xor_sync(0xffffffffu, v.c[i], d);
-  return r;
-}
-__device__ __forceinline__ ef shfl_idx_ef(const ef& v, int src) {
-  ef r;
-#pragma unroll
-  for (int i = 0; i < 8; i++) r.c[i] = __shfl_sync(0xffffffffu, v.c[i], src);
-  return r;
-}
-
-__global__ void __launch_bounds__(ZCE_THREADS) k_zc_ef(const ef* __restrict__ cols, int m, const ef* __restrict__ eq,
-                                                      const ef* __restrict__ alphas, const ef* __restrict__ betas,
-                                                      const __grid_constant__ AirConsts K, ef* __restrict__ partial) {
+__global__ void __launch_bounds__(ZCS_THREADS, 2) k_zc_sbox(ZcCols cols, int m, const ef* __restrict__ eq,
+                                                            const ef* __restrict__ gam,
+                                                            const __grid_constant__ AirConsts K,
+                                                            ef* __restrict__ partial) {
+  __shared__ ef red[3][ZCS_COLS];
   const size_t len = size_t(1) << m, half = len >> 1;
-  const size_t x = blockIdx.x / 3;
-  const int zi = blockIdx.x - int(x) * 3;
-  auto get = [&](int c) -> ef {
-    const ef lo = cols[size_t(c) * len + x];
-    if (zi == 0) return lo;
-    const ef hi = cols[size_t(c) * len + half + x];
-    ef d = ef_sub(hi, lo);
-    ef v = ef_add(hi, d);               // z = 2: 2 hi - lo
-    return zi == 1 ? v : ef_add(v, d);  // z = 3: 3 hi - 2 lo
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, zi = warp % 3, cg = warp / 3;
+  const size_t x = size_t(blockIdx.x) * 32 + lane;
+  const bool valid = x < half;
+  const size_t xs = valid ? x : 0;
+  auto at = [&](const ef* col) {  // the column's value at the warp's z
+    ef lo = col[xs];
+    if (zi) {
+      const ef d = ef_sub(col[xs + half], lo);
+      const ef d2 = ef_add(d, d);
+      lo = ef_add(lo, zi == 1 ? d2 : ef_add(d2, d));
+    }
+    return lo;
   };
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  ef acc = ef_zero();
-  if (warp < 4) {
-    if (tid < 112) {
-      const int seg = tid >> 4, j = tid & 15;
-      const int f = seg < 4 ? seg : seg + 1;
-      const uint32_t rc = seg < 4 ? K.begin[seg][j] : K.end[seg - 3][j];
-      const int post = seg < 4 ? 17 + 16 * seg : 101 + 16 * (seg - 3);
-      ef in;
-      if (seg == 0) {
-        // MDS(inputs)_j: the M4 output of chunk j / 4 plus the sum over chunks of position j % 4
-        const int q0 = j >> 2, k0 = j & 3;
-        ef S = ef_zero(), own = ef_zero();
+  EfMacE acc;
+  acc.init();
 #pragma unroll 1
-        for (int q = 0; q < 4; q++) {
-          ef y[4] = {get(1 + 4 * q), get(2 + 4 * q), get(3 + 4 * q), get(4 + 4 * q)};
-          m4_ef(y[0], y[1], y[2], y[3]);
-          const ef yk = k0 == 0 ? y[0] : k0 == 1 ? y[1] : k0 == 2 ? y[2] : y[3];
-          S = ef_add(S, yk);
-          if (q == q0) own = yk;
-        }
-        in = ef_add(own, S);
-      } else {
-        in = get(post - 16 + j);
-      }
-      acc = ef_mul(betas[16 * f + j], ef_cube(ef_add_f(in, rc)));
-    }
-  } else {
-    const int i = lane & 15;
-    ef st = get(65 + i);                          // state after beginning round 3
-    const ef pr = lane < 20 ? get(81 + lane) : ef_zero();  // partial posts
-    const uint32_t dg = p2_diag<16>(i);
-    ef s0r = ef_zero();  // lane r: state word 0 at partial round r
-#pragma unroll 1
-    for (int r = 0; r < 20; r++) {
-      const ef w0 = shfl_idx_ef(st, 0);
-      if (lane == r) s0r = w0;
-      const ef p = shfl_idx_ef(pr, r);
-      ef sp = i == 0 ? p : st;
-      ef sum = sp;
-#pragma unroll
-      for (int d = 8; d > 0; d >>= 1) sum = ef_add(sum, shfl_xor_ef(sum, d));
-      st = ef_add(ef_mul_f(sp, dg), sum);
-    }
-    if (lane < 20) {
-      const ef x0 = ef_cube(ef_add_f(s0r, K.partial[lane]));
-      acc = ef_mul(alphas[64 + lane], x0);
-    }
-    if (lane < 16) {
-      acc = ef_add(acc, ef_mul(betas[16 * 4 + i], ef_cube(ef_add_f(st, K.end[0][i]))));
-    }
+  for (int c = blockIdx.y * ZCS_COLS + cg; c < AIR_NC; c += gridDim.y * ZCS_COLS) {
+    const ef u = ef_add_f(at(cols.col(c, len)), zc_const(c, K));
+    acc.mac3(ef_cube(u), gam[2 * c], gam[2 * c + 1]);
   }
-  acc = warp_reduce_ef(acc);
-  __shared__ ef wsum[ZCE_THREADS / 32];
-  if (lane == 0) wsum[warp] = acc;
+  ef v = acc.value();
+  if (blockIdx.y == 0 && cg == 0) v = ef_sub(v, at(cols.col(AIR_NC, len)));
+  v = warp_reduce_ef(valid ? ef_mul(v, eq[xs]) : ef_zero());
+  if (lane == 0) red[zi][cg] = v;
   __syncthreads();
-  if (tid == 0) {
-    ef tot = wsum[0];
+  if (threadIdx.x < 24) {
+    const int z = threadIdx.x >> 3, n = threadIdx.x & 7;
+    uint32_t s = red[z][0].c[n];
 #pragma unroll
-    for (int w = 1; w < ZCE_THREADS / 32; w++) tot = ef_add(tot, wsum[w]);
-    // the committed-post terms of all 148 constraints: the carried column
-    partial[blockIdx.x] = ef_mul(ef_sub(tot, get(AIR_W)), eq[x]);
+    for (int g = 1; g < ZCS_COLS; g++) s = add(s, red[z][g].c[n]);
+    partial[(size_t(blockIdx.y) * gridDim.x + blockIdx.x) * 3 + z].c[n] = s;
   }
-}
-
-// Dense forms of k_zc_ef for large rounds, in two kernels so that each keeps few
-// registers; both weight each point by eq[x] and write one partial sum per block and z
-// (blockIdx.y), first the full-round kernel's blocks, then the partial-round kernel's.
-//  * k_zc_full_dense: 16 lanes per point (2 points per warp); lane j evaluates constraint j
-//    of the 7 stateless full rounds. Beginning round 0 takes MDS(inputs): the lane's M4
-//    output plus the sum over the point's 4 chunks (two shuffles).
-//  * k_zc_partial_dense: 8 lanes per point (4 per warp); lane sub holds state words 2 sub,
-//    2 sub + 1 through the 20 partial rounds (the internal layer's sum is a local add plus
-//    three shuffles), keeps state word 0 of rounds r = sub (mod 8) for their S-box
-//    constraints, evaluated after the chain, and evaluates its two words of ending round 0.
-constexpr int ZCD_WARPS = 4;
-constexpr int ZCD_FULL_PTS = ZCD_WARPS * 2;     // points per block
-constexpr int ZCD_PARTIAL_PTS = ZCD_WARPS * 4;
-
-template <int PTS>
-__device__ __forceinline__ void zcd_block_store(ef v, ef* __restrict__ partial, size_t blk, int zi) {
-  __shared__ ef wsum[ZCD_WARPS];
-  v = warp_reduce_ef(v);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (lane == 0) wsum[warp] = v;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    ef t = wsum[0];
-#pragma unroll
-    for (int w = 1; w < ZCD_WARPS; w++) t = ef_add(t, wsum[w]);
-    partial[blk * 3 + zi] = t;
-  }
-}
-
-#define ZCD_GET                                                            \
-  auto get = [&](int c) -> ef {                                             \
-    const ef lo = cols[size_t(c) * len + xs];                               \
-    if (zi == 0) return lo;                                                 \
-    const ef hi = cols[size_t(c) * len + half + xs];                        \
-    ef d = ef_sub(hi, lo);                                                  \
-    ef v = ef_add(hi, d);                                                   \
-    return zi == 1 ? v : ef_add(v, d);                                      \
-  }
-
-__global__ void __launch_bounds__(ZCD_WARPS * 32) k_zc_full_dense(const ef* __restrict__ cols, int m,
-                                                                 const ef* __restrict__ eq,
-                                                                 const ef* __restrict__ alphas,
-                                                                 const ef* __restrict__ betas,
-                                                                 const __grid_constant__ AirConsts K,
-                                                                 ef* __restrict__ partial) {
-  const size_t len = size_t(1) << m, half = len >> 1;
-  const int lane = threadIdx.x & 31, zi = blockIdx.y;
-  const int j = lane & 15;
-  const size_t x = size_t(blockIdx.x) * ZCD_FULL_PTS + (threadIdx.x >> 4);
-  const bool valid = x < half;
-  const size_t xs = valid ? x : 0;
-  ZCD_GET;
-  ef in;
-  {
-    const int q = j >> 2;
-    ef y0 = get(1 + 4 * q), y1 = get(2 + 4 * q), y2 = get(3 + 4 * q), y3 = get(4 + 4 * q);
-    m4_ef(y0, y1, y2, y3);
-    const int k0 = j & 3;
-    const ef y = k0 == 0 ? y0 : k0 == 1 ? y1 : k0 == 2 ? y2 : y3;
-    ef t = ef_add(y, shfl_xor_ef(y, 4));
-    t = ef_add(t, shfl_xor_ef(t, 8));
-    in = ef_add(y, t);
-  }
-  EfMacE pos;  // beta * cube terms
-  pos.init();
-  // A round's input is the previous round's post, which this lane already holds, except for
-  // ending round 1 (segment 4), whose input is ending round 0's post. The next segment's
-  // post (and that one input) are loaded a segment ahead.
-  auto post_of = [](int seg) { return seg < 4 ? 17 + 16 * seg : 101 + 16 * (seg - 3); };
-  ef pv = get(post_of(0) + j);
-  ef in4 = ef_zero();
-#pragma unroll 1
-  for (int seg = 0; seg < 7; seg++) {
-    const int f = seg < 4 ? seg : seg + 1;
-    const uint32_t rc = seg < 4 ? K.begin[seg][j] : K.end[seg - 3][j];
-    const ef pv_next = seg < 5 ? get(post_of(seg + 1) + j) : ef_zero();
-    if (seg == 3) in4 = get(101 + j);
-    pos.mac(betas[16 * f + j], ef_cube(ef_add_f(in, rc)));
-    in = seg == 3 ? in4 : pv;
-    pv = pv_next;
-  }
-  // the committed-post terms of all 148 constraints are the carried column sum_i alpha_i
-  // col_(17+i), subtracted once per point
-  const ef acc = j == 0 ? ef_sub(pos.value(), get(AIR_W)) : pos.value();
-  // fold the point's 16 lanes, weight by eq, then the block sum
-  ef pt = acc;
-#pragma unroll
-  for (int d = 8; d > 0; d >>= 1) pt = ef_add(pt, shfl_xor_ef(pt, d));
-  const ef res = (j == 0 && valid) ? ef_mul(pt, eq[xs]) : ef_zero();
-  zcd_block_store<ZCD_FULL_PTS>(res, partial, blockIdx.x, zi);
-}
-
-__global__ void __launch_bounds__(ZCD_WARPS * 32) k_zc_partial_dense(const ef* __restrict__ cols, int m,
-                                                                    const ef* __restrict__ eq,
-                                                                    const ef* __restrict__ alphas,
-                                                                    const ef* __restrict__ betas,
-                                                                    const __grid_constant__ AirConsts K,
-                                                                    ef* __restrict__ partial) {
-  const size_t len = size_t(1) << m, half = len >> 1;
-  const int lane = threadIdx.x & 31, zi = blockIdx.y;
-  const int sub = lane & 7, gbase = lane & ~7;
-  const size_t x = size_t(blockIdx.x) * ZCD_PARTIAL_PTS + (threadIdx.x >> 3);
-  const bool valid = x < half;
-  const size_t xs = valid ? x : 0;
-  ZCD_GET;
-  ef st[2];
-  uint32_t dg[2];
-#pragma unroll
-  for (int kk = 0; kk < 2; kk++) {
-    st[kk] = get(65 + 2 * sub + kk);
-    dg[kk] = p2_diag<16>(2 * sub + kk);
-  }
-  // rounds in groups of 8 (a rolled loop keeps the code small): in group t, lane sub holds
-  // the partial post p_(8t+sub), records state word 0 of round 8t + sub, and evaluates that
-  // round's S-box constraint once the group is done
-  EfMacE pos;  // S-box / cube terms (the committed-post terms are in k_zc_full_dense)
-  pos.init();
-  ef p_cur = get(81 + sub);
-#pragma unroll 1
-  for (int t = 0; t < 3; t++) {
-    ef s0_cur = ef_zero();
-#pragma unroll
-    for (int o = 0; o < 8; o++) {
-      if (8 * t + o >= 20) break;
-      const ef w0 = shfl_idx_ef(st[0], gbase);
-      if (sub == o) s0_cur = w0;
-      const ef p = shfl_idx_ef(p_cur, gbase | o);
-      if (sub == 0) st[0] = p;
-      ef sum = ef_add(st[0], st[1]);
-      sum = ef_add(sum, shfl_xor_ef(sum, 1));
-      sum = ef_add(sum, shfl_xor_ef(sum, 2));
-      sum = ef_add(sum, shfl_xor_ef(sum, 4));
-#pragma unroll
-      for (int kk = 0; kk < 2; kk++) st[kk] = ef_add(ef_mul_f(st[kk], dg[kk]), sum);
-    }
-    const int r = 8 * t + sub;
-    if (r < 20) {
-      pos.mac(alphas[64 + r], ef_cube(ef_add_f(s0_cur, K.partial[r])));
-    }
-    if (t < 2) p_cur = (r + 8 < 20) ? get(81 + r + 8) : ef_zero();
-  }
-#pragma unroll
-  for (int kk = 0; kk < 2; kk++) {
-    const int j = 2 * sub + kk;
-    pos.mac(betas[16 * 4 + j], ef_cube(ef_add_f(st[kk], K.end[0][j])));
-  }
-  ef pt = pos.value();
-#pragma unroll
-  for (int d = 4; d > 0; d >>= 1) pt = ef_add(pt, shfl_xor_ef(pt, d));
-  const ef res = (sub == 0 && valid) ? ef_mul(pt, eq[xs]) : ef_zero();
-  zcd_block_store<ZCD_PARTIAL_PTS>(res, partial, blockIdx.x, zi);
 }
 
 // Folds every column at the challenge (*r, or rv when r is null) and, in the extra column
@@ -912,7 +716,7 @@ __device__ __forceinline__ void lerp16_mma(const ef* __restrict__ lo, const ef* 
 // column slot (blockIdx.y == ncols) sums the next eq table as k_fold_cols does.
 // The challenge comes by value (rv) or, when rptr is set, from device memory (a challenge
 // sampled on the device by the round-finishing kernel).
-__global__ void __launch_bounds__(256) k_fold_cols_mma(const ef* __restrict__ in, ef* __restrict__ out, size_t half,
+__global__ void __launch_bounds__(256) k_fold_cols_mma(ZcCols in, ef* __restrict__ out, size_t half,
                                                       int ncols, ef rv, const ef* __restrict__ rptr,
                                                       const ef* __restrict__ eq_in, ef* __restrict__ eq_out,
                                                       size_t eq_half) {
@@ -927,7 +731,7 @@ __global__ void __launch_bounds__(256) k_fold_cols_mma(const ef* __restrict__ in
   if (x0 >= half) return;  // whole warp
   uint32_t bf[4][2];
   fold_frag(rptr ? *rptr : rv, g, t, bf);
-  const ef* src = in + size_t(c) * 2 * half;
+  const ef* src = in.col(c, 2 * half);
   const uint32_t nv = half - x0 < 16 ? uint32_t(half - x0) : 16u;
   lerp16_mma(src + x0, src + half + x0, out + size_t(c) * half + x0, nv, bf, g, t);
 }
@@ -2151,35 +1955,46 @@ void launch_zc0_eval(const uint32_t* wit, const uint32_t* q, int log_n, int k, i
                                                                                  alphas, betas, K, partial);
   WL_LAUNCH_CHECK();
 }
-void launch_zc0_fold(const uint32_t* wit, const ef* arow, int log_n, int k, const ef* sel, ef* out,
+void launch_zc0_fold(const uint32_t* src, int log_n, int k, int cb, int ce, const ef* sel, const ef* arow, ef* out,
                      cudaStream_t s) {
   size_t S = size_t(1) << (log_n - k);
   if (S < 2) throw std::invalid_argument("zc0_fold: at least 2 points per skip block");
-  const int tiles = zc0_tiles(log_n, k), splits = zc0_splits(tiles, (AIR_W + ZC0_GROUP - 1) / ZC0_GROUP);
-  k_zc0_fold_mma<<<dim3(tiles, splits + 1), ZC0M_WARPS * 32, 0, s>>>(wit, log_n, k, sel, arow, out);
+  const int tiles = zc0_tiles(log_n, k), splits = zc0_splits(tiles, (ce - cb + ZC0_GROUP - 1) / ZC0_GROUP);
+  k_zc0_fold_mma<<<dim3(tiles, splits + (arow ? 1 : 0)), ZC0M_WARPS * 32, 0, s>>>(src, log_n, k, cb, ce, sel, arow,
+                                                                                 out);
   WL_LAUNCH_CHECK();
 }
-// Rounds with at least ZC_DENSE_MIN_HALF points per z use the dense kernels.
-constexpr size_t ZC_DENSE_MIN_HALF = size_t(1) << 10;
-bool zc_eval_is_dense(int m) { return (size_t(1) << (m - 1)) >= ZC_DENSE_MIN_HALF; }
-int zc_ef_blocks(int m) {  // partial sums per z
-  const size_t half = size_t(1) << (m - 1);
-  if (half < ZC_DENSE_MIN_HALF) return (int)half;
-  return (int)((half + ZCD_FULL_PTS - 1) / ZCD_FULL_PTS + (half + ZCD_PARTIAL_PTS - 1) / ZCD_PARTIAL_PTS);
+bool zc_eval_is_dense(int m) { return m - 1 >= 10; }
+// x blocks of 32, and the split of the columns that gives at least ZCS_FILL blocks.
+constexpr int ZCS_FILL = 2 * 2 * 148;
+static dim3 zcs_grid(int m) {
+  const size_t bx = ((size_t(1) << (m - 1)) + 31) / 32;
+  constexpr int most = AIR_NC / ZCS_COLS;  // one column per warp
+  const int want = (int)std::min<size_t>((ZCS_FILL + bx - 1) / bx, most);
+  const int per = (most + want - 1) / want;
+  return dim3((unsigned)bx, (unsigned)((most + per - 1) / per));
 }
-void launch_zc_eval_ef(const ef* cols, int m, const ef* eq, const ef* alphas, const ef* betas, const AirConsts& K,
-                       ef* partial, cudaStream_t s) {
-  const size_t half = size_t(1) << (m - 1);
-  if (half >= ZC_DENSE_MIN_HALF) {
-    const unsigned bf = (unsigned)((half + ZCD_FULL_PTS - 1) / ZCD_FULL_PTS);
-    const unsigned bp = (unsigned)((half + ZCD_PARTIAL_PTS - 1) / ZCD_PARTIAL_PTS);
-    k_zc_full_dense<<<dim3(bf, 3), ZCD_WARPS * 32, 0, s>>>(cols, m, eq, alphas, betas, K, partial);
-    WL_LAUNCH_CHECK();
-    k_zc_partial_dense<<<dim3(bp, 3), ZCD_WARPS * 32, 0, s>>>(cols, m, eq, alphas, betas, K,
-                                                              partial + size_t(bf) * 3);
-  } else {
-    k_zc_ef<<<(unsigned)(half * 3), ZCE_THREADS, 0, s>>>(cols, m, eq, alphas, betas, K, partial);
+int zc_ef_blocks(int m) {
+  const dim3 g = zcs_grid(m);
+  return (int)(g.x * g.y);
+}
+std::vector<ef> zc_gammas(const std::vector<ef>& alphas, const std::vector<ef>& betas) {
+  std::vector<ef> g(2 * AIR_NC);
+  for (int c = 0; c < AIR_NC; c++) {
+    const ef v = c < 16   ? betas[c]
+                 : c < 36 ? alphas[c + 48]   // partial round c - 16: constraint 64 + (c - 16)
+                 : c < 52 ? betas[c + 28]    // ending round 0
+                 : c < 100 ? betas[c - 36]   // beginning rounds 1..3
+                           : betas[c - 20];  // ending rounds 1..3
+    g[2 * c] = v;
+    g[2 * c + 1] = kb::ef_add(kb::ef_add(v, v), v);
   }
+  return g;
+}
+void launch_zc_eval_ef(const ef* cols, const ef* cols2, int m, const ef* eq, const ef* gammas, const AirConsts& K,
+                       ef* partial, cudaStream_t s) {
+  k_zc_sbox<<<zcs_grid(m), ZCS_THREADS, 0, s>>>(ZcCols{cols, cols2, cols2 ? ZC0_NQ : ZC_COLS}, m, eq, gammas, K,
+                                                partial);
   WL_LAUNCH_CHECK();
 }
 void launch_fold_cols(const ef* in, ef* out, int ncols, size_t half, const ef* r, cudaStream_t s, const ef* eq_in,
@@ -2190,18 +2005,18 @@ void launch_fold_cols(const ef* in, ef* out, int ncols, size_t half, const ef* r
   WL_LAUNCH_CHECK();
 }
 void launch_fold_cols_at(const ef* in, ef* out, int ncols, size_t half, const ef& r, cudaStream_t s, const ef* eq_in,
-                         ef* eq_out, size_t eq_half) {
+                         ef* eq_out, size_t eq_half, const ef* in2, int split) {
   // 128 values per block for the columns, 256 for the eq table
   const size_t bx = std::max((half + 127) / 128, eq_in ? (eq_half + 255) / 256 : size_t(0));
   dim3 grid((unsigned)std::max<size_t>(bx, 1), ncols + (eq_in ? 1 : 0));
-  k_fold_cols_mma<<<grid, 256, 0, s>>>(in, out, half, ncols, r, nullptr, eq_in, eq_out, eq_half);
+  k_fold_cols_mma<<<grid, 256, 0, s>>>(ZcCols{in, in2, in2 ? split : ncols}, out, half, ncols, r, nullptr, eq_in, eq_out, eq_half);
   WL_LAUNCH_CHECK();
 }
 void launch_fold_cols_dev(const ef* in, ef* out, int ncols, size_t half, const ef* r_dev, cudaStream_t s,
-                          const ef* eq_in, ef* eq_out, size_t eq_half) {
+                          const ef* eq_in, ef* eq_out, size_t eq_half, const ef* in2, int split) {
   const size_t bx = std::max((half + 127) / 128, eq_in ? (eq_half + 255) / 256 : size_t(0));
   dim3 grid((unsigned)std::max<size_t>(bx, 1), ncols + (eq_in ? 1 : 0));
-  k_fold_cols_mma<<<grid, 256, 0, s>>>(in, out, half, ncols, ef_zero(), r_dev, eq_in, eq_out, eq_half);
+  k_fold_cols_mma<<<grid, 256, 0, s>>>(ZcCols{in, in2, in2 ? split : ncols}, out, half, ncols, ef_zero(), r_dev, eq_in, eq_out, eq_half);
   WL_LAUNCH_CHECK();
 }
 void launch_inner_sums(const uint32_t* wit, int log_n, int k, int ll, const ef* eq_hi, const ef* eq_lo,

@@ -5,6 +5,7 @@
 
 #include <cstddef>
 #include <cstdint>
+#include <vector>
 
 #include "air.cuh"
 #include "common.cuh"
@@ -110,28 +111,35 @@ void launch_zc0_rows(const uint32_t* wit, int log_n, int k, int nz, const uint32
 void launch_zc0_eval(const uint32_t* wit, const uint32_t* q, int log_n, int k, int nz, const uint32_t* lw,
                      const ef* eq, const ef* alphas, const ef* betas, const AirConsts& K, ef* partial,
                      cudaStream_t s);
-// Round-0 fold: out[c 2^(log_n-k) + x] = sum_j sel[j] up_c[j 2^(log_n-k) + x] for the AIR_W
-// columns and, as column AIR_W, the committed-column combination arow (2^log_n EF, one per
-// row): the committed-post terms of every constraint, summed once per point.
-void launch_zc0_fold(const uint32_t* wit, const ef* arow, int log_n, int k, const ef* sel, ef* out, cudaStream_t s);
+// Round-0 fold of the cube inputs cb <= c < ce of the carried columns: out[(c - cb) 2^(log_n-k) + x]
+// = sum_j sel[j] v_c[j 2^(log_n-k) + x], from src = launch_zc0_rows' q (ce <= ZC0_NQ) or src = the
+// witness (cb >= ZC0_NQ); with arow (2^log_n EF, one per row) its fold is column ce.
+constexpr int ZC_COLS = AIR_NC + 1;  // the carried columns: 148 cube inputs and the combination
+void launch_zc0_fold(const uint32_t* src, int log_n, int k, int cb, int ce, const ef* sel, const ef* arow, ef* out,
+                     cudaStream_t s);
 int zc_ef_blocks(int m);
-// True when the round over m variables runs on the dense kernels (k_zc_full_dense,
-// k_zc_partial_dense) rather than one block per point (k_zc_ef).
+// Rounds of at least 2^10 points per z (timed in a class of their own).
 bool zc_eval_is_dense(int m);
-// cols: AIR_W + 1 folded columns (the last one the committed-column combination).
-// betas: the 8 full rounds' 16 weights beta_f = MDS^T (alpha_(c0(f)+i))_i, f = 0..7.
-void launch_zc_eval_ef(const ef* cols, int m, const ef* eq, const ef* alphas, const ef* betas, const AirConsts& K,
+// cols: the ZC_COLS carried columns, the ones from ZC0_NQ on at cols2 when it is given.
+// Writes zc_ef_blocks(m) partial sums for each of z = 0, 2, 3.
+// gammas: the cube inputs' weights, each beside its triple (zc_gammas, from the 148 alphas and
+// the 8 full rounds' 16 weights beta_f = MDS^T (alpha_(c0(f)+i))_i, f = 0..7).
+std::vector<ef> zc_gammas(const std::vector<ef>& alphas, const std::vector<ef>& betas);
+void launch_zc_eval_ef(const ef* cols, const ef* cols2, int m, const ef* eq, const ef* gammas, const AirConsts& K,
                        ef* partial, cudaStream_t s);
 // Folds every column at r; with eq_in, also writes the next round's eq table
 // eq_out[x] = eq_in[x] + eq_in[x + eq_half].
 void launch_fold_cols(const ef* in, ef* out, int ncols, size_t half, const ef* r, cudaStream_t s,
                       const ef* eq_in = nullptr, ef* eq_out = nullptr, size_t eq_half = 0);
-// The same with the challenge passed by value (no device copy of it).
+// The same with the challenge passed by value (no device copy of it); with in2, the columns from
+// `split` on are read there.
 void launch_fold_cols_at(const ef* in, ef* out, int ncols, size_t half, const ef& r, cudaStream_t s,
-                         const ef* eq_in = nullptr, ef* eq_out = nullptr, size_t eq_half = 0);
+                         const ef* eq_in = nullptr, ef* eq_out = nullptr, size_t eq_half = 0,
+                         const ef* in2 = nullptr, int split = 0);
 // The same with the challenge in device memory (sampled by a round-finishing kernel).
 void launch_fold_cols_dev(const ef* in, ef* out, int ncols, size_t half, const ef* r_dev, cudaStream_t s,
-                          const ef* eq_in = nullptr, ef* eq_out = nullptr, size_t eq_half = 0);
+                          const ef* eq_in = nullptr, ef* eq_out = nullptr, size_t eq_half = 0,
+                          const ef* in2 = nullptr, int split = 0);
 // Up/down evaluations of every column at (r0; tail), with eq(tail, .) factored as
 // eq_hi (2^(log_n-k-ll) entries) x eq_lo (2^ll entries). out_up / out_down must hold
 // AIR_W * (1 + 2^k * 2^(log_n-k-ll)) elements; the first AIR_W are the results.

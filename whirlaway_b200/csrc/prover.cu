@@ -1153,9 +1153,10 @@ std::vector<uint32_t> prove_air(Context& ctx, const ProofJob& job, const uint32_
   const int nz = 3 * (nsk - 1) - nsk + 1;
   const std::vector<uint32_t> lw = prog ? std::vector<uint32_t>() : point_weights_cached(nsk, nz);
   UploadSet up;
-  const int ia = up.add(alphas), ib = up.add(betas), il = up.add(lw);
+  const std::vector<ef> gammas = prog ? std::vector<ef>() : zc_gammas(alphas, betas);
+  const int ia = up.add(alphas), ib = up.add(betas), ig = up.add(gammas), il = up.add(lw);
   up.upload(ctx);
-  const ef *d_alphas = up.at<ef>(ia), *d_betas = up.at<ef>(ib);
+  const ef *d_alphas = up.at<ef>(ia), *d_betas = up.at<ef>(ib), *d_gammas = up.at<ef>(ig);
   std::vector<ef> zc_tail(zc.begin() + 1, zc.end());
   DBuf eq0 = eq_table_dev(ctx, zc_tail);
   std::vector<ef> challenges;
@@ -1165,19 +1166,17 @@ std::vector<uint32_t> prove_air(Context& ctx, const ProofJob& job, const uint32_
   } else {
     ef sum = kb::ef_zero();
     ef mmf = kb::ef_one();
-    DBuf cols;
-    // the committed-column combination sum_i alpha_i col_(17+i) of every row; folded, it is the
-    // last of the W + 1 columns of the rounds >= 1
-    DBuf arow(sizeof(ef) * N, st);
+    // the columns of the rounds >= 1 (ZC_COLS, see launch_zc_eval_ef): after round 0 the computed
+    // ones in `cols` and the others in `cols2`, so that q is gone before the second is allocated
+    DBuf cols, cols2;
+    // the committed-column combination sum_i alpha_i col_(17+i) of every row
+    DBuf arow(sizeof(ef) * N, st), q(sizeof(uint32_t) * ZC0_NQ * N, st);
     {
       const uint32_t* d_lw = up.at<uint32_t>(il);
       const int nb = zc0_blocks(n, k), nbr = zc0_row_blocks(n);
       ef* part = ctx.partials(size_t(nb + nbr) * nz);
-      {
-        DBuf q(sizeof(uint32_t) * ZC0_NQ * N, st);
-        { ProfScope _ps(ctx, "zc0_rows"); launch_zc0_rows(wit, n, k, nz, d_lw, eq0.as<ef>(), d_alphas, job.air, q.as<uint32_t>(), part + size_t(nb) * nz, arow.as<ef>(), st); }
-        { ProfScope _ps(ctx, "zc0_eval"); launch_zc0_eval(wit, q.as<uint32_t>(), n, k, nz, d_lw, eq0.as<ef>(), d_alphas, d_betas, job.air, part, st); }
-      }
+      { ProfScope _ps(ctx, "zc0_rows"); launch_zc0_rows(wit, n, k, nz, d_lw, eq0.as<ef>(), d_alphas, job.air, q.as<uint32_t>(), part + size_t(nb) * nz, arow.as<ef>(), st); }
+      { ProfScope _ps(ctx, "zc0_eval"); launch_zc0_eval(wit, q.as<uint32_t>(), n, k, nz, d_lw, eq0.as<ef>(), d_alphas, d_betas, job.air, part, st); }
       std::vector<ef> sums = reduce_to_host(ctx, part, nb + nbr, nz);
       std::vector<ef> ys(nsk, kb::ef_zero());
       ys.insert(ys.end(), sums.begin(), sums.end());
@@ -1194,8 +1193,11 @@ std::vector<uint32_t> prove_air(Context& ctx, const ProofJob& job, const uint32_
       const std::vector<ef> selr = upoly_eval_all(sel, r0);
       mmf = hv_dot(qv.data(), selr.data(), selr.size());
       DBuf d_sel = upload(ctx, selr);
-      cols = DBuf(sizeof(ef) * size_t(W + 1) * S, st);
-      { ProfScope _ps(ctx, "zc0_fold"); launch_zc0_fold(wit, arow.as<ef>(), n, k, d_sel.as<ef>(), cols.as<ef>(), st); }
+      cols = DBuf(sizeof(ef) * size_t(ZC0_NQ) * S, st);
+      { ProfScope _ps(ctx, "zc0_fold"); launch_zc0_fold(q.as<uint32_t>(), n, k, 0, ZC0_NQ, d_sel.as<ef>(), nullptr, cols.as<ef>(), st); }
+      q.reset();
+      cols2 = DBuf(sizeof(ef) * size_t(ZC_COLS - ZC0_NQ) * S, st);
+      { ProfScope _ps(ctx, "zc0_fold"); launch_zc0_fold(wit, n, k, ZC0_NQ, AIR_NC, d_sel.as<ef>(), arow.as<ef>(), cols2.as<ef>(), st); }
       arow.reset();
     }
     const auto basis4 = lagrange_basis_cached(4);
@@ -1216,13 +1218,14 @@ std::vector<uint32_t> prove_air(Context& ctx, const ProofJob& job, const uint32_
         const size_t half = size_t(1) << (m - 1);
         const int nb = zc_ef_blocks(m);
         ef* part = ctx.partials(size_t(nb) * 3);
-        { ProfScope _ps(ctx, zc_eval_is_dense(m) ? "zc_eval_dense" : "zc_eval_ef"); launch_zc_eval_ef(cols.as<ef>(), m, eqr.as<ef>(), d_alphas, d_betas, job.air, part, st); }
+        { ProfScope _ps(ctx, zc_eval_is_dense(m) ? "zc_eval_dense" : "zc_eval_ef"); launch_zc_eval_ef(cols.as<ef>(), cols2.as<ef>(), m, eqr.as<ef>(), d_gammas, job.air, part, st); }
         ph.finish_round(FIN_EQSC4, part, nb);
-        DBuf nc(sizeof(ef) * size_t(W + 1) * half, st);
+        DBuf nc(sizeof(ef) * size_t(ZC_COLS) * half, st);
         DBuf eqn(sizeof(ef) * std::max<size_t>(half / 2, 1), st);
-        { ProfScope _ps(ctx, "fold"); launch_fold_cols_dev(cols.as<ef>(), nc.as<ef>(), W + 1, half, ph.chs + (round - 1), st,
-                                                      half >= 2 ? eqr.as<ef>() : nullptr, eqn.as<ef>(), half / 2); }
+        { ProfScope _ps(ctx, "fold"); launch_fold_cols_dev(cols.as<ef>(), nc.as<ef>(), ZC_COLS, half, ph.chs + (round - 1), st,
+                                                      half >= 2 ? eqr.as<ef>() : nullptr, eqn.as<ef>(), half / 2, cols2.as<ef>(), ZC0_NQ); }
         cols = std::move(nc);
+        cols2.reset();
         eqr = std::move(eqn);
       }
       const std::vector<ef> ch = ph.finish(&sum, &mmf);
@@ -1233,7 +1236,7 @@ std::vector<uint32_t> prove_air(Context& ctx, const ProofJob& job, const uint32_
       const size_t half = size_t(1) << (m - 1);
       const int nb = zc_ef_blocks(m);
       ef* part = ctx.partials(size_t(nb) * 3);
-      { ProfScope _ps(ctx, zc_eval_is_dense(m) ? "zc_eval_dense" : "zc_eval_ef"); launch_zc_eval_ef(cols.as<ef>(), m, eqr.as<ef>(), d_alphas, d_betas, job.air, part, st); }
+      { ProfScope _ps(ctx, zc_eval_is_dense(m) ? "zc_eval_dense" : "zc_eval_ef"); launch_zc_eval_ef(cols.as<ef>(), cols2.as<ef>(), m, eqr.as<ef>(), d_gammas, job.air, part, st); }
       std::vector<ef> s3 = reduce_to_host(ctx, part, nb, 3);
       const ef& r = zc[round];
       ef e0 = kb::ef_mul(s3[0], mmf), e2 = kb::ef_mul(s3[1], mmf), e3 = kb::ef_mul(s3[2], mmf);
@@ -1247,11 +1250,12 @@ std::vector<uint32_t> prove_air(Context& ctx, const ProofJob& job, const uint32_
       grind(ctx, ts, job.p16, sumcheck_pow_bits(s.security_bits, 4));
       mmf = kb::ef_mul(kb::ef_add(kb::ef_mul(kb::ef_sub(kb::ef_one(), r), kb::ef_sub(kb::ef_one(), c)), kb::ef_mul(r, c)),
                        mmf);
-      DBuf nc(sizeof(ef) * size_t(W + 1) * half, st);
+      DBuf nc(sizeof(ef) * size_t(ZC_COLS) * half, st);
       DBuf eqn(sizeof(ef) * std::max<size_t>(half / 2, 1), st);
-      { ProfScope _ps(ctx, "fold"); launch_fold_cols_at(cols.as<ef>(), nc.as<ef>(), W + 1, half, c, st,
-                                                     half >= 2 ? eqr.as<ef>() : nullptr, eqn.as<ef>(), half / 2); }
+      { ProfScope _ps(ctx, "fold"); launch_fold_cols_at(cols.as<ef>(), nc.as<ef>(), ZC_COLS, half, c, st,
+                                                     half >= 2 ? eqr.as<ef>() : nullptr, eqn.as<ef>(), half / 2, cols2.as<ef>(), ZC0_NQ); }
       cols = std::move(nc);
+      cols2.reset();
       eqr = std::move(eqn);
     }
     // inner sums: every up / down column evaluated at (r_0 over the skipped variables, r_tail)

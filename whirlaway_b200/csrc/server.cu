@@ -20,8 +20,8 @@ double steady_ms() {
 // ones (128 columns; the first of them 2^(n+4+rho-d) rows for an RS domain reduction d, each
 // next one half as many).
 //  * zerocheck: round 0 holds the per-row combination (N values), then either the 52 computed
-//    cube inputs per row or the W + 1 folded columns (N / 2^k values each); round 1 holds the
-//    folded columns and their halves, with the eq tables.
+//    cube inputs per row with their folds (N / 2^k values each) or the folds of all 149 carried
+//    columns; round 1 holds the folded columns and their halves, with the eq tables.
 //  * inner sumcheck: two tables of N values and their halves.
 //  * WHIR: g and the weights (2N values each), their halves, the later commitments.
 // A margin covers the small tables (eq tables, partial sums, query rows, OOD work) and the
@@ -34,8 +34,8 @@ uint64_t proof_footprint_bytes(const Settings& s, int log_n) {
   const uint64_t rows0 = N << (1 + rho);
   const uint64_t c0 = rows0 * 88 * 4 + rows0 * 2 * 32;
   const uint64_t S = N >> k;
-  const uint64_t zc0 = E * N + std::max<uint64_t>(4ull * ZC0_NQ * N, uint64_t(AIR_W + 1) * S * E) + E * S;
-  const uint64_t zc1 = uint64_t(AIR_W + 1) * S * E * 3 / 2 + E * S * 3 / 2;
+  const uint64_t zc0 = E * N + std::max<uint64_t>(4ull * ZC0_NQ * N + uint64_t(ZC0_NQ) * S * E, uint64_t(ZC_COLS) * S * E) + E * S;
+  const uint64_t zc1 = uint64_t(ZC_COLS) * S * E * 3 / 2 + E * S * 3 / 2;
   const uint64_t zc = std::max(zc0, zc1);
   const uint64_t inner = E * (S + 3 * N);
   // later commitments: 2^(n+4+rho-d) rows of 128 columns and a tree (d the RS domain

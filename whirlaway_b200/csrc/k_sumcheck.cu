@@ -118,6 +118,10 @@ __device__ __forceinline__ void cp_async4(uint32_t* smem, const uint32_t* gmem) 
   unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(sa), "l"(gmem));
 }
+__device__ __forceinline__ void cp_async16(uint32_t* smem, const uint32_t* gmem) {  // 16-byte aligned
+  unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem));
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
@@ -149,6 +153,43 @@ __device__ __forceinline__ uint32_t zc0_rc(const AirConsts& K, int i) {
   return 0u;
 }
 
+// The constant operands of k_zc0_eval_mma as its lanes hold them: the Lagrange weights,
+// frags[((mt * 32 + lane) * 4 + b) * 8 + 4 kk + o] = byte b of L_j(z) 2^(8a + 16) in byte a, z = 16 mt + g + 8 (o & 1), j = 8 kk + t + 4 (o >> 1); and the
+// weights gamma, frags[ZC0_FRAG_G + (grp * 32 + lane) * 8 + 2 b + h] = the same of the Montgomery
+// form of 2^(8a) times coefficient g of gamma_i, i = 8 grp + 2t + h (zero past the last input).
+constexpr int ZC0_GRPS = (AIR_NC + 7) / 8;
+constexpr int ZC0_FRAG_G = 2 * 32 * 32;
+static_assert(ZC0_FRAG_G + ZC0_GRPS * 32 * 8 == ZC0_FRAG_WORDS, "operand table");
+template <int E>  // w[b] = byte b of v 2^(8a + E - 32), a = 0..3 (v in Montgomery form)
+__device__ __forceinline__ void limb_columns(uint32_t v, uint32_t (&w)[4]) {
+  uint32_t m[4];
+#pragma unroll
+  for (int a = 0; a < 4; a++) m[a] = kb::mul(v, uint32_t(kb::detail::cpow(2, 8 * a + E)));
+#pragma unroll
+  for (int b = 0; b < 4; b++)
+    w[b] = ((m[0] >> (8 * b)) & 0xffu) | (((m[1] >> (8 * b)) & 0xffu) << 8) | (((m[2] >> (8 * b)) & 0xffu) << 16) |
+           (((m[3] >> (8 * b)) & 0xffu) << 24);
+}
+__device__ void zc0_fragments(int nz, int nsk, const uint32_t* __restrict__ lw, const ef* __restrict__ alphas,
+                              const ef* __restrict__ betas, uint32_t* __restrict__ frags) {
+  for (int e = threadIdx.x; e < 2 * 32 * 8; e += blockDim.x) {
+    const int lane = (e >> 3) & 31, kk = (e >> 2) & 1, o = e & 3;
+    const int z = 16 * (e >> 8) + (lane >> 2) + 8 * (o & 1), j = 8 * kk + (lane & 3) + 4 * (o >> 1);
+    uint32_t w[4];
+    limb_columns<16>(z < nz && j < nsk ? lw[z * nsk + j] : 0u, w);
+#pragma unroll
+    for (int b = 0; b < 4; b++) frags[(e >> 3) * 32 + b * 8 + 4 * kk + o] = w[b];
+  }
+  for (int e = threadIdx.x; e < ZC0_GRPS * 32 * 2; e += blockDim.x) {
+    const int lane = (e >> 1) & 31, i = 8 * (e >> 6) + 2 * (lane & 3) + (e & 1);
+    const ef* gm = i < 64 ? betas + i : i < 84 ? alphas + i : betas + i - 20;
+    uint32_t w[4];
+    limb_columns<32>(i < AIR_NC ? gm->c[lane >> 2] : 0u, w);
+#pragma unroll
+    for (int b = 0; b < 4; b++) frags[ZC0_FRAG_G + (e >> 1) * 8 + 2 * b + (e & 1)] = w[b];
+  }
+}
+
 // One thread per row r = j S + x, reading the row's up row. Writes q[c * N + r]:
 //   c < 16       MDS(inputs)_c + rc_begin[0][c]
 //   16 <= c < 36 state word 0 before partial round c - 16, plus its round constant
@@ -167,9 +208,14 @@ __global__ void __launch_bounds__(ZC0R_THREADS) k_zc0_rows(const uint32_t* __res
                                                            int nz, const uint32_t* __restrict__ lw,
                                                            const ef* __restrict__ eq,
                                                            const ef* __restrict__ alphas_g,
+                                                           const ef* __restrict__ betas_g,
                                                            const __grid_constant__ AirConsts K,
                                                            uint32_t* __restrict__ q, ef* __restrict__ partial,
-                                                           ef* __restrict__ arow) {
+                                                           ef* __restrict__ arow, uint32_t* __restrict__ frags) {
+  if (blockIdx.x == gridDim.x - 1) {
+    zc0_fragments(nz, 1 << k, lw, alphas_g, betas_g, frags);
+    return;
+  }
   __shared__ ef alphas[AIR_NC];
   __shared__ ef scratch[32];
   __shared__ ef total;
@@ -260,182 +306,152 @@ __global__ void __launch_bounds__(ZC0R_THREADS) k_zc0_rows(const uint32_t* __res
 
 // The 148 cube inputs of every row x are extended from their values at rows j S + x, j < 2^k,
 // to the points z by the Lagrange weights L_j(z), cubed, weighted by gamma and summed, weighted
-// by eq[x]. The extension runs on the tensor cores: sum_j L_j(z) v_j(x) is an exact modular
-// dot product over j, computed as a byte-limb integer matrix product whose rows are x, whose
-// reduction index is (j, a) for the 16 points j and the 4 bytes a of v_j(x), and whose
-// columns are (z, b) for the 4 bytes b of M(j, z, a) = the Montgomery form of L_j(z) 2^(8a).
-// The reduction index needs no byte shuffling: the staged words [x][j] are the A operand as
-// they lie (byte a of word j is k = 4j + a). With acc_b = sum_(j,a) v_(j,a) M_b(j, z, a) below
-// 2^22, v = sum_b acc_b 2^(8b) < 2^46 is congruent to (sum_j v_j L_j(z)) R^2, so one Montgomery
-// reduction (with the round constant in the high word) gives the cube input in Montgomery form.
-// A block holds 32 x (two 16-row tiles) and the z-octets of all points; warp (tile, octet)
-// issues 4 n8 tiles (b = 0..3) per k32 step, so each lane ends with all limbs of 4 (x, z)
-// sums, and the B fragments (16 words per lane) depend on z only. The 16 x 32 values of each
-// input are staged in shared memory by a cp.async pipeline, ZC0_GROUP inputs per stage; the
+// by eq[x]. Both contractions run on the tensor cores as byte-limb integer products.
+// Extension: u(z) = sum_j L_j(z) v_j(x) with rows z, reduction index (j, a) over the 16 points j
+// and the 4 bytes a of v_j(x), columns the 8 inputs of a group, one product per byte b of
+// M(j, z, a) = L_j(z) 2^(8a + 16). The staged words [input][j][x] are the B operand as they lie
+// (byte a of word j is k = 4j + a). The accumulators start from the two halves of the round
+// constant times 2^16 (bytes 0 and 2). With acc_b <= 64 255^2 + 2^16, the sum sum_b acc_b 2^(8b) =
+// lo + 2^16 hi, lo and hi below 1.07 10^9, is congruent to 2^16 times the cube input; since
+// p = 1 mod 2^16, dividing by 2^16 takes hi + (lo >> 16) - (lo mod 2^16) (p - 1) / 2^16, which
+// lies in (-p, 1.08 10^9): one small multiply where a Montgomery reduction takes two wide ones.
+// Weights: sum_i gamma_i cube_i with rows z, reduction index (i, a) over the inputs and the bytes
+// of the cube, columns (coefficient n of gamma, byte b). The lane that ends the extension with
+// inputs 2t, 2t + 1 of rows g, g + 8 needs exactly these words as its A operand when k-slot t
+// stands for input 2t and slot t + 4 for 2t + 1, so the cubes never leave their lane; they need
+// not be reduced either (any word congruent to the cube serves, here below 2p).
+// A block holds 8 x and the 32 point slots; warp (z-tile mt, xg) takes x = 2 xg, 2 xg + 1: per
+// group of 8 inputs and x, 8 products for the extension and 4 for the weights. The values are
+// staged by a cp.async pipeline, 8 inputs per stage, a warp per input and 16 bytes per lane;
 // weights of j >= 2^k are zero, so unstaged entries contribute nothing.
-// A block walks 19 groups of inputs one after the other, ~5.5 us each; with too few x blocks to
-// fill the chip (2 an SM) the groups are split over blockIdx.y, each block with its own partial
-// sums: 2^12 rows (8 x blocks) 110 us before, 17 after (19 splits). From 256 x blocks on
-// (2^17 rows) one block keeps all groups.
+// 2^20 rows: 1.23 ms with the weights as 8 multiply-adds per cube on the multiply pipe, 0.94 with
+// both contractions here, 0.88 with the division by 2^16, 0.78 with 16-byte staging (4-byte pieces
+// took a quarter of the instructions); 2^16 rows 0.101 -> 0.064. Bound by latency at 16 warps an SM
+// (the operands held in registers allow no more): 45% of issue slots, multiply pipe 55%.
+// A block walks 19 groups of inputs one after the other; with too few x blocks to fill the chip
+// (2 an SM) the groups are split over blockIdx.y, each block with its own partial sums: 2^12 rows
+// on the multiply pipe 110 us without the split, 17 with it.
 constexpr int ZC0_FILL = 2 * 148;
-constexpr int ZC0M_WARPS = 8;  // 2 x-tiles x 4 z-octets (30 points)
+constexpr int ZC0M_WARPS = 8;
+constexpr int ZE_X = 8;
+constexpr int ZE_IN = 16 * ZE_X + 12;  // words per staged input (8-byte reads of lanes (g, t): every bank twice)
 __global__ void __launch_bounds__(ZC0M_WARPS * 32, 2) k_zc0_eval_mma(const uint32_t* __restrict__ wit,
                                                                     const uint32_t* __restrict__ q, int log_n,
-                                                                    int k, int nz, const uint32_t* __restrict__ lw,
-                                                                    const ef* __restrict__ eq,
-                                                                    const ef* __restrict__ alphas_g,
-                                                                    const ef* __restrict__ betas_g,
+                                                                    int k, int nz, const ef* __restrict__ eq,
+                                                                    const uint32_t* __restrict__ frags,
                                                                     const __grid_constant__ AirConsts K,
                                                                     ef* __restrict__ partial) {
-  __shared__ ef gam[AIR_NC];
-  __shared__ uint32_t rcs[AIR_NC];
-  __shared__ __align__(16) uint32_t tile[ZC0_STAGES][ZC0_GROUP][ZC0_X * ZC0_PAD];
-  __shared__ ef red[4][8];  // per z-octet and point: the sum over the second x-tile
-  constexpr int NT = ZC0M_WARPS * 32;
+  __shared__ __align__(16) uint32_t tile[ZC0_STAGES][8 * ZE_IN];
+  __shared__ ef sums[ZE_X][32];
+  __shared__ int rcs[ZC0_GRPS * 8];  // the round constants times 2^16
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int g = lane >> 2, t = lane & 3, mt = warp & 1, zo = warp >> 1;
-  for (int i = tid; i < AIR_NC; i += NT) {
-    gam[i] = i < 64 ? betas_g[i] : (i < 84 ? alphas_g[i] : betas_g[i - 20]);
-    rcs[i] = zc0_rc(K, i);
-  }
-  const int nsk = 1 << k;
-  const size_t N = size_t(1) << log_n;
-  const size_t S = N >> k;
-  const size_t x0 = size_t(blockIdx.x) * ZC0_X;
-  const bool zwarp = zo * 8 < nz;  // warps of octets past the last point only stage
-
-  // B fragments: bf[b][kk][h] packs, in byte a, byte b of M(j, z, a) for j = 8 kk + 4 h + t
-  // and z = 8 zo + g (the lane's B column)
-  uint32_t bf[4][2][2];
-  {
-    const int z = zo * 8 + g;
+  const int g = lane >> 2, t = lane & 3, mt = warp & 1, xg = warp >> 1;
+  for (int i = tid; i < ZC0_GRPS * 8; i += ZC0M_WARPS * 32) rcs[i] = i < AIR_NC ? int(kb::mul(zc0_rc(K, i), uint32_t(kb::detail::cpow(2, 48)))) : 0;
+  const size_t N = size_t(1) << log_n, S = N >> k;
+  const size_t x0 = size_t(blockIdx.x) * ZE_X;
+  uint32_t af[4][2][4];
 #pragma unroll
-    for (int kk = 0; kk < 2; kk++)
+  for (int b = 0; b < 4; b++)
 #pragma unroll
-      for (int h = 0; h < 2; h++) {
-        const int j = 8 * kk + 4 * h + t;
-        const uint32_t L = (z < nz && j < nsk) ? lw[z * nsk + j] : 0u;
-        uint32_t m[4];
-#pragma unroll
-        for (int a = 0; a < 4; a++) m[a] = kb::mul(L, uint32_t(kb::detail::cpow(2, 8 * a + 32)));
-#pragma unroll
-        for (int b = 0; b < 4; b++)
-          bf[b][kk][h] = ((m[0] >> (8 * b)) & 0xffu) | (((m[1] >> (8 * b)) & 0xffu) << 8) |
-                         (((m[2] >> (8 * b)) & 0xffu) << 16) | (((m[3] >> (8 * b)) & 0xffu) << 24);
-      }
-  }
-
-  // staged entries of this thread: e = tid, tid + NT of the 16 x 32 (j, x) grid; source row
-  // j S + x (the up row for committed columns differs only at row N - 1)
-  constexpr int NE = (16 * ZC0_X + NT - 1) / NT;
-  uint32_t srow[NE], sdst[NE];
-  bool sval[NE], slast[NE];
-#pragma unroll
-  for (int e = 0; e < NE; e++) {
-    const int idx = tid + e * NT;
-    const int j = idx / ZC0_X, xl = idx % ZC0_X;
-    size_t xx = x0 + xl;
-    if (xx >= S) xx = 0;
-    sval[e] = idx < 16 * ZC0_X && j < nsk;
-    srow[e] = uint32_t(size_t(j) * S + xx);
-    slast[e] = size_t(j) * S + xx == N - 1;
-    sdst[e] = uint32_t(xl * ZC0_PAD + j);
-  }
-  constexpr int NG = (AIR_NC + ZC0_GROUP - 1) / ZC0_GROUP;
-  const int per = (NG + gridDim.y - 1) / gridDim.y, g0 = blockIdx.y * per, g1 = min(g0 + per, NG);
+    for (int kk = 0; kk < 2; kk++) {
+      const uint4 v = reinterpret_cast<const uint4*>(frags)[(mt * 32 + lane) * 8 + b * 2 + kk];
+      af[b][kk][0] = v.x;
+      af[b][kk][1] = v.y;
+      af[b][kk][2] = v.z;
+      af[b][kk][3] = v.w;
+    }
+  // staged piece of this thread: x0 + 4 h .. + 3 of row block j of its warp's input of each group;
+  // one by one where the block is cut short or holds row N - 1, whose up row is N - 2 (committed
+  // columns only)
+  const int j = lane >> 1, h = lane & 1;
+  const bool stage = j < (1 << k), whole = x0 + ZE_X <= S && S % 4 == 0;
+  const size_t row = size_t(j) * S + x0 + 4 * h;
+  const int per = (ZC0_GRPS + gridDim.y - 1) / gridDim.y, g0 = blockIdx.y * per, g1 = min(g0 + per, ZC0_GRPS);
   auto issue = [&](int grp) {
-#pragma unroll
-    for (int cc = 0; cc < ZC0_GROUP; cc++) {
-      const int i = ZC0_GROUP * grp + cc;
-      if (i < AIR_NC && grp < g1) {
-        const int qc = zc0_qcol(i);
-        const uint32_t* col = qc >= 0 ? q + size_t(qc) * N : wit + size_t(1 + i) * N;
-        uint32_t* dst = tile[grp % ZC0_STAGES][cc];
-#pragma unroll
-        for (int e = 0; e < NE; e++)
-          if (sval[e]) cp_async4(dst + sdst[e], col + (srow[e] - uint32_t(slast[e] && qc < 0)));
+    const int i = 8 * grp + warp;
+    if (stage && i < AIR_NC && grp < g1) {
+      const int qc = zc0_qcol(i);
+      const uint32_t* col = qc >= 0 ? q + size_t(qc) * N : wit + size_t(1 + i) * N;
+      uint32_t* dst = tile[grp % ZC0_STAGES] + warp * ZE_IN + j * ZE_X + 4 * h;
+      if (whole && (qc >= 0 || row + 4 != N)) {
+        cp_async16(dst, col + row);
+      } else {
+        for (int e = 0; e < 4; e++) {
+          const size_t r = row + e;
+          if (x0 + 4 * h + e < S) cp_async4(dst + e, col + (r == N - 1 && qc < 0 ? N - 2 : r));
+        }
       }
     }
     cp_async_commit();
   };
   for (int grp = g0; grp < g0 + ZC0_STAGES - 1; grp++) issue(grp);
-  EfMacF m[4];  // (x, z) = (g, 2t), (g, 2t + 1), (g + 8, 2t), (g + 8, 2t + 1) of the warp's tile
+  int acc2[2][4][4];
 #pragma unroll
-  for (int o = 0; o < 4; o++) m[o].init();
-  static_assert(ZC0_GROUP % 4 == 0 && AIR_NC % 4 == 0, "flushes after every 4 products");
+  for (int xq = 0; xq < 2; xq++)
+#pragma unroll
+    for (int b = 0; b < 4; b++)
+#pragma unroll
+      for (int o = 0; o < 4; o++) acc2[xq][b][o] = 0;
 #pragma unroll 1
   for (int grp = g0; grp < g1; grp++) {
+    const uint4* gf = reinterpret_cast<const uint4*>(frags + ZC0_FRAG_G) + (grp * 32 + lane) * 2;
+    const uint4 gl = __ldg(gf), gh = __ldg(gf + 1);
+    const uint32_t gb[4][2] = {{gl.x, gl.y}, {gl.z, gl.w}, {gh.x, gh.y}, {gh.z, gh.w}};
     cp_async_wait<ZC0_STAGES - 2>();
     __syncthreads();  // group grp landed for every thread; the slot of group grp - 1 is free
     issue(grp + ZC0_STAGES - 1);
-    if (zwarp) {
-#pragma unroll 2
-      for (int cc = 0; cc < ZC0_GROUP; cc++) {
-        const int i = ZC0_GROUP * grp + cc;
-        if (i >= AIR_NC) break;  // the last group is partial
-        const uint32_t* r0 = tile[grp % ZC0_STAGES][cc] + (16 * mt + g) * ZC0_PAD;
-        const uint32_t* r1 = r0 + 8 * ZC0_PAD;
-        int acc[4][4];
+    const int rc[2] = {rcs[8 * grp + 2 * t], rcs[8 * grp + 2 * t + 1]};
+    uint2 vw[4];  // words j = t, t + 4, t + 8, t + 12 of input g at the warp's two x
 #pragma unroll
-        for (int b = 0; b < 4; b++)
+    for (int e = 0; e < 4; e++)
+      vw[e] = *reinterpret_cast<const uint2*>(tile[grp % ZC0_STAGES] + g * ZE_IN + (t + 4 * e) * ZE_X + 2 * xg);
 #pragma unroll
-          for (int o = 0; o < 4; o++) acc[b][o] = 0;
+    for (int xq = 0; xq < 2; xq++) {
+      const uint32_t v0 = xq ? vw[0].y : vw[0].x, v1 = xq ? vw[1].y : vw[1].x;
+      const uint32_t v2 = xq ? vw[2].y : vw[2].x, v3 = xq ? vw[3].y : vw[3].x;
+      int acc[4][4];
 #pragma unroll
-        for (int kk = 0; kk < 2; kk++) {
-          const uint32_t af[4] = {r0[8 * kk + t], r1[8 * kk + t], r0[8 * kk + t + 4], r1[8 * kk + t + 4]};
-#pragma unroll
-          for (int b = 0; b < 4; b++) mma_u8_16832(acc[b], af, bf[b][kk][0], bf[b][kk][1]);
-        }
-        const uint64_t rc_hi = uint64_t(rcs[i]) << 32;
-        const ef& gm = gam[i];
-#pragma unroll
-        for (int o = 0; o < 4; o++) {
-          const uint32_t lo = uint32_t(acc[0][o]) + (uint32_t(acc[1][o]) << 8);  // < 2^31
-          const uint32_t hi = uint32_t(acc[2][o]) + (uint32_t(acc[3][o]) << 8);  // < 2^31
-          const uint32_t u = kb::redc(uint64_t(lo) + (uint64_t(hi) << 16) + rc_hi);
-          m[o].mac(gm, kb::cube(u));
-        }
-        if ((cc & 3) == 3) {
-#pragma unroll
-          for (int o = 0; o < 4; o++) m[o].flush();
-        }
+      for (int b = 0; b < 4; b++) {
+        const int r0 = b == 0 ? rc[0] & 0xffff : b == 2 ? rc[0] >> 16 : 0;
+        const int r1 = b == 0 ? rc[1] & 0xffff : b == 2 ? rc[1] >> 16 : 0;
+        mma_u8_16832_from(acc[b], af[b][0], v0, v1, r0, r1, r0, r1);
+        mma_u8_16832_from(acc[b], af[b][1], v2, v3, acc[b][0], acc[b][1], acc[b][2], acc[b][3]);
       }
+      uint32_t w[4];  // (z, input) = (g, 2t), (g, 2t + 1), (g + 8, 2t), (g + 8, 2t + 1)
+#pragma unroll
+      for (int o = 0; o < 4; o++) {
+        const uint32_t lo = uint32_t(acc[0][o]) + (uint32_t(acc[1][o]) << 8);
+        const uint32_t hi = uint32_t(acc[2][o]) + (uint32_t(acc[3][o]) << 8);
+        const uint32_t r = hi + (lo >> 16) + kb::P - (lo & 0xffffu) * ((kb::P - 1) >> 16);
+        const uint32_t u = kb::umin(r, r - kb::P);
+        w[o] = kb::mul_lazy(kb::mul_lazy(u, u), u);
+      }
+      const uint32_t ca[4] = {w[0], w[2], w[1], w[3]};
+#pragma unroll
+      for (int b = 0; b < 4; b++)
+        mma_u8_16832_from(acc2[xq][b], ca, gb[b][0], gb[b][1], acc2[xq][b][0], acc2[xq][b][1], acc2[xq][b][2],
+                          acc2[xq][b][3]);
     }
   }
   cp_async_wait<0>();
-  // weight by eq[x], sum over the 16 x of the tile (lanes of equal t), then over the two tiles
-  ef sz[2];
+  // lane (g, t) holds coefficients 2t, 2t + 1 of rows z = 16 mt + g and + 8 (acc2 < 2^26 each)
 #pragma unroll
-  for (int c = 0; c < 2; c++) {
-    ef acc = ef_zero();
+  for (int xq = 0; xq < 2; xq++)
 #pragma unroll
-    for (int hh = 0; hh < 2; hh++) {
-      const size_t x = x0 + 16 * mt + g + 8 * hh;
-      const ef v = m[2 * hh + c].value();
-      if (zwarp && x < S) acc = ef_add(acc, ef_mul(v, eq[x]));
-    }
-#pragma unroll
-    for (int d = 4; d < 32; d <<= 1) {
-      ef o;
-#pragma unroll
-      for (int w = 0; w < 8; w++) o.c[w] = __shfl_xor_sync(0xffffffffu, acc.c[w], d);
-      acc = ef_add(acc, o);
-    }
-    sz[c] = acc;
-  }
-  if (mt == 1 && g == 0) {
-    red[zo][2 * t] = sz[0];
-    red[zo][2 * t + 1] = sz[1];
-  }
+    for (int o = 0; o < 4; o++)
+      sums[2 * xg + xq][16 * mt + g + 8 * (o >> 1)].c[2 * t + (o & 1)] =
+          kb::redc(uint64_t(uint32_t(acc2[xq][0][o])) + (uint64_t(uint32_t(acc2[xq][1][o])) << 8) +
+                   (uint64_t(uint32_t(acc2[xq][2][o])) << 16) + (uint64_t(uint32_t(acc2[xq][3][o])) << 24));
   __syncthreads();
-  if (mt == 0 && g == 0) {
+  if (x0 + warp < S) sums[warp][lane] = ef_mul(sums[warp][lane], eq[x0 + warp]);
+  else sums[warp][lane] = ef_zero();
+  __syncthreads();
+  const int z = tid >> 3, n = tid & 7;
+  if (z >= nz) return;
+  uint32_t s = 0;
 #pragma unroll
-    for (int c = 0; c < 2; c++) {
-      const int z = zo * 8 + 2 * t + c;
-      if (z < nz)
-        partial[(size_t(blockIdx.y) * gridDim.x + blockIdx.x) * nz + z] = ef_add(sz[c], red[zo][2 * t + c]);
-    }
-  }
+  for (int x = 0; x < ZE_X; x++) s = add(s, sums[x][z].c[n]);
+  partial[(size_t(blockIdx.y) * gridDim.x + blockIdx.x) * nz + z].c[n] = s;
 }
 
 // out[x] = sum_j sel[j] * a[j S + x] for the block's 32 x of an extension-field table a that is
@@ -1921,19 +1937,18 @@ void launch_reduce_partials(const ef* partial, int nblk, int k, ef* out, cudaStr
   WL_LAUNCH_CHECK();
 }
 
-static int zc0_tiles(int log_n, int k) {  // blocks of 32 x
+static int zc0_tiles(int log_n, int k, int xs) {  // blocks of xs x
   size_t S = size_t(1) << (log_n - k);
-  return (int)((S + ZC0_X - 1) / ZC0_X);
+  return (int)((S + xs - 1) / xs);
 }
 static int zc0_splits(int tiles, int groups) {
   const int want = std::min(std::max(ZC0_FILL / tiles, 1), groups);
   const int per = (groups + want - 1) / want;
   return (groups + per - 1) / per;  // no empty range
 }
-static int zc0_eval_splits(int tiles) { return zc0_splits(tiles, (AIR_NC + ZC0_GROUP - 1) / ZC0_GROUP); }
 int zc0_blocks(int log_n, int k) {
-  const int tiles = zc0_tiles(log_n, k);
-  return tiles * zc0_eval_splits(tiles);
+  const int tiles = zc0_tiles(log_n, k, ZE_X);
+  return tiles * zc0_splits(tiles, ZC0_GRPS);
 }
 static int zc0_row_threads(int log_n) { return (size_t(1) << log_n) < size_t(148) * ZC0R_THREADS ? ZC0R_SMALL : ZC0R_THREADS; }
 int zc0_row_blocks(int log_n) {
@@ -1941,25 +1956,26 @@ int zc0_row_blocks(int log_n) {
   return (int)(((size_t(1) << log_n) + t - 1) / t);
 }
 void launch_zc0_rows(const uint32_t* wit, int log_n, int k, int nz, const uint32_t* lw, const ef* eq,
-                     const ef* alphas, const AirConsts& K, uint32_t* q, ef* partial, ef* arow, cudaStream_t s) {
-  k_zc0_rows<<<zc0_row_blocks(log_n), zc0_row_threads(log_n), 0, s>>>(wit, log_n, k, nz, lw, eq, alphas, K, q,
-                                                                      partial, arow);
+                     const ef* alphas, const ef* betas, const AirConsts& K, uint32_t* q, ef* partial, ef* arow,
+                     cudaStream_t s) {
+  if (nz > 32) throw std::invalid_argument("zc0_rows: at most 32 points");
+  k_zc0_rows<<<zc0_row_blocks(log_n) + 1, zc0_row_threads(log_n), 0, s>>>(
+      wit, log_n, k, nz, lw, eq, alphas, betas, K, q, partial, arow, q + (size_t(ZC0_NQ) << log_n));
   WL_LAUNCH_CHECK();
 }
-void launch_zc0_eval(const uint32_t* wit, const uint32_t* q, int log_n, int k, int nz, const uint32_t* lw,
-                     const ef* eq, const ef* alphas, const ef* betas, const AirConsts& K, ef* partial,
-                     cudaStream_t s) {
+void launch_zc0_eval(const uint32_t* wit, const uint32_t* q, int log_n, int k, int nz, const ef* eq,
+                     const AirConsts& K, ef* partial, cudaStream_t s) {
   if (nz > 32) throw std::invalid_argument("zc0_eval: at most 32 points");
-  const int tiles = zc0_tiles(log_n, k);
-  k_zc0_eval_mma<<<dim3(tiles, zc0_eval_splits(tiles)), ZC0M_WARPS * 32, 0, s>>>(wit, q, log_n, k, nz, lw, eq,
-                                                                                 alphas, betas, K, partial);
+  const int tiles = zc0_tiles(log_n, k, ZE_X);
+  k_zc0_eval_mma<<<dim3(tiles, zc0_splits(tiles, ZC0_GRPS)), ZC0M_WARPS * 32, 0, s>>>(
+      wit, q, log_n, k, nz, eq, q + (size_t(ZC0_NQ) << log_n), K, partial);
   WL_LAUNCH_CHECK();
 }
 void launch_zc0_fold(const uint32_t* src, int log_n, int k, int cb, int ce, const ef* sel, const ef* arow, ef* out,
                      cudaStream_t s) {
   size_t S = size_t(1) << (log_n - k);
   if (S < 2) throw std::invalid_argument("zc0_fold: at least 2 points per skip block");
-  const int tiles = zc0_tiles(log_n, k), splits = zc0_splits(tiles, (ce - cb + ZC0_GROUP - 1) / ZC0_GROUP);
+  const int tiles = zc0_tiles(log_n, k, ZC0_X), splits = zc0_splits(tiles, (ce - cb + ZC0_GROUP - 1) / ZC0_GROUP);
   k_zc0_fold_mma<<<dim3(tiles, splits + (arow ? 1 : 0)), ZC0M_WARPS * 32, 0, s>>>(src, log_n, k, cb, ce, sel, arow,
                                                                                  out);
   WL_LAUNCH_CHECK();

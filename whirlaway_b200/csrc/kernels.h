@@ -100,17 +100,19 @@ void launch_reduce_partials(const ef* partial, int nblk, int k, ef* out, cudaStr
 // Round 0 with univariate skip over the top k variables: for the nz points z_0.. given by
 // their Lagrange weights lw[z * 2^k + j], the eq-weighted batched constraint over the up
 // columns, as partial sums partial[blk * nz + z] of two kernels. launch_zc0_rows writes the
-// ZC0_NQ computed cube inputs of every row to q (ZC0_NQ * 2^log_n words) and its
-// zc0_row_blocks partial sums (the committed-column term); launch_zc0_eval reads q and writes
-// zc0_blocks partial sums (the S-box term). The point sums are the sums over both.
+// ZC0_NQ computed cube inputs of every row to q (ZC0_NQ * 2^log_n words, then ZC0_FRAG_WORDS of
+// operand tables) and its zc0_row_blocks partial sums (the committed-column term);
+// launch_zc0_eval reads q and writes zc0_blocks partial sums (the S-box term). The point sums
+// are the sums over both.
 constexpr int ZC0_NQ = 52;
+constexpr int ZC0_FRAG_WORDS = 2 * 32 * 32 + 19 * 32 * 8;
 int zc0_blocks(int log_n, int k);
 int zc0_row_blocks(int log_n);
 void launch_zc0_rows(const uint32_t* wit, int log_n, int k, int nz, const uint32_t* lw, const ef* eq,
-                     const ef* alphas, const AirConsts& K, uint32_t* q, ef* partial, ef* arow, cudaStream_t s);
-void launch_zc0_eval(const uint32_t* wit, const uint32_t* q, int log_n, int k, int nz, const uint32_t* lw,
-                     const ef* eq, const ef* alphas, const ef* betas, const AirConsts& K, ef* partial,
+                     const ef* alphas, const ef* betas, const AirConsts& K, uint32_t* q, ef* partial, ef* arow,
                      cudaStream_t s);
+void launch_zc0_eval(const uint32_t* wit, const uint32_t* q, int log_n, int k, int nz, const ef* eq,
+                     const AirConsts& K, ef* partial, cudaStream_t s);
 // Round-0 fold of the cube inputs cb <= c < ce of the carried columns: out[(c - cb) 2^(log_n-k) + x]
 // = sum_j sel[j] v_c[j 2^(log_n-k) + x], from src = launch_zc0_rows' q (ce <= ZC0_NQ) or src = the
 // witness (cb >= ZC0_NQ); with arow (2^log_n EF, one per row) its fold is column ce.

@@ -17,6 +17,13 @@ __device__ __forceinline__ void mma_u8_16832(int (&c)[4], const uint32_t (&a)[4]
       : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+// The same as c = c0 + a b, free to move among other instructions.
+__device__ __forceinline__ void mma_u8_16832_from(int (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, int c0,
+                                                  int c1, int c2, int c3) {
+  asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.u8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};\n"
+      : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(c0), "r"(c1), "r"(c2), "r"(c3));
+}
 // Byte a of four consecutive values, packed (limb a of a k-quad of the A fragment).
 __device__ __forceinline__ void byte_transpose4(const uint4 q, uint32_t (&r)[4]) {
   const uint32_t p01l = __byte_perm(q.x, q.y, 0x5140), p01h = __byte_perm(q.x, q.y, 0x7362);

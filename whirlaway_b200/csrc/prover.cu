@@ -1170,13 +1170,13 @@ std::vector<uint32_t> prove_air(Context& ctx, const ProofJob& job, const uint32_
     // ones in `cols` and the others in `cols2`, so that q is gone before the second is allocated
     DBuf cols, cols2;
     // the committed-column combination sum_i alpha_i col_(17+i) of every row
-    DBuf arow(sizeof(ef) * N, st), q(sizeof(uint32_t) * ZC0_NQ * N, st);
+    DBuf arow(sizeof(ef) * N, st), q(sizeof(uint32_t) * (ZC0_NQ * N + ZC0_FRAG_WORDS), st);
     {
       const uint32_t* d_lw = up.at<uint32_t>(il);
       const int nb = zc0_blocks(n, k), nbr = zc0_row_blocks(n);
       ef* part = ctx.partials(size_t(nb + nbr) * nz);
-      { ProfScope _ps(ctx, "zc0_rows"); launch_zc0_rows(wit, n, k, nz, d_lw, eq0.as<ef>(), d_alphas, job.air, q.as<uint32_t>(), part + size_t(nb) * nz, arow.as<ef>(), st); }
-      { ProfScope _ps(ctx, "zc0_eval"); launch_zc0_eval(wit, q.as<uint32_t>(), n, k, nz, d_lw, eq0.as<ef>(), d_alphas, d_betas, job.air, part, st); }
+      { ProfScope _ps(ctx, "zc0_rows"); launch_zc0_rows(wit, n, k, nz, d_lw, eq0.as<ef>(), d_alphas, d_betas, job.air, q.as<uint32_t>(), part + size_t(nb) * nz, arow.as<ef>(), st); }
+      { ProfScope _ps(ctx, "zc0_eval"); launch_zc0_eval(wit, q.as<uint32_t>(), n, k, nz, eq0.as<ef>(), job.air, part, st); }
       std::vector<ef> sums = reduce_to_host(ctx, part, nb + nbr, nz);
       std::vector<ef> ys(nsk, kb::ef_zero());
       ys.insert(ys.end(), sums.begin(), sums.end());

@@ -738,18 +738,20 @@ __global__ void __launch_bounds__(256) k_fold_cols_mma(ZcCols in, ef* __restrict
                                                       size_t eq_half) {
   const int c = blockIdx.y;
   if (c == ncols) {
-    const size_t x = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (x < eq_half) eq_out[x] = ef_add(eq_in[x], eq_in[x + eq_half]);
+    for (size_t x = size_t(blockIdx.x) * blockDim.x + threadIdx.x; x < eq_half; x += size_t(gridDim.x) * blockDim.x)
+      eq_out[x] = ef_add(eq_in[x], eq_in[x + eq_half]);
     return;
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-  const size_t x0 = (size_t(blockIdx.x) * 8 + warp) * 16;
+  size_t x0 = (size_t(blockIdx.x) * 8 + warp) * 16;
   if (x0 >= half) return;  // whole warp
   uint32_t bf[4][2];
   fold_frag(rptr ? *rptr : rv, g, t, bf);
   const ef* src = in.col(c, 2 * half);
-  const uint32_t nv = half - x0 < 16 ? uint32_t(half - x0) : 16u;
-  lerp16_mma(src + x0, src + half + x0, out + size_t(c) * half + x0, nv, bf, g, t);
+  for (; x0 < half; x0 += size_t(gridDim.x) * 128) {
+    const uint32_t nv = half - x0 < 16 ? uint32_t(half - x0) : 16u;
+    lerp16_mma(src + x0, src + half + x0, out + size_t(c) * half + x0, nv, bf, g, t);
+  }
 }
 // lo + r (hi - lo) for two tables with the challenge by value: blockIdx.y selects (a, oa) or (b, ob).
 __global__ void __launch_bounds__(256) k_fold2_mma(const ef* __restrict__ a, const ef* __restrict__ b,
@@ -2020,18 +2022,24 @@ void launch_fold_cols(const ef* in, ef* out, int ncols, size_t half, const ef* r
   k_fold_cols<<<grid, 256, 0, s>>>(in, out, half, ncols, r, ef_zero(), eq_in, eq_out, eq_half);
   WL_LAUNCH_CHECK();
 }
+// 128 values of a column at a time per block; a block of a large table goes on to further ones (up
+// to FOLD_TILES) while at least FOLD_FILL blocks are left, as forming the challenge's operand costs
+// a warp about as much as a tile: the folds of 2^20 rows 0.40 ms with one tile a block, 0.32 so.
+constexpr size_t FOLD_TILES = 8, FOLD_FILL = 8 * 148;
+static dim3 fold_cols_grid(int ncols, size_t half, bool eq) {
+  const size_t tiles = std::max<size_t>((half + 127) / 128, 1);
+  const size_t per = std::min(std::max<size_t>(tiles * size_t(ncols) / FOLD_FILL, 1), FOLD_TILES);
+  return dim3((unsigned)((tiles + per - 1) / per), ncols + (eq ? 1 : 0));
+}
 void launch_fold_cols_at(const ef* in, ef* out, int ncols, size_t half, const ef& r, cudaStream_t s, const ef* eq_in,
                          ef* eq_out, size_t eq_half, const ef* in2, int split) {
-  // 128 values per block for the columns, 256 for the eq table
-  const size_t bx = std::max((half + 127) / 128, eq_in ? (eq_half + 255) / 256 : size_t(0));
-  dim3 grid((unsigned)std::max<size_t>(bx, 1), ncols + (eq_in ? 1 : 0));
+  const dim3 grid = fold_cols_grid(ncols, half, eq_in != nullptr);
   k_fold_cols_mma<<<grid, 256, 0, s>>>(ZcCols{in, in2, in2 ? split : ncols}, out, half, ncols, r, nullptr, eq_in, eq_out, eq_half);
   WL_LAUNCH_CHECK();
 }
 void launch_fold_cols_dev(const ef* in, ef* out, int ncols, size_t half, const ef* r_dev, cudaStream_t s,
                           const ef* eq_in, ef* eq_out, size_t eq_half, const ef* in2, int split) {
-  const size_t bx = std::max((half + 127) / 128, eq_in ? (eq_half + 255) / 256 : size_t(0));
-  dim3 grid((unsigned)std::max<size_t>(bx, 1), ncols + (eq_in ? 1 : 0));
+  const dim3 grid = fold_cols_grid(ncols, half, eq_in != nullptr);
   k_fold_cols_mma<<<grid, 256, 0, s>>>(ZcCols{in, in2, in2 ? split : ncols}, out, half, ncols, ef_zero(), r_dev, eq_in, eq_out, eq_half);
   WL_LAUNCH_CHECK();
 }

@@ -234,94 +234,111 @@ __global__ void k_add_eq_terms_f(ef* __restrict__ w, int lh, int ll, int npts, c
   w[v] = m.value();
 }
 
-// The same on the tensor cores (byte-limb matrix products): the block's rows share v_hi,
-// so B[t][n] = coefficient n of coefs[t] hi_t[v_hi] (its limbs in shared memory,
-// bs[(b * 8 + n) * Kp + t]); each warp's 16 rows v_lo read lo_t[v_lo] (consecutive rows are
-// consecutive words) and own all 16 limb pairs, so every accumulator position is recombined
-// by the lane that holds it.
+// The same on the tensor cores as byte-limb products: rows v_lo, reduction index (t, byte of
+// lo_t[v_lo]) (the table's words as they lie), columns (coefficient n, byte b) of the Montgomery
+// form of coefs[t] hi_t[v_hi] 2^(8a), a the row's byte. The block's rows share v_hi, so that operand
+// is formed once per block, in shared memory as the lanes read it (bs[(step * 32 + lane) * 8 + 2 b +
+// h], 8 points a step). It costs a block about as much as one 16-row tile costs a warp, so a block
+// takes AEQ_ROWS rows where the table fills the chip twice with them. Bound by issue (loads, the
+// reductions) at about 4 products per 8 points: 112 points on 2^21 entries 0.38 ms with 16 products
+// of separate limb pairs per 32 points and 128 rows a block, 0.27 here.
 constexpr int AEQ_WARPS = 8;
-constexpr int AEQ_MAX_K = 1024;
+constexpr uint32_t AEQ_ROWS = 1024, AEQ_MIN_ROWS = 128;
+constexpr int AEQ_MAX_K = 352;  // points a launch (44 KB of operands)
 __global__ void __launch_bounds__(AEQ_WARPS * 32) k_add_eq_terms_f_mma(ef* __restrict__ w, int lh, int ll, int npts,
-                                                                      int Kp, const uint32_t* __restrict__ hi,
+                                                                      uint32_t rows, const uint32_t* __restrict__ hi,
                                                                       const uint32_t* __restrict__ lo,
                                                                       const ef* __restrict__ coefs) {
-  extern __shared__ __align__(16) uint8_t bs[];
+  extern __shared__ __align__(16) uint32_t bs[];
   const uint32_t nhi = 1u << lh, nlo = 1u << ll;
-  const uint32_t rows = nlo < AEQ_WARPS * 16 ? nlo : AEQ_WARPS * 16;  // one 16-row tile per warp
   const uint32_t per_vh = nlo / rows;
   const uint32_t vh = blockIdx.x / per_vh, xl0 = (blockIdx.x % per_vh) * rows;
-  for (int idx = threadIdx.x; idx < 8 * Kp; idx += blockDim.x) {
-    const int n = idx / Kp, t = idx - n * Kp;
-    const uint32_t v = t < npts ? mul(coefs[t].c[n], hi[size_t(t) * nhi + vh]) : 0u;
+  const int steps = (npts + 7) / 8;
+#pragma unroll 4
+  for (int idx = threadIdx.x; idx < steps * 64; idx += AEQ_WARPS * 32) {  // (point, coefficient)
+    const int n = idx & 7, k = idx >> 3;
+    const uint32_t v = k < npts ? mul(coefs[k].c[n], hi[size_t(k) * nhi + vh]) : 0u;
+    uint32_t m[4];
 #pragma unroll
-    for (int b = 0; b < 4; b++) bs[(b * 8 + n) * Kp + t] = uint8_t(v >> (8 * b));
+    for (int a = 0; a < 4; a++) m[a] = mul(v, uint32_t(kb::detail::cpow(2, 8 * a + 32)));
+    uint32_t* d = bs + ((k >> 3) * 32 + n * 4 + (k & 3)) * 8 + ((k >> 2) & 1);
+#pragma unroll
+    for (int b = 0; b < 4; b++)
+      d[2 * b] = ((m[0] >> (8 * b)) & 0xffu) | (((m[1] >> (8 * b)) & 0xffu) << 8) | (((m[2] >> (8 * b)) & 0xffu) << 16) |
+                 (((m[3] >> (8 * b)) & 0xffu) << 24);
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, t = lane & 3;
   for (uint32_t x0 = xl0 + uint32_t(warp) * 16; x0 < xl0 + rows; x0 += AEQ_WARPS * 16) {  // no barrier in here
     const uint32_t xa = x0 + g, xb = xa + 8;
-    int acc[4][4][4];
+    int acc[4][4];
 #pragma unroll
-    for (int a = 0; a < 4; a++)
+    for (int b = 0; b < 4; b++)
 #pragma unroll
-      for (int b = 0; b < 4; b++)
-#pragma unroll
-        for (int q = 0; q < 4; q++) acc[a][b][q] = 0;
-    auto ld = [&](int k, uint32_t x) -> uint32_t { return k < npts ? __ldg(lo + size_t(k) * nlo + x) : 0u; };
-    // the next step's values are requested before this step's products (two steps in flight)
-    auto load_step = [&](int k0, uint4 (&q)[4]) {
-#pragma unroll
-      for (int h = 0; h < 2; h++) {
-        const int kb0 = k0 + 16 * h + 4 * t;
-        q[2 * h] = make_uint4(ld(kb0, xa), ld(kb0 + 1, xa), ld(kb0 + 2, xa), ld(kb0 + 3, xa));
-        q[2 * h + 1] = make_uint4(ld(kb0, xb), ld(kb0 + 1, xb), ld(kb0 + 2, xb), ld(kb0 + 3, xb));
-      }
+      for (int q = 0; q < 4; q++) acc[b][q] = 0;
+    auto load = [&](int s, uint32_t (&q)[4]) {  // points past the last have zero weights
+      const uint32_t* r0 = lo + size_t(min(8 * s + t, npts - 1)) * nlo;
+      const uint32_t* r1 = lo + size_t(min(8 * s + t + 4, npts - 1)) * nlo;
+      q[0] = __ldg(r0 + xa);
+      q[1] = __ldg(r0 + xb);
+      q[2] = __ldg(r1 + xa);
+      q[3] = __ldg(r1 + xb);
     };
-    uint4 nq[4];
-    load_step(0, nq);
-#pragma unroll 1
-    for (int k0 = 0; k0 < Kp; k0 += 32) {
-      uint4 q[4];
-#pragma unroll
-      for (int i = 0; i < 4; i++) q[i] = nq[i];
-      if (k0 + 32 < Kp) load_step(k0 + 32, nq);
-      uint32_t l[4][4];
-#pragma unroll
-      for (int i = 0; i < 4; i++) byte_transpose4(q[i], l[i]);
-#pragma unroll
-      for (int b = 0; b < 4; b++) {
-        const uint32_t* col = reinterpret_cast<const uint32_t*>(bs + (b * 8 + g) * Kp + k0) + t;
-        const uint32_t b0 = col[0], b1 = col[4];
-#pragma unroll
-        for (int a = 0; a < 4; a++) {
-          const uint32_t af[4] = {l[0][a], l[1][a], l[2][a], l[3][a]};
-          mma_u8_16832(acc[a][b], af, b0, b1);
-        }
-      }
+    uint32_t nq[4];
+    load(0, nq);
+#pragma unroll 2
+    for (int s = 0; s < steps; s++) {
+      const uint32_t af[4] = {nq[0], nq[1], nq[2], nq[3]};
+      if (s + 1 < steps) load(s + 1, nq);
+      const uint4* f = reinterpret_cast<const uint4*>(bs) + (s * 32 + lane) * 2;
+      const uint4 f0 = f[0], f1 = f[1];
+      mma_u8_16832(acc[0], af, f0.x, f0.y);
+      mma_u8_16832(acc[1], af, f0.z, f0.w);
+      mma_u8_16832(acc[2], af, f1.x, f1.y);
+      mma_u8_16832(acc[3], af, f1.z, f1.w);
     }
     // lane (g, t) holds coefficients 2t, 2t + 1 of rows xa (q = 0, 1) and xb (q = 2, 3)
+    auto val = [&](int q) {
+      return kb::redc(uint64_t(uint32_t(acc[0][q])) + (uint64_t(uint32_t(acc[1][q])) << 8) +
+                      (uint64_t(uint32_t(acc[2][q])) << 16) + (uint64_t(uint32_t(acc[3][q])) << 24));
+    };
     uint2* pa = reinterpret_cast<uint2*>(w + (size_t(vh) << ll) + xa) + t;
     uint2* pb = reinterpret_cast<uint2*>(w + (size_t(vh) << ll) + xb) + t;
     const uint2 oa = *pa, ob = *pb;
-    *pa = make_uint2(add(oa.x, limb_recombine_lane(acc, 0)), add(oa.y, limb_recombine_lane(acc, 1)));
-    *pb = make_uint2(add(ob.x, limb_recombine_lane(acc, 2)), add(ob.y, limb_recombine_lane(acc, 3)));
+    *pa = make_uint2(add(oa.x, val(0)), add(oa.y, val(1)));
+    *pb = make_uint2(add(ob.x, val(2)), add(ob.y, val(3)));
   }
 }
 
-// w[v] += sum_t coefs[t] * hi_t[v_hi] * lo_t[v_lo]   (extension-field points)
+// w[v] += sum_t coefs[t] * hi_t[v_hi] * lo_t[v_lo]   (extension-field points). A block's entries
+// share v_hi: a_t = coefs[t] hi_t[v_hi] and 3 a_t are formed once per block, and an entry's terms
+// a_t lo_t[v_lo] are one sum with a single reduction. Bound by the wide multiplies, 80 per term
+// (128 and two reductions per coefficient with both products per entry).
 struct AddEqCoefs {
   ef c[ADD_EQ_MAX];
 };
-__global__ void k_add_eq_terms_ef(ef* __restrict__ w, int lh, int ll, int npts, const ef* __restrict__ hi,
-                                  const ef* __restrict__ lo, const __grid_constant__ AddEqCoefs coefs) {
-  const size_t v = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (v >= (size_t(1) << (lh + ll))) return;
-  const size_t vh = v >> ll, vl = v & ((size_t(1) << ll) - 1);
+constexpr int AEE_THREADS = 256;
+__global__ void __launch_bounds__(AEE_THREADS) k_add_eq_terms_ef(ef* __restrict__ w, int lh, int ll, int npts, int per,
+                                                                const ef* __restrict__ hi, const ef* __restrict__ lo,
+                                                                const __grid_constant__ AddEqCoefs coefs) {
+  __shared__ __align__(16) ef a[ADD_EQ_MAX][2];
   const size_t nhi = size_t(1) << lh, nlo = size_t(1) << ll;
-  ef acc = w[v];
-  for (int t = 0; t < npts; t++) acc = ef_add(acc, ef_mul(ef_mul(coefs.c[t], hi[t * nhi + vh]), lo[t * nlo + vl]));
-  w[v] = acc;
+  const size_t v0 = size_t(blockIdx.x) * blockDim.x * per;
+  for (int t = threadIdx.x; t < npts; t += blockDim.x) {
+    const ef v = ef_mul(coefs.c[t], hi[t * nhi + (v0 >> ll)]);
+    a[t][0] = v;
+    a[t][1] = ef_add(ef_add(v, v), v);
+  }
+  __syncthreads();
+  for (int i = 0; i < per; i++) {
+    const size_t v = v0 + size_t(i) * blockDim.x + threadIdx.x, vl = v & (nlo - 1);
+    EfMacE m;
+    m.init();
+#pragma unroll 1
+    for (int t = 0; t < npts; t++) m.mac3(lo[t * nlo + vl], a[t][0], a[t][1]);
+    w[v] = ef_add(w[v], m.value());
+  }
 }
 
 constexpr int WSC_THREADS = 256;
@@ -407,12 +424,15 @@ void launch_add_eq_terms_f(ef* w, int lh, int ll, int npts, const uint32_t* hi, 
                            cudaStream_t s) {
   if (!npts) return;
   size_t n = size_t(1) << (lh + ll);
-  const int Kp = (npts + 31) / 32 * 32;
-  if (ll >= 4 && Kp <= AEQ_MAX_K) {
-    const uint32_t rows = (1u << ll) < AEQ_WARPS * 16 ? (1u << ll) : AEQ_WARPS * 16;
-    k_add_eq_terms_f_mma<<<(unsigned)(n / rows), AEQ_WARPS * 32, size_t(32) * Kp, s>>>(w, lh, ll, npts, Kp, hi, lo,
-                                                                                       coefs);
-    WL_LAUNCH_CHECK();
+  if (ll >= 4) {
+    uint32_t rows = std::min<uint32_t>(1u << ll, AEQ_ROWS);
+    while (rows > AEQ_MIN_ROWS && n / rows < 2 * 148) rows /= 2;
+    for (int t0 = 0; t0 < npts; t0 += AEQ_MAX_K) {
+      const int np = std::min(npts - t0, AEQ_MAX_K);
+      k_add_eq_terms_f_mma<<<(unsigned)(n / rows), AEQ_WARPS * 32, size_t(1024) * ((np + 7) / 8), s>>>(
+          w, lh, ll, np, rows, hi + (size_t(t0) << lh), lo + (size_t(t0) << ll), coefs + t0);
+      WL_LAUNCH_CHECK();
+    }
     return;
   }
   k_add_eq_terms_f<<<(unsigned)((n + 255) / 256), 256, sizeof(ef) * npts, s>>>(w, lh, ll, npts, hi, lo, coefs);
@@ -421,11 +441,14 @@ void launch_add_eq_terms_f(ef* w, int lh, int ll, int npts, const uint32_t* hi, 
 void launch_add_eq_terms_ef(ef* w, int lh, int ll, int npts, const ef* hi, const ef* lo, const ef* coefs,
                             cudaStream_t s) {
   if (!npts) return;
-  size_t n = size_t(1) << (lh + ll);
   if (npts > ADD_EQ_MAX) throw std::invalid_argument("add_eq_terms_ef: too many points");
   AddEqCoefs c{};
   for (int t = 0; t < npts; t++) c.c[t] = coefs[t];
-  k_add_eq_terms_ef<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(w, lh, ll, npts, hi, lo, c);
+  // whole blocks of one v_hi; four entries a thread once that leaves two blocks of every SM
+  const int threads = (1 << ll) < AEE_THREADS ? (1 << ll) : AEE_THREADS;
+  const int per = ll >= 10 && (size_t(1) << (lh + ll)) >= size_t(4) * 2 * 148 * AEE_THREADS ? 4 : 1;
+  k_add_eq_terms_ef<<<(unsigned)((size_t(1) << (lh + ll)) / (size_t(threads) * per)), threads, 0, s>>>(w, lh, ll, npts,
+                                                                                                     per, hi, lo, c);
   WL_LAUNCH_CHECK();
 }
 int whir_sc_blocks(size_t half) {

@@ -34,26 +34,6 @@ __device__ __forceinline__ void byte_transpose4(const uint4 q, uint32_t (&r)[4])
   r[3] = __byte_perm(p01h, p23h, 0x7632);
 }
 
-// Sum over the limb pairs of one accumulator position held by this lane: acc[a][b][q] for
-// the 16 pairs (a, b), combined by diagonal a + b = d (below 4 * 2^12 * 255^2 < 2^31),
-// weighted by 2^(8d) mod p and reduced once (the sum stays below 4 p^2). Montgomery inputs
-// give the Montgomery product.
-__device__ __forceinline__ uint32_t limb_recombine_lane(const int (&acc)[4][4][4], int q) {
-  constexpr uint32_t W8[7] = {uint32_t(kb::detail::cpow(2, 0)),  uint32_t(kb::detail::cpow(2, 8)),
-                              uint32_t(kb::detail::cpow(2, 16)), uint32_t(kb::detail::cpow(2, 24)),
-                              uint32_t(kb::detail::cpow(2, 32)), uint32_t(kb::detail::cpow(2, 40)),
-                              uint32_t(kb::detail::cpow(2, 48))};  // 2^(8d) mod p
-  uint64_t v = 0;
-#pragma unroll
-  for (int d = 0; d < 7; d++) {
-    uint32_t dd = 0;
-#pragma unroll
-    for (int a = 0; a < 4; a++)
-      if (d - a >= 0 && d - a < 4) dd += uint32_t(acc[a][d - a][q]);
-    v += kb::wmul(dd, W8[d]);
-  }
-  return kb::redc(v);
-}
 #endif
 
 }  // namespace wl

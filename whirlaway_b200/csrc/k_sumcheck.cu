@@ -1553,8 +1553,8 @@ __global__ void __launch_bounds__(FE_THREADS) k_abc_fold_eval(const ef* __restri
 }
 
 // ------------------------------------------------------------------ the last rounds of a phase
-// Once a phase's tables fit one block's shared memory, all rounds that remain run in one
-// launch: fold at the last challenge, the round's sums, the finish, and again, with the tables
+// Once a phase's tables fit the shared memory of one block or cluster, all rounds that remain run
+// in one launch: fold at the last challenge, the round's sums, the finish, and again, with the tables
 // folded in place and the phase state kept in shared memory between the rounds. As a launch of
 // its own such a round also cost a kernel boundary, a count of blocks through device memory and
 // the reload of all it needs: 26.6 us a round of the a*b - c sumcheck, 16.4 us here on average
@@ -1564,19 +1564,49 @@ __global__ void __launch_bounds__(FE_THREADS) k_abc_fold_eval(const ef* __restri
 // product the last rounds have one warp walk through a dozen products in turn, and their code, a
 // few hundred instructions each, does not stay in the instruction cache from round to round:
 // 20.3 us a round. For many points the other form needs half the instructions, so the tail
-// starts at TAIL_MAX_H = 256 points: from 512 on its first round would take longer (23 us a round
-// on average with 256 threads) than the several blocks of the separate launch.
+// holds at most 256 points in a block: from 512 on its first round would take longer (23 us a round
+// on average with 256 threads) than the several blocks of a separate launch.
 //
 // h is the number of points of the first round. With fold_in the tables come in at length 4h
 // (the eq table at 2h), to be folded at challenge *ch0; else at length 2h (h), to be evaluated as
 // they are.
+//
+// From more than TAIL_BLOCK_H = 256 up to TAIL_MAX_H points the launch is a cluster of
+// TAIL_CLUSTER blocks (CL): block c holds the entries x = c (mod TAIL_CLUSTER), so every fold stays
+// in its block; a round's partial sums go to block 0's shared memory, which finishes the round and
+// writes the challenge into the others'. The fold that leaves 2 TAIL_BLOCK_H entries writes them
+// to block 0, which goes on alone. Such a round as a launch of its own, on 2 to 8 blocks: 27 us
+// (product), 31 (WHIR), 28 (a*b - c); here 14 to 18. The line: with 4096 points (512 a block) the
+// round took 32 and 44 us, as eight lanes per product issue more than twice the instructions of one
+// thread per product. Loading the first fold's entries eight at a time changed nothing.
 constexpr int TAIL_THREADS = 512;
 constexpr int TAIL_GROUPS = TAIL_THREADS / 8;
+constexpr uint32_t TAIL_BLOCK_H = 256;
+constexpr uint32_t TAIL_CLUSTER = uint32_t(TAIL_MAX_H) / TAIL_BLOCK_H;
+static_assert(TAIL_CLUSTER <= 8, "portable cluster size");
+__shared__ ef tail_red[TAIL_CLUSTER][3];  // block 0: every block's sums of the round
+
+__device__ __forceinline__ uint32_t cl_rank() {
+  uint32_t r;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cl_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+// The address of block `rank`'s copy of a shared-memory object.
+template <class T>
+__device__ __forceinline__ T* cl_map(T* p, uint32_t rank) {
+  uint64_t r;
+  asm("mapa.u64 %0, %1, %2;" : "=l"(r) : "l"(p), "r"(rank));
+  return reinterpret_cast<T*>(r);
+}
 
 // Adds the groups' sums acc[z] (coordinate lane & 7) over the block into fin_sm.red and finishes
-// the round on warp 0. fin_sm.chal is valid for every thread on return.
+// the round on warp 0 (with cl, over the cluster's blocks and on block 0's). fin_sm.chal is valid
+// for every thread on return.
 template <int NS>
-__device__ __forceinline__ void tail_finish(int kind, const FinArgs& fin, const uint32_t* acc) {
+__device__ __forceinline__ void tail_finish(int kind, const FinArgs& fin, const uint32_t* acc, bool cl, uint32_t rank) {
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
   for (int z = 0; z < NS; z++) {
@@ -1591,59 +1621,85 @@ __device__ __forceinline__ void tail_finish(int kind, const FinArgs& fin, const 
       uint32_t v = 0;
 #pragma unroll
       for (int u = 0; u < TAIL_THREADS / 32; u++) v = kb::add(v, fin_sm.tmp[z * (TAIL_THREADS / 32) + u].c[k]);
+      (cl ? cl_map(&tail_red[rank][z], 0) : &fin_sm.red[z])->c[k] = v;
+    }
+    __syncwarp();
+  }
+  if (cl) cl_sync();
+  if (w == 0 && rank == 0) {
+    const int z = lane >> 3, k = lane & 7;
+    if (cl && z < NS) {
+      uint32_t v = 0;
+#pragma unroll
+      for (uint32_t c = 0; c < TAIL_CLUSTER; c++) v = kb::add(v, tail_red[c][z].c[k]);
       fin_sm.red[z].c[k] = v;
     }
     __syncwarp();
     fin_round(kind, fin);
+    __syncwarp();
+    if (cl)
+      for (uint32_t c = 1 + (lane >> 3); c < TAIL_CLUSTER; c += 4) cl_map(&fin_sm.chal, c)->c[k] = fin_sm.chal.c[k];
   }
-  __syncthreads();
+  if (cl) cl_sync();
+  else __syncthreads();
 }
-// Entries [0, n) of each of NT tables (length 2n at src + q sstride) folded at r (coordinate
-// lane & 7) into dst + q dstride; dst may be src, as an entry that is written is read only by the
-// group that writes it.
+// The entries of a table that a block holds: x_0, x_0 + m, ... of the whole table.
+struct TailMap {
+  uint32_t m = 1, x0 = 0;
+};
+// Entries [0, n) of each of NT tables (length 2n at src + q sstride, in the places of sm) folded at r
+// (coordinate lane & 7) into dst + q dstride (places of dm); dst may be src, as an entry that is
+// written is read only by the group that writes it.
 template <int NT>
-__device__ __forceinline__ void tail_fold(const ef* src, size_t sstride, ef* dst, size_t dstride, uint32_t n, uint32_t r) {
+__device__ __forceinline__ void tail_fold(const ef* src, size_t sstride, ef* dst, size_t dstride, uint32_t n, uint32_t r,
+                                          TailMap sm = {}, TailMap dm = {}) {
   const uint32_t g = threadIdx.x >> 3, k = threadIdx.x & 7;
 #pragma unroll 1
   for (uint32_t t0 = 0; t0 < NT * n; t0 += TAIL_GROUPS) {
     const uint32_t t = t0 + g;
     const bool on = t < NT * n;
     const uint32_t q = on ? t / n : 0, x = on ? t - q * n : 0;
-    const ef* s = src + q * sstride + x;
-    const uint32_t lo = s[0].c[k], hi = s[n].c[k];
+    const ef* s = src + q * sstride + x * sm.m + sm.x0;
+    const uint32_t lo = s[0].c[k], hi = s[n * sm.m].c[k];
     const uint32_t v = kb::add(lo, fin_mul(r, kb::sub(hi, lo)));
-    if (on) dst[q * dstride + x].c[k] = v;
+    if (on) dst[q * dstride + x * dm.m + dm.x0].c[k] = v;
   }
 }
 // The same entries copied.
 template <int NT>
-__device__ __forceinline__ void tail_copy(const ef* src, size_t sstride, ef* dst, size_t dstride, uint32_t n) {
+__device__ __forceinline__ void tail_copy(const ef* src, size_t sstride, ef* dst, size_t dstride, uint32_t n,
+                                          TailMap sm = {}) {
   for (uint32_t t = threadIdx.x; t < NT * n * 8; t += TAIL_THREADS) {
     const uint32_t e = t >> 3, q = e / n, x = e - q * n;
-    dst[q * dstride + x].c[t & 7] = src[q * sstride + x].c[t & 7];
+    dst[q * dstride + x].c[t & 7] = src[q * sstride + x * sm.m + sm.x0].c[t & 7];
   }
 }
 
 // Product (NS = 2) and WHIR (NS = 3) rounds; the tables folded at the last challenge go to oa, ob.
-template <int NS>
+template <int NS, bool CL>
 __global__ void __launch_bounds__(TAIL_THREADS, 1)
     k_pair_tail(const ef* __restrict__ a, const ef* __restrict__ b, uint32_t h, bool fold_in,
                 const ef* __restrict__ ch0, int rounds, ef* __restrict__ oa, ef* __restrict__ ob, const FinArgs fin) {
   extern __shared__ __align__(16) char tail_smem[];
-  ef* sa = reinterpret_cast<ef*>(tail_smem);
-  const uint32_t stride = 2 * h, g = threadIdx.x >> 3, k = threadIdx.x & 7;
-  ef* sb = sa + stride;
+  const uint32_t rank = CL ? cl_rank() : 0, g = threadIdx.x >> 3, k = threadIdx.x & 7;
+  bool cl = CL;
+  TailMap mp{CL ? TAIL_CLUSTER : 1u, rank};
+  if (CL) h /= TAIL_CLUSTER;  // this block's points
+  uint32_t stride = 2 * h;
+  ef *sa = reinterpret_cast<ef*>(tail_smem), *sb = sa + stride;
+  ef* const joined = sb + stride;  // CL, block 0: the joined tables, 2 TAIL_BLOCK_H entries each
   constexpr int kind = NS == 2 ? FIN_PROD : FIN_WHIR;
-  fin_load(kind, fin);
+  if (rank == 0) fin_load(kind, fin);
   if (fold_in) {
     const uint32_t r = ch0->c[k];
-    tail_fold<1>(a, 0, sa, 0, 2 * h, r);
-    tail_fold<1>(b, 0, sb, 0, 2 * h, r);
+    tail_fold<1>(a, 0, sa, 0, 2 * h, r, mp);
+    tail_fold<1>(b, 0, sb, 0, 2 * h, r, mp);
   } else {
-    tail_copy<1>(a, 0, sa, 0, 2 * h);
-    tail_copy<1>(b, 0, sb, 0, 2 * h);
+    tail_copy<1>(a, 0, sa, 0, 2 * h, mp);
+    tail_copy<1>(b, 0, sb, 0, 2 * h, mp);
   }
-  __syncthreads();
+  if (CL) cl_sync();  // every block runs: from here its shared memory may be written
+  else __syncthreads();
 #pragma unroll 1
   for (int t = 0;; t++, h >>= 1) {
     uint32_t acc[NS];
@@ -1659,40 +1715,61 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1)
       if (NS == 3) acc[1] = kb::add(acc[1], fin_mul(ah, bh));
       acc[NS - 1] = kb::add(acc[NS - 1], fin_mul(kb::sub(kb::dbl(ah), al), kb::sub(kb::dbl(bh), bl)));
     }
-    tail_finish<NS>(kind, fin, acc);
+    tail_finish<NS>(kind, fin, acc, cl, rank);
     if (t == rounds - 1) break;
-    tail_fold<2>(sa, stride, sa, stride, h, fin_sm.chal.c[k]);
-    __syncthreads();
+    if (CL && cl && h * TAIL_CLUSTER == 2 * TAIL_BLOCK_H) {
+      tail_fold<2>(sa, stride, cl_map(joined, 0), 2 * TAIL_BLOCK_H, h, fin_sm.chal.c[k], {}, mp);
+      cl_sync();
+      if (rank) return;
+      cl = false;
+      mp = {};
+      h *= TAIL_CLUSTER;
+      stride = 2 * TAIL_BLOCK_H;
+      sa = joined;
+      sb = joined + stride;
+    } else {
+      tail_fold<2>(sa, stride, sa, stride, h, fin_sm.chal.c[k]);
+      __syncthreads();
+    }
   }
-  tail_fold<1>(sa, 0, oa, 0, h, fin_sm.chal.c[k]);
-  tail_fold<1>(sb, 0, ob, 0, h, fin_sm.chal.c[k]);
-  if (threadIdx.x < 32) fin_commit(fin);
+  tail_fold<1>(sa, 0, oa, 0, h, fin_sm.chal.c[k], {}, mp);
+  tail_fold<1>(sb, 0, ob, 0, h, fin_sm.chal.c[k], {}, mp);
+  if (rank == 0 && threadIdx.x < 32) fin_commit(fin);
 }
 
 // The a*b - c zerocheck's rounds, to the end; the three columns folded at the last challenge go
 // to oc (column q at q times the last round's points).
+template <bool CL>
 __global__ void __launch_bounds__(TAIL_THREADS, 1)
     k_abc_tail(const ef* __restrict__ cols, const ef* __restrict__ eq_in, uint32_t h, bool fold_in,
                const ef* __restrict__ ch0, int rounds, ef* __restrict__ oc, const FinArgs fin) {
   extern __shared__ __align__(16) char tail_smem[];
-  ef* sc = reinterpret_cast<ef*>(tail_smem);
-  const uint32_t stride = 2 * h, g = threadIdx.x >> 3, k = threadIdx.x & 7;
-  ef* se = sc + 3 * stride;
-  fin_load(FIN_EQSC3, fin);
+  const uint32_t rank = CL ? cl_rank() : 0, g = threadIdx.x >> 3, k = threadIdx.x & 7;
+  bool cl = CL;
+  TailMap mp{CL ? TAIL_CLUSTER : 1u, rank};
+  const uint32_t whole = h;
+  if (CL) h /= TAIL_CLUSTER;  // this block's points
+  uint32_t stride = 2 * h;
+  ef *sc = reinterpret_cast<ef*>(tail_smem), *se = sc + 3 * stride;
+  ef* const joined = se + h;  // CL, block 0: the joined columns (2 TAIL_BLOCK_H entries each) and eq table
+  if (rank == 0) fin_load(FIN_EQSC3, fin);
   if (fold_in) {
-    tail_fold<3>(cols, 2 * stride, sc, stride, stride, ch0->c[k]);
-    for (uint32_t i = threadIdx.x; i < 8 * h; i += TAIL_THREADS)
-      se[i >> 3].c[k] = kb::add(eq_in[i >> 3].c[k], eq_in[(i >> 3) + h].c[k]);
+    tail_fold<3>(cols, size_t(4) * whole, sc, stride, stride, ch0->c[k], mp);
+    for (uint32_t i = threadIdx.x; i < 8 * h; i += TAIL_THREADS) {
+      const uint32_t x = (i >> 3) * mp.m + mp.x0;
+      se[i >> 3].c[k] = kb::add(eq_in[x].c[k], eq_in[x + whole].c[k]);
+    }
   } else {
-    tail_copy<3>(cols, stride, sc, stride, stride);
-    tail_copy<1>(eq_in, 0, se, 0, h);
+    tail_copy<3>(cols, size_t(2) * whole, sc, stride, stride, mp);
+    tail_copy<1>(eq_in, 0, se, 0, h, mp);
   }
-  __syncthreads();
+  if (CL) cl_sync();  // every block runs: from here its shared memory may be written
+  else __syncthreads();
   const int round0 = fin_sm.st.round;
 #pragma unroll 1
   for (int t = 0;; t++, h >>= 1) {
     // the eq challenge of a round after the first of the launch
-    if (t && threadIdx.x >= TAIL_THREADS - 16)
+    if (t && rank == 0 && threadIdx.x >= TAIL_THREADS - 16)
       (threadIdx.x < TAIL_THREADS - 8 ? fin_sm.r : fin_sm.rinv).c[k] =
           (threadIdx.x < TAIL_THREADS - 8 ? fin.req : fin.rinv)[round0 + t].c[k];
     uint32_t acc[2] = {0, 0};
@@ -1711,17 +1788,32 @@ __global__ void __launch_bounds__(TAIL_THREADS, 1)
       acc[0] = kb::add(acc[0], fin_mul(kb::sub(fin_mul(lo[0], lo[1]), lo[2]), e));
       acc[1] = kb::add(acc[1], fin_mul(kb::sub(fin_mul(d[0], d[1]), d[2]), e));
     }
-    tail_finish<2>(FIN_EQSC3, fin, acc);
+    tail_finish<2>(FIN_EQSC3, fin, acc, cl, rank);
     if (t == rounds - 1) break;
-    tail_fold<3>(sc, stride, sc, stride, h, fin_sm.chal.c[k]);
+    const bool join = CL && cl && h * TAIL_CLUSTER == 2 * TAIL_BLOCK_H;
+    ef* dst = join ? cl_map(joined, 0) : sc;
+    ef* edst = join ? dst + 6 * TAIL_BLOCK_H : se;
+    const TailMap dm = join ? mp : TailMap{};
+    tail_fold<3>(sc, stride, dst, join ? 2 * TAIL_BLOCK_H : stride, h, fin_sm.chal.c[k], {}, dm);
     // the eq table without its leading variable (in place: an entry written is read by the same
     // thread only)
     for (uint32_t i = threadIdx.x; i < 4 * h; i += TAIL_THREADS)
-      se[i >> 3].c[k] = kb::add(se[i >> 3].c[k], se[(i >> 3) + h / 2].c[k]);
-    __syncthreads();
+      edst[(i >> 3) * dm.m + dm.x0].c[k] = kb::add(se[i >> 3].c[k], se[(i >> 3) + h / 2].c[k]);
+    if (join) {
+      cl_sync();
+      if (rank) return;
+      cl = false;
+      mp = {};
+      h *= TAIL_CLUSTER;
+      stride = 2 * TAIL_BLOCK_H;
+      sc = joined;
+      se = joined + 6 * TAIL_BLOCK_H;
+    } else {
+      __syncthreads();
+    }
   }
-  tail_fold<3>(sc, stride, oc, h, h, fin_sm.chal.c[k]);
-  if (threadIdx.x < 32) fin_commit(fin);
+  tail_fold<3>(sc, stride, oc, size_t(h) * mp.m, h, fin_sm.chal.c[k], {}, mp);
+  if (rank == 0 && threadIdx.x < 32) fin_commit(fin);
 }
 
 // ------------------------------------------------------------------ a*b - c
@@ -2174,27 +2266,45 @@ void tail_smem_limit(K kernel, size_t bytes) {
 }
 }  // namespace
 
+// One block up to TAIL_BLOCK_H points, else a cluster (local tables and the joined ones); entries per
+// point: `per` in the round's tables.
+template <class K, class... A>
+static void launch_tail(K one, K cluster, size_t h, size_t per, cudaStream_t s, A... args) {
+  const bool cl = h > TAIL_BLOCK_H;
+  const size_t smem = sizeof(ef) * per * (cl ? h / TAIL_CLUSTER + TAIL_BLOCK_H : h);
+  tail_smem_limit(cl ? cluster : one, smem);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(cl ? TAIL_CLUSTER : 1);
+  cfg.blockDim = dim3(TAIL_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = TAIL_CLUSTER;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = cl ? 1 : 0;
+  WL_CUDA(cudaLaunchKernelEx(&cfg, cl ? cluster : one, args...));
+}
+static void tail_check(size_t h, int rounds) {
+  if (h < 1 || h > TAIL_MAX_H || (h & (h - 1)) || rounds < 1 || (h >> (rounds - 1)) < 1)
+    throw std::invalid_argument("sumcheck tail: size");
+}
 void launch_pair_tail(int nsums, const ef* a, const ef* b, size_t h, const ef* fold_ch, int rounds, ef* oa, ef* ob,
                       const FinArgs& fin, cudaStream_t s) {
-  if (h < 1 || h > TAIL_MAX_H || rounds < 1 || (h >> (rounds - 1)) < 1) throw std::invalid_argument("sumcheck tail: size");
-  const size_t smem = sizeof(ef) * 4 * h;
-  if (nsums == 2) {
-    tail_smem_limit(k_pair_tail<2>, smem);
-    k_pair_tail<2><<<1, TAIL_THREADS, smem, s>>>(a, b, uint32_t(h), fold_ch != nullptr, fold_ch, rounds, oa, ob, fin);
-  } else {
-    tail_smem_limit(k_pair_tail<3>, smem);
-    k_pair_tail<3><<<1, TAIL_THREADS, smem, s>>>(a, b, uint32_t(h), fold_ch != nullptr, fold_ch, rounds, oa, ob, fin);
-  }
-  WL_LAUNCH_CHECK();
+  tail_check(h, rounds);
+  if (nsums == 2)
+    launch_tail(k_pair_tail<2, false>, k_pair_tail<2, true>, h, 4, s, a, b, uint32_t(h), fold_ch != nullptr, fold_ch,
+                rounds, oa, ob, fin);
+  else
+    launch_tail(k_pair_tail<3, false>, k_pair_tail<3, true>, h, 4, s, a, b, uint32_t(h), fold_ch != nullptr, fold_ch,
+                rounds, oa, ob, fin);
 }
-
-void launch_abc_tail(const ef* cols, const ef* eq, size_t h, const ef* fold_ch, int rounds, ef* oc, const FinArgs& fin,
-                     cudaStream_t s) {
-  if (h < 1 || h > TAIL_MAX_H || rounds < 1 || (h >> (rounds - 1)) < 1) throw std::invalid_argument("sumcheck tail: size");
-  const size_t smem = sizeof(ef) * 7 * h;
-  tail_smem_limit(k_abc_tail, smem);
-  k_abc_tail<<<1, TAIL_THREADS, smem, s>>>(cols, eq, uint32_t(h), fold_ch != nullptr, fold_ch, rounds, oc, fin);
-  WL_LAUNCH_CHECK();
+void launch_abc_tail(const ef* cols, const ef* eq_in, size_t h, const ef* fold_ch, int rounds, ef* oc,
+                     const FinArgs& fin, cudaStream_t s) {
+  tail_check(h, rounds);
+  launch_tail(k_abc_tail<false>, k_abc_tail<true>, h, 7, s, cols, eq_in, uint32_t(h), fold_ch != nullptr, fold_ch, rounds,
+              oc, fin);
 }
 
 void launch_abc_fold_eval(const ef* cols, const ef* r_dev, const ef* eq_prev, ef* nc, ef* eq_new, size_t h, ef* partial,

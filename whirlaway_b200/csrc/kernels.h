@@ -184,12 +184,12 @@ void launch_pair_fold_eval(int nsums, const ef* a, const ef* b, const ef* r_dev,
 void launch_abc_fold_eval(const ef* cols, const ef* r_dev, const ef* eq_prev, ef* nc, ef* eq_new, size_t h, ef* partial,
                           const FinArgs* fin, cudaStream_t s);
 
-// The last `rounds` rounds of a phase in one launch of one block (k_pair_tail, k_abc_tail), the
-// first over h <= TAIL_MAX_H points: with fold_ch the tables have 4h entries (eq: 2h), folded
+// The last `rounds` rounds of a phase in one launch of one block or cluster (k_pair_tail, k_abc_tail), the
+// first over h <= TAIL_MAX_H points (a power of two): with fold_ch the tables have 4h entries (eq: 2h), folded
 // first at that challenge; without, 2h (eq: h), evaluated as they are. Each round is finished as
 // by launch_pair_fold_eval / launch_abc_fold_eval with fin; the tables folded at the last
 // challenge, (h >> (rounds - 1)) entries each, go to oa and ob (oc: three columns).
-constexpr size_t TAIL_MAX_H = 256;
+constexpr size_t TAIL_MAX_H = 2048;
 void launch_pair_tail(int nsums, const ef* a, const ef* b, size_t h, const ef* fold_ch, int rounds, ef* oa, ef* ob,
                       const FinArgs& fin, cudaStream_t s);
 void launch_abc_tail(const ef* cols, const ef* eq, size_t h, const ef* fold_ch, int rounds, ef* oc, const FinArgs& fin,

@@ -801,7 +801,7 @@ void whir_sumcheck_dev(Context& ctx, Transcript& ts, DBuf& g, DBuf& w, int& m, e
     // round 0 evaluates the tables as they are (the finish its own kernel); round t >= 1 folds
     // at challenge t - 1, evaluates and finishes in one kernel; the last challenge's fold
     // closes the block
-    // (tables that fit one block run all their rounds in one launch, the last fold included)
+    // (tables that fit one cluster run all their rounds in one launch, the last fold included)
     bool folded = false;
     for (int t = 0; t < rounds && !folded; t++) {
       const size_t half = size_t(1) << (m - 1 - t);
@@ -1654,7 +1654,7 @@ std::vector<uint32_t> prove_abc(Context& ctx, const kb::P16Consts& p16, int n, i
     int tail = 0;  // rounds of the last launch
     // round 1 makes the round-0 fold and evaluates it; round r >= 2 folds the columns (and sums the
     // eq table's leading variable out) at challenge r - 1 and evaluates in one pass; the last
-    // launch runs all rounds that fit one block and leaves the three final values
+    // launch runs all rounds that fit one cluster and leaves the three final values
     for (int round = 1; round <= n - k; round++) {
       const int m = n - k - round + 1;
       const size_t half = size_t(1) << (m - 1);

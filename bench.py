@@ -35,9 +35,11 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 METRIC = "Poseidon2 perms proven/sec on 1 B200 (batched vs plain); p50/p99 proof latency"
-P24_MODMUL = 8 * 24 * 2 + 23 * (2 + 24)   # Montgomery products per Poseidon2-24 permutation
-P16_MODMUL = 8 * 16 * 2 + 20 * (2 + 16)
-ZC0_MODMUL_PER_POINT = 165 * 16 + 148 * 8 + 8 * 16 * 2 + 20 * (2 + 16)  # extension + batching + AIR
+# field products on the CUDA cores: the S-boxes (the partial rounds' linear layers and, in the
+# zerocheck's round 0, the extension and the weights run on the tensor cores)
+P24_MODMUL = 8 * 24 * 2 + 23 * 2
+P16_MODMUL = 8 * 16 * 2 + 20 * 2
+ZC0_MODMUL_PER_POINT = 148 * 2
 
 
 def parse_args():
@@ -314,7 +316,7 @@ def roofline(profile, breakdown, log_n, peaks, hbm_peak_gbs, steps, hbm_source):
         traffic = (rows[0] * (88 * 4 + LEAF_EXTRA_DRAM_BYTES)
                    + sum(r * (128 * 4 + LEAF_EXTRA_DRAM_BYTES) for r in rows[1:])) * steps / max(launches, 1)
         out.update({"bound": "int", "achieved": achieved / 1e12, "peak": modmul_peak / 1e12,
-                    "unit": "T field multiplications/s (982 per Poseidon2-24, the textbook count)",
+                    "unit": "T S-box products/s (430 per Poseidon2-24; the partial rounds' linear layers run on the tensor cores)",
                     "frac": achieved / modmul_peak, "traffic": traffic,
                     "traffic_source": "ncu capture of the leaf kernel at 2^17 rows, scaled by rows",
                     "peak_source": ("hardware: 32-bit multiplies measured in this run by dependency-free mul.lo / "
@@ -323,8 +325,8 @@ def roofline(profile, breakdown, log_n, peaks, hbm_peak_gbs, steps, hbm_source):
                     "same_code_probe_view": {"achieved": perms / (ms * 1e-3) / 1e9,
                                              "peak": peaks["p24_perms_per_s"] / 1e9, "unit": "G Poseidon2-24 perms/s",
                                              "frac": perms / (ms * 1e-3) / peaks["p24_perms_per_s"],
-                                             "note": "against back-to-back permutations of the same code from "
-                                                     "registers: the cost of memory and orchestration only"},
+                                             "note": "against back-to-back permutations of the one-thread form "
+                                                     "from registers (no tensor cores)"},
                     "hbm": {"achieved": byts / (ms * 1e-3) / 1e9, "peak": hbm_peak_gbs, "unit": "GB/s",
                             "frac": byts / (ms * 1e-3) / 1e9 / hbm_peak_gbs,
                             "peak_source": hbm_source}})

@@ -224,9 +224,9 @@ wl_status wl_sumcheck_abc_verify(const uint32_t* p16_constants, int32_t log_n, i
  * unchanged; the proof (host buffer, its exact length is returned with WL_E_BUFFER_TOO_SMALL
  * when short) equals wl_sumcheck_abc_prove_device's. `stream` is a cudaStream_t (NULL: the
  * default stream). All calls share the scratch array: calls that overlap on the GPU race and
- * must be serialised. The call copies between host and device and waits for its stream
- * between rounds, so it must not be called from a stream callback or host function (where
- * CUDA calls are not permitted) and rejects a stream under graph capture (WL_E_INVALID_ARG).
+ * must be serialised. The call copies between host and device and waits for its stream (after
+ * round 0 and for the later rounds' results), so it must not be called from a stream callback or
+ * host function (where CUDA calls are not permitted) and rejects a stream under graph capture (WL_E_INVALID_ARG).
  * The first call on a device looks up the array's address (a failed lookup is retried by the
  * next call). */
 wl_status wl_sumcheck_abc_prove_noalloc(const uint32_t* p16_constants, int32_t log_n, int32_t skips,

@@ -29,13 +29,22 @@ __device__ __forceinline__ size_t down_row(size_t i, size_t N) { return i == N -
 // consecutive entries: x = (block << nbits) + (a << nb) + b, eq = H * A[a] * B[b], where A and
 // B are tables over the block's two groups of low variables (<= 16 entries each, built in
 // shared memory) and H is the product over the block's high variables (a product tree).
+// The tree and the tables are a chain of a dozen products before the block's one product per
+// entry, so a large table's block writes 2^EQ_BIG_BITS entries: H joins a third table C of 16
+// entries, C x A is formed once (one product a thread), and each thread writes 16 entries. From
+// EQ_BIG_VARS variables on that leaves 128 blocks or more. 2^20 entries: 52 us with blocks of
+// 2^8, 31 here; the a*b - c sumcheck of 2^24 1324 to 1277 us.
 constexpr int EQ_MAX_VARS = 32;
 constexpr int EQ_BLK_BITS = 8;
+constexpr int EQ_BIG_BITS = 12, EQ_BIG_VARS = 19;
 constexpr int EQ_THREADS = 1 << EQ_BLK_BITS;
+__host__ __device__ inline int eq_block_bits(int nvars) {
+  return nvars >= EQ_BIG_VARS ? EQ_BIG_BITS : nvars < EQ_BLK_BITS ? nvars : EQ_BLK_BITS;
+}
 __device__ __forceinline__ void eq_table_block(const ef* __restrict__ pt, int nvars, size_t xhi, ef* __restrict__ out) {
-  __shared__ ef r1[EQ_MAX_VARS], r0[EQ_MAX_VARS], fac[EQ_MAX_VARS], A[16], B[16];
-  const int nbits = nvars < EQ_BLK_BITS ? nvars : EQ_BLK_BITS;
-  const int nhi = nvars - nbits, na = nbits / 2, nb = nbits - na;
+  __shared__ ef r1[EQ_MAX_VARS], r0[EQ_MAX_VARS], fac[EQ_MAX_VARS], A[16], B[16], C[16], CA[256];
+  const int nbits = eq_block_bits(nvars), low = nbits < EQ_BLK_BITS ? nbits : EQ_BLK_BITS, nc = nbits - low;
+  const int nhi = nvars - nbits, ia = nhi + nc, na = low / 2, nb = low - na;
   const int tid = threadIdx.x;
   for (int i = tid; i < nvars; i += blockDim.x) {
     const ef r = pt[i];
@@ -47,14 +56,20 @@ __device__ __forceinline__ void eq_table_block(const ef* __restrict__ pt, int nv
   if (tid >= 64 && tid - 64 < (1 << na)) {
     const int a = tid - 64;
     ef v = ef_one();
-    for (int i = 0; i < na; i++) v = ef_mul(v, ((a >> (na - 1 - i)) & 1) ? r1[nhi + i] : r0[nhi + i]);
+    for (int i = 0; i < na; i++) v = ef_mul(v, ((a >> (na - 1 - i)) & 1) ? r1[ia + i] : r0[ia + i]);
     A[a] = v;
   }
   if (tid >= 96 && tid - 96 < (1 << nb)) {
     const int b = tid - 96;
     ef v = ef_one();
-    for (int i = 0; i < nb; i++) v = ef_mul(v, ((b >> (nb - 1 - i)) & 1) ? r1[nhi + na + i] : r0[nhi + na + i]);
+    for (int i = 0; i < nb; i++) v = ef_mul(v, ((b >> (nb - 1 - i)) & 1) ? r1[ia + na + i] : r0[ia + na + i]);
     B[b] = v;
+  }
+  if (nc && tid >= 128 && tid - 128 < (1 << nc)) {
+    const int c = tid - 128;
+    ef v = ef_one();
+    for (int i = 0; i < nc; i++) v = ef_mul(v, ((c >> (nc - 1 - i)) & 1) ? r1[nhi + i] : r0[nhi + i]);
+    C[c] = v;
   }
   __syncthreads();
   for (int len = nhi; len > 1;) {
@@ -62,6 +77,16 @@ __device__ __forceinline__ void eq_table_block(const ef* __restrict__ pt, int nv
     if (tid < len - m) fac[tid] = ef_mul(fac[tid], fac[tid + m]);
     __syncthreads();
     len = m;
+  }
+  if (nc) {  // 12 bits: four each in C, A and B
+    if (tid < 16) C[tid] = ef_mul(fac[0], C[tid]);
+    __syncthreads();
+    CA[tid] = ef_mul(C[tid >> 4], A[tid & 15]);
+    __syncthreads();
+    const ef b = B[tid & 15];
+#pragma unroll 1
+    for (int q = 0; q < 16; q++) out[(xhi << nbits) + q * 256 + tid] = ef_mul(CA[q * 16 + (tid >> 4)], b);
+    return;
   }
   // the block's factor joins A first: one product per entry
   if (nhi) {
@@ -1998,8 +2023,7 @@ __global__ void k_abc_eval_ef(const ef* __restrict__ cols, int m, const ef* __re
 // ------------------------------------------------------------------ launchers
 void launch_eq_table(const ef* point, int nvars, ef* out, cudaStream_t s) {
   if (nvars > EQ_MAX_VARS) throw std::invalid_argument("eq table: too many variables");
-  const int nbits = nvars < EQ_BLK_BITS ? nvars : EQ_BLK_BITS;
-  k_eq_table<<<(unsigned)(size_t(1) << (nvars - nbits)), EQ_THREADS, 0, s>>>(point, nvars, out);
+  k_eq_table<<<(unsigned)(size_t(1) << (nvars - eq_block_bits(nvars))), EQ_THREADS, 0, s>>>(point, nvars, out);
   WL_LAUNCH_CHECK();
 }
 bool EqTables::add(const ef* point, int nv, ef* table) {
@@ -2011,7 +2035,7 @@ bool EqTables::add(const ef* point, int nv, ef* table) {
   out[n] = table;
   for (int i = 0; i < nv; i++) pt[used + i] = point[i];
   if (!n) first[0] = 0;
-  first[n + 1] = first[n] + (1 << (nv < EQ_BLK_BITS ? 0 : nv - EQ_BLK_BITS));
+  first[n + 1] = first[n] + (1 << (nv - eq_block_bits(nv)));
   n++;
   return true;
 }

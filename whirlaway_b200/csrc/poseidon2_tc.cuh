@@ -33,8 +33,8 @@
 // That is 4 fp64 instructions and 4 integer multiplies per S-box.
 //
 // Measured (33.5M width-24 permutations, the leaves of 2^22 rows): 6.8 ms against 10.3 ms for
-// one thread per permutation with the internal layers word by word (p2_permute_fd): 4,600
-// instead of 8,960 instructions a permutation. What bounds it is register bandwidth: an S-box
+// one thread per permutation with the internal layers word by word (p2_permute_fd): 4,870 instead
+// of 8,960 instructions a permutation, the leaf's own work included. What bounds it is register bandwidth: an S-box
 // reads 22 32-bit operands, the fp64 pipe's pairs among them, and takes 14-15 clocks a warp and
 // scheduler where its pipes (fp64 and integer multiply, 8 clocks each) would allow 9 to 10.
 // Without the groups of 8 rounds: 7.3 ms; with mma.sync in place of tcgen05.mma: 9.5 ms, since

@@ -1859,7 +1859,6 @@ __device__ __forceinline__ uint32_t abc_in(uint32_t x) {
 }
 constexpr int ABC_X = 32;
 constexpr int ABC0_THREADS = 256;
-constexpr int ABC0_MAX_Z = 7;  // 2 (2^k - 1) - 2^k + 1 points for k <= 3
 template <int K>
 __global__ void __launch_bounds__(ABC0_THREADS, 2) k_abc0_eval(const uint32_t* __restrict__ a,
                                                            const uint32_t* __restrict__ b,

@@ -367,7 +367,7 @@ __global__ void __launch_bounds__(kb::TC_ROWS, 4)
   kb::P2TcShared<24>& sh = *reinterpret_cast<kb::P2TcShared<24>*>(leaf_smem);
   kb::p2_tc_begin<24>(sh);
   const size_t rows = size_t(1) << T;
-  uint32_t parity = 0;
+  kb::TcPhase ph;
 #pragma unroll 1
   for (int i = 0; i < tiles; i++) {
     const size_t t = (size_t(blockIdx.x) * tiles + i) * kb::TC_ROWS + threadIdx.x;
@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(kb::TC_ROWS, 4)
 #pragma unroll 1
     for (int ch = 0; ch < 8; ch++) {
       leaf_rate(lde, T, row, n_cols, log_elem, ch, st);
-      kb::p2_permute_tc<24>(st, c, sh, parity, ch == 7, o);
+      kb::p2_permute_tc<24>(st, c, sh, ph, ch == 7, o);
 #pragma unroll
       for (int j = 0; j < 8; j++) st[16 + j] = kb::umin(o[j], o[j] - kb::P);
     }
@@ -388,7 +388,7 @@ __global__ void __launch_bounds__(kb::TC_ROWS, 4)
       out[1] = make_uint4(st[20], st[21], st[22], st[23]);
     }
   }
-  kb::p2_tc_end<24>(sh, timeouts);
+  kb::p2_tc_end<24>(sh, ph, timeouts);
 }
 
 // One absorption (chunk ch) for every row, the capacity carried between launches in cap
@@ -402,7 +402,7 @@ __global__ void __launch_bounds__(kb::TC_ROWS, 4)
   kb::P2TcShared<24>& sh = *reinterpret_cast<kb::P2TcShared<24>*>(leaf_smem);
   kb::p2_tc_begin<24>(sh);
   const size_t rows = size_t(1) << T;
-  uint32_t parity = 0;
+  kb::TcPhase ph;
 #pragma unroll 1
   for (int i = 0; i < tiles; i++) {
     const size_t t = (size_t(blockIdx.x) * tiles + i) * kb::TC_ROWS + threadIdx.x;
@@ -417,7 +417,7 @@ __global__ void __launch_bounds__(kb::TC_ROWS, 4)
       st[16] = a.x, st[17] = a.y, st[18] = a.z, st[19] = a.w, st[20] = b.x, st[21] = b.y, st[22] = b.z, st[23] = b.w;
     }
     leaf_rate(lde, T, row, n_cols, log_elem, ch, st);
-    kb::p2_permute_tc<24>(st, c, sh, parity, ch == 7, o);
+    kb::p2_permute_tc<24>(st, c, sh, ph, ch == 7, o);
 #pragma unroll
     for (int j = 0; j < 8; j++) o[j] = kb::umin(o[j], o[j] - kb::P);
     if (t < rows) {
@@ -426,7 +426,7 @@ __global__ void __launch_bounds__(kb::TC_ROWS, 4)
       out[1] = make_uint4(o[4], o[5], o[6], o[7]);
     }
   }
-  kb::p2_tc_end<24>(sh, timeouts);
+  kb::p2_tc_end<24>(sh, ph, timeouts);
 }
 
 // `levels` levels of the tree above level l0 (level l0 + i has 2^(LL-l0-i) digests), 128
@@ -439,7 +439,7 @@ __global__ void __launch_bounds__(kb::TC_ROWS, 4)
   extern __shared__ __align__(16) char merkle_smem[];
   kb::P2TcShared<16>& sh = *reinterpret_cast<kb::P2TcShared<16>*>(merkle_smem);
   kb::p2_tc_begin<16>(sh);
-  uint32_t parity = 0;
+  kb::TcPhase ph;
 #pragma unroll 1
   for (int i = 1; i <= levels; i++) {
     const int l = l0 + i, tiles = 1 << (levels - i);
@@ -453,7 +453,7 @@ __global__ void __launch_bounds__(kb::TC_ROWS, 4)
         const uint4 u = src[q];
         st[4 * q] = u.x, st[4 * q + 1] = u.y, st[4 * q + 2] = u.z, st[4 * q + 3] = u.w;
       }
-      kb::p2_permute_tc<16>(st, c, sh, parity, true, o);
+      kb::p2_permute_tc<16>(st, c, sh, ph, true, o);
 #pragma unroll
       for (int j = 0; j < 8; j++) o[j] = kb::umin(o[j], o[j] - kb::P);
       uint4* out = reinterpret_cast<uint4*>(tree + (tree_off(LL, l) + m) * 8);
@@ -462,7 +462,7 @@ __global__ void __launch_bounds__(kb::TC_ROWS, 4)
     }
     __syncthreads();  // the level's digests before the next one reads them
   }
-  kb::p2_tc_end<16>(sh, timeouts);
+  kb::p2_tc_end<16>(sh, ph, timeouts);
 }
 
 // `levels` <= SUB_LEVELS levels above level l0, one warp per compression: each block turns
@@ -559,7 +559,7 @@ __global__ void __launch_bounds__(kb::TC_ROWS, 4)
   __shared__ uint32_t known;
   kb::p2_tc_begin<16>(sh);
   const uint32_t G = gridDim.x * kb::TC_ROWS, mask = (1u << bits) - 1;
-  uint32_t parity = 0;
+  kb::TcPhase ph;
 #pragma unroll 1
   for (uint32_t off = blockIdx.x * kb::TC_ROWS; off < count && base + off < kb::P; off += G) {
     if (threadIdx.x == 0) known = *reinterpret_cast<volatile const uint32_t*>(result);
@@ -575,11 +575,11 @@ __global__ void __launch_bounds__(kb::TC_ROWS, 4)
 #pragma unroll
     for (int i = 0; i < 8; i++)
       if (i == inlen) st[i] = w < kb::P ? w : 0u;
-    kb::p2_permute_tc<16>(st, c, sh, parity, true, o);  // its barriers order the next write of known
+    kb::p2_permute_tc<16>(st, c, sh, ph, true, o);  // its barriers order the next write of known
     const uint32_t s = kb::umin(o[7], o[7] - kb::P);
     if ((s & mask) == 0 && w < kb::P && off + threadIdx.x < count) atomicMin(result, w);
   }
-  kb::p2_tc_end<16>(sh, timeouts);
+  kb::p2_tc_end<16>(sh, ph, timeouts);
 }
 
 __global__ void k_to_mont(uint32_t* x, size_t n) {

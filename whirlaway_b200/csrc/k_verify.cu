@@ -31,7 +31,8 @@ __global__ void __launch_bounds__(kb::TC_ROWS, 4)
   if (threadIdx.x == 0) levels = 0;
   kb::p2_tc_begin<24>(sh.p24);
   atomicMax(&levels, op.ll);
-  uint32_t parity = 0, s[24], cur[8];
+  kb::TcPhase ph;
+  uint32_t s[24], cur[8];
 #pragma unroll
   for (int j = 0; j < 8; j++) cur[j] = 0;
 #pragma unroll 1
@@ -40,7 +41,7 @@ __global__ void __launch_bounds__(kb::TC_ROWS, 4)
     for (int j = 0; j < 16; j++) s[j] = words[op.row + 16 * ch + j];
 #pragma unroll
     for (int j = 0; j < 8; j++) s[16 + j] = cur[j];
-    kb::p2_permute_tc<24>(s, c24, sh.p24, parity, ch == 7, cur);
+    kb::p2_permute_tc<24>(s, c24, sh.p24, ph, ch == 7, cur);
 #pragma unroll
     for (int j = 0; j < 8; j++) cur[j] = kb::umin(cur[j], cur[j] - kb::P);
   }
@@ -58,11 +59,11 @@ __global__ void __launch_bounds__(kb::TC_ROWS, 4)
       t[j] = right ? b : cur[j];
       t[8 + j] = right ? cur[j] : b;
     }
-    kb::p2_permute_tc<16>(t, c16, sh.p16, parity, true, o);
+    kb::p2_permute_tc<16>(t, c16, sh.p16, ph, true, o);
 #pragma unroll
     for (int j = 0; j < 8; j++) cur[j] = on ? kb::umin(o[j], o[j] - kb::P) : cur[j];
   }
-  kb::p2_tc_end<16>(sh.p16, timeouts);
+  kb::p2_tc_end<16>(sh.p16, ph, timeouts);
   bool same = true;
 #pragma unroll
   for (int j = 0; j < 8; j++) same = same && cur[j] == words[op.root + j];

@@ -379,6 +379,20 @@ KB_HD uint32_t limb_word(uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uin
   return uint32_t(v >> 32) - umulhi(uint32_t(v) * PINV, P) + add;
 }
 
+// ---------------------------------------------------------------- waits that run out
+// A thread's account of its block's matrix products, each of which completes one phase of the
+// mbarrier: the parity of the phase to wait for, and whether a wait of this thread ran out. From
+// then on the parity stays at that phase, and as the block starts no product once a thread's wait
+// has run out (tc_product), that one is the last and the only one that may still be running.
+struct TcPhase {
+  uint32_t parity = 0;
+  bool expired = false;
+  KB_HD void waited(bool done) {
+    if (done) parity ^= 1;
+    else expired = true;
+  }
+};
+
 #ifdef __CUDACC__
 // ---------------------------------------------------------------- one tile of 128 permutations
 // A block is one tile: 128 threads, one permutation each, thread t on row t of the A operand and
@@ -393,7 +407,6 @@ struct P2TcShared {
   static constexpr int EA = 2 * (T::KS + T::KX) * TC_ROWS;  // 16-byte entries of A
   uint64_t bar;
   uint32_t tmem;
-  uint32_t dead;  // a bounded wait ran out
   uint4 b[T::E1 + T::E2 + T::E3];
   uint4 a[EA];
 };
@@ -426,22 +439,39 @@ __device__ __forceinline__ void p2_tc_begin(P2TcShared<W>& sh) {
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   if (threadIdx.x == 0) {
-    sh.dead = 0;
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(tc_smem(&sh.bar)) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   p2_tc_load(sh);
 }
-// Frees the accumulators; every thread has passed its last wait. Counts a wait that ran out.
+// Waits for the phase of the given parity; false when TC_WAIT_CLOCKS have passed without it.
+__device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity) {
+  uint32_t done = 0;
+  const long long t0 = clock64();
+  do {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+  } while (!done && clock64() - t0 < TC_WAIT_CLOCKS);
+  return done;
+}
+// Frees the accumulators. A product whose wait ran out may still read shared memory and write the
+// accumulators, so it is waited for once more (with the same limit) before they and the block go;
+// the block then counts as one that ran out.
 template <int W>
-__device__ __forceinline__ void p2_tc_end(P2TcShared<W>& sh, unsigned* timeouts) {
+__device__ __forceinline__ void p2_tc_end(P2TcShared<W>& sh, const TcPhase& ph, unsigned* timeouts) {
+  if (ph.expired) tc_wait(tc_smem(&sh.bar), ph.parity);
+  __syncwarp();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
+  const bool expired = __syncthreads_or(ph.expired);
   if (threadIdx.x < 32) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(sh.tmem), "r"(TC_COLS));
   }
-  if (threadIdx.x == 0 && sh.dead) atomicAdd(timeouts, 1u);
+  if (threadIdx.x == 0 && expired) atomicAdd(timeouts, 1u);
 }
 // Shared-memory matrix descriptor: K-major, no swizzle; lbo / sbo are the byte distances of core
 // matrices along k and along the rows.
@@ -450,14 +480,14 @@ __device__ __forceinline__ uint64_t tc_desc(uint32_t addr, uint32_t lbo, uint32_
 }
 // D = A B (ADD: D += A B) over KT k-steps: u8 x u8 -> s32, M = 128 rows, N columns from column
 // `col` of the accumulators; a and b are the operands' first entries (b has NB rows). The block
-// has written A; one thread issues the products, and every thread waits for them.
+// has written A; one thread issues the products, and every thread waits for them. Once a wait of any
+// thread has run out the block issues none: the results are void (p2_tc_end counts them).
 template <int W, int KT, int N, int NB, bool ADD>
-__device__ __forceinline__ void tc_product(P2TcShared<W>& sh, const uint4* a, const uint4* b, int col,
-                                           uint32_t& parity) {
+__device__ __forceinline__ void tc_product(P2TcShared<W>& sh, const uint4* a, const uint4* b, int col, TcPhase& ph) {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  if (threadIdx.x == 0) {
+  const bool stop = __syncthreads_or(ph.expired);
+  if (threadIdx.x == 0 && !stop) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     // instruction descriptor: D s32 (2 at bit 4), A and B unsigned 8 bit, both K-major
     constexpr uint32_t idesc = 2u << 4 | uint32_t(N / 8) << 17 | uint32_t(TC_ROWS / 16) << 24;
@@ -476,21 +506,8 @@ __device__ __forceinline__ void tc_product(P2TcShared<W>& sh, const uint4* a, co
                  : "memory");
   }
   __syncwarp();
-  uint32_t done = 0;
-  if (!*reinterpret_cast<volatile uint32_t*>(&sh.dead)) {
-    const long long t0 = clock64();
-    do {
-      asm volatile(
-          "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-          "selp.u32 %0, 1, 0, p;\n\t}"
-          : "=r"(done)
-          : "r"(tc_smem(&sh.bar)), "r"(parity)
-          : "memory");
-    } while (!done && clock64() - t0 < TC_WAIT_CLOCKS);
-    if (!done) *reinterpret_cast<volatile uint32_t*>(&sh.dead) = 1;
-  }
+  if (!stop) ph.waited(tc_wait(tc_smem(&sh.bar), ph.parity));
   __syncwarp();
-  parity ^= 1;
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 // 32 accumulator columns of this thread's row, from column `col`.
@@ -516,7 +533,7 @@ __device__ __forceinline__ void tc_store_words(uint4* a, const uint32_t* w) {
 // integer pipe, and when a group is done its x words are multiplied into the accumulators of
 // all later outputs, so that no sum has more than 8 terms.
 template <int W, int G>
-__device__ __forceinline__ void tc_chain(P2TcShared<W>& sh, const P2ConstsTc<W>& c, uint32_t& parity, int32_t* x) {
+__device__ __forceinline__ void tc_chain(P2TcShared<W>& sh, const P2ConstsTc<W>& c, TcPhase& ph, int32_t* x) {
   using T = P2TcTab<W>;
   constexpr int R0 = 8 * G, M = T::O1 - R0 < 8 ? T::O1 - R0 : 8;
   uint32_t r[32];
@@ -529,8 +546,8 @@ __device__ __forceinline__ void tc_chain(P2TcShared<W>& sh, const P2ConstsTc<W>&
   uint4* xa = sh.a + 2 * (T::KS + G) * TC_ROWS;
   tc_store_words<8>(xa, xs);
   if constexpr (R0 + 8 < T::O1) {
-    tc_product<W, 1, T::N1 - 4 * (R0 + 8), T::N3, true>(sh, xa, sh.b + T::E1 + T::E2, 4 * (R0 + 8), parity);
-    tc_chain<W, G + 1>(sh, c, parity, x);
+    tc_product<W, 1, T::N1 - 4 * (R0 + 8), T::N3, true>(sh, xa, sh.b + T::E1 + T::E2, 4 * (R0 + 8), ph);
+    tc_chain<W, G + 1>(sh, c, ph, x);
   }
 }
 
@@ -539,7 +556,7 @@ __device__ __forceinline__ void tc_chain(P2TcShared<W>& sh, const P2ConstsTc<W>&
 // (0, 2p); the other words are not formed.
 template <int W>
 __device__ __forceinline__ void p2_permute_tc(const uint32_t* s, const P2ConstsTc<W>& c, P2TcShared<W>& sh,
-                                              uint32_t& parity, bool first8, uint32_t* out) {
+                                              TcPhase& ph, bool first8, uint32_t* out) {
   using T = P2TcTab<W>;
   uint32_t w[W];
   double z[W];
@@ -557,10 +574,10 @@ __device__ __forceinline__ void p2_permute_tc(const uint32_t* s, const P2ConstsT
   for (int i = 0; i < W; i++) w[i] = fb_word<W>(z[i]);
   tc_store_words<W>(sh.a, w);
   x[0] = part_cube(umin(w[0], w[0] - P) + c.rc0);
-  tc_product<W, T::KS, T::N1, T::N1, false>(sh, sh.a, sh.b, 0, parity);
-  tc_chain<W, 0>(sh, c, parity, x);
+  tc_product<W, T::KS, T::N1, T::N1, false>(sh, sh.a, sh.b, 0, ph);
+  tc_chain<W, 0>(sh, c, ph, x);
   static_assert((T::O1 - 1) / 8 + 1 == T::KX, "the last group stores the last x words");
-  tc_product<W, T::KS + T::KX, T::N2, T::N2, false>(sh, sh.a, sh.b + T::E1, 0, parity);
+  tc_product<W, T::KS + T::KX, T::N2, T::N2, false>(sh, sh.a, sh.b + T::E1, 0, ph);
 #pragma unroll
   for (int g = 0; g < W / 8; g++) {
     uint32_t r[32];

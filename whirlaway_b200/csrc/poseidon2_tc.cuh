@@ -114,7 +114,7 @@ struct P2TcTab {
   static constexpr int N2 = 4 * W;
   static constexpr int N3 = N1 - 32;                     // x of 8 rounds into the outputs after them
   static constexpr int E1 = 2 * KS * N1, E2 = 2 * (KS + KX) * N2, E3 = 2 * N3;  // 16-byte entries
-  uint32_t w[(E1 + E2 + E3) * 4] = {};
+  alignas(16) uint32_t w[(E1 + E2 + E3) * 4] = {};  // read 16 bytes at a time
 };
 namespace p2lin {
 // Coefficient of word j in output o of stage 1 (y_1 .. y_(RP-1) from the state), stage 2 (the

@@ -495,6 +495,7 @@ wl_status wl_verify_batch_device(wl_ctx* ctx, const wl_air_settings* s, const ui
       }
     if (ops.empty()) return WL_OK;
     wl::Context& c = *ctx->c;
+    c.begin_waits();
     wl::DBuf words(sizeof(uint32_t) * base[n], c.stream), dops(sizeof(wl::OpeningCheck) * ops.size(), c.stream),
         dok(ops.size(), c.stream);
     for (int i = 0; i < n; i++)
@@ -514,7 +515,7 @@ wl_status wl_verify_batch_device(wl_ctx* ctx, const wl_air_settings* s, const ui
     WL_CUDA(cudaMemcpyAsync(ok.data(), dok.as<void>(), ok.size(), cudaMemcpyDeviceToHost, c.stream));
     WL_CUDA(cudaMemcpyAsync(&timeouts, c.pipe_timeouts, sizeof timeouts, cudaMemcpyDeviceToHost, c.stream));
     c.wait_stream();
-    if (timeouts) throw std::runtime_error("Merkle openings: a bounded wait ran out on the device");
+    c.end_waits(timeouts);
     // 3) a failed opening comes before whatever ended the replay: an opening error
     for (size_t j = 0; j < ok.size(); j++)
       if (!ok[j]) statuses[owner[j]] = WL_E_INVALID_PCS_OPENING;
@@ -733,6 +734,19 @@ wl_status wl_server_stats(wl_server* s, uint64_t* peak_bytes, int32_t* peak_runn
   if (peak_bytes) *peak_bytes = s->s->peak_in_use();
   if (peak_running) *peak_running = s->s->peak_running();
   return WL_OK;
+}
+
+// For tests only (not in the header): counts n bounded waits as run out on the context's device, as
+// a kernel would; with `unread`, as if the call they belonged to had ended in another error before
+// it read the count.
+wl_status wl_ctx_count_expired_waits(wl_ctx* ctx, uint32_t n, int32_t unread) {
+  if (!ctx) return WL_E_INVALID_ARG;
+  return guarded(ctx, [&] {
+    WL_CUDA(cudaMemcpyAsync(ctx->c->pipe_timeouts, &n, sizeof n, cudaMemcpyHostToDevice, ctx->c->stream));
+    WL_CUDA(cudaStreamSynchronize(ctx->c->stream));
+    ctx->c->waits_open = unread != 0;
+    return WL_OK;
+  });
 }
 
 void* wl_ctx_stream(wl_ctx* ctx) { return ctx ? (void*)ctx->c->stream : nullptr; }

@@ -553,7 +553,7 @@ struct GrindState {
 // p2_permute_fd in 2^17 threads, 21 us here; the grid is at most the blocks that are resident.
 __global__ void __launch_bounds__(kb::TC_ROWS, 4)
     k_grind(const __grid_constant__ kb::P2ConstsTc<16> c, const __grid_constant__ GrindState g, int inlen, int bits,
-            uint32_t base, uint32_t count, uint32_t* result, unsigned* __restrict__ timeouts) {
+            uint32_t base, uint32_t count, uint32_t* result) {
   extern __shared__ __align__(16) char grind_smem[];
   kb::P2TcShared<16>& sh = *reinterpret_cast<kb::P2TcShared<16>*>(grind_smem);
   __shared__ uint32_t known;
@@ -579,7 +579,7 @@ __global__ void __launch_bounds__(kb::TC_ROWS, 4)
     const uint32_t s = kb::umin(o[7], o[7] - kb::P);
     if ((s & mask) == 0 && w < kb::P && off + threadIdx.x < count) atomicMin(result, w);
   }
-  kb::p2_tc_end<16>(sh, ph, timeouts);
+  kb::p2_tc_end<16>(sh, ph, result + 1);
 }
 
 __global__ void k_to_mont(uint32_t* x, size_t n) {
@@ -817,8 +817,7 @@ void launch_gather_u32(const uint32_t* src, const uint64_t* idx, int width, int 
 }
 
 void launch_grind(const kb::P16Consts& p16, const uint32_t* state16, const uint32_t* inbuf, int inlen, int bits,
-                  uint32_t base, uint32_t count, uint32_t threads, uint32_t* result, unsigned* timeouts,
-                  cudaStream_t s) {
+                  uint32_t base, uint32_t count, uint32_t threads, uint32_t* result, cudaStream_t s) {
   if (bits < 1 || bits > 31 || inlen < 0 || inlen > 7) throw std::invalid_argument("grinding: bits 1..31, inlen 0..7");
   GrindState g;
   for (int i = 0; i < 16; i++) g.st[i] = kb::from_mont(state16[i]);
@@ -827,7 +826,7 @@ void launch_grind(const kb::P16Consts& p16, const uint32_t* state16, const uint3
   constexpr size_t smem = sizeof(kb::P2TcShared<16>);
   leaf_smem_limit(k_grind, smem);
   k_grind<<<std::min(blocks, 4 * uint32_t(ntt_sm_count())), kb::TC_ROWS, smem, s>>>(kb::p2_consts_tc(p16), g, inlen, bits,
-                                                                                    base, count, result, timeouts);
+                                                                                    base, count, result);
   WL_LAUNCH_CHECK();
 }
 

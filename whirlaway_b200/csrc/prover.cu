@@ -249,6 +249,17 @@ void Context::wait_stream() {
   host_wait_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - w0).count();
   if (hclk.on) hclk.last_wait_end = host_now_ms();
 }
+void Context::begin_waits() {
+  if (waits_open) WL_CUDA(cudaMemsetAsync(pipe_timeouts, 0, sizeof(unsigned), stream));  // the last call's count, unread
+  waits_open = true;
+}
+void Context::check_waits(unsigned ran_out) {
+  if (ran_out) throw std::runtime_error("a bounded wait ran out on the device (" + std::to_string(ran_out) + " blocks or threads)");
+}
+void Context::end_waits(unsigned ran_out) {
+  check_waits(ran_out);  // leaves waits_open set: the next call starts from zero
+  waits_open = false;
+}
 const ef* Context::reduce_wide(const ef* partial, int& nb, int k) {
   if (nb <= 2 * kWideBlocks || k > 32) return partial;
   {
@@ -514,7 +525,7 @@ struct DevPhase {
 // challenger replays observe(w) + sample_bits exactly as check_witness does.
 void grind(Context& ctx, Transcript& ts, const kb::P16Consts& p16, int bits) {
   if (bits <= 0) return;
-  DBuf res(sizeof(uint32_t), ctx.stream);
+  DBuf res(2 * sizeof(uint32_t), ctx.stream);
   // 2^(bits+3) candidates per batch: a witness is missed with probability e^-8 (one more
   // round trip then); the search stops soon after the first witness, so a larger batch costs
   // no device work
@@ -523,11 +534,13 @@ void grind(Context& ctx, Transcript& ts, const kb::P16Consts& p16, int bits) {
   // almost always; 2^(bits-2) threads take a few passes and stop about 2^bits candidates in
   const uint32_t threads = ctx.grind_lean ? 1u << std::max(8, bits - 2) : 1u << std::min(20, bits + 1);
   for (uint64_t base = 0; base < kb::P; base += batch) {
-    WL_CUDA(cudaMemsetAsync(res.as<void>(), 0xff, 4, ctx.stream));  // UINT32_MAX: none yet
+    WL_CUDA(cudaMemsetAsync(res.as<void>(), 0xff, 8, ctx.stream));  // UINT32_MAX: none yet, no wait ran out
     { ProfScope _ps(ctx, "grind"); launch_grind(p16, ts.ch.state, ts.ch.in, ts.ch.in_len, bits, (uint32_t)base, batch, threads, res.as<uint32_t>(),
-                 ctx.pipe_timeouts, ctx.stream); }
-    uint32_t r;
-    ctx.to_host(&r, res.as<uint32_t>(), 4);
+                 ctx.stream); }
+    uint32_t res_h[2];
+    ctx.to_host(res_h, res.as<uint32_t>(), 8);
+    if (res_h[1] != UINT32_MAX) throw std::runtime_error("grinding: a bounded wait ran out on the device");
+    const uint32_t r = res_h[0];
     if (r != UINT32_MAX) {
       uint32_t w = kb::to_mont(r);
       ts.ch.observe(w);
@@ -1060,6 +1073,7 @@ std::vector<uint32_t> prove_air(Context& ctx, const ProofJob& job, const uint32_
   const int m0 = n + LOGW;
   const WhirSchedule ws = WhirSchedule::build(m0, s);
   cudaStream_t st = ctx.stream;
+  ctx.begin_waits();
   Transcript ts(&job.p16);
   TranscriptLog tlog;
   if (ctx.dump_transcript) ts.log = &tlog;
@@ -1280,7 +1294,7 @@ std::vector<uint32_t> prove_air(Context& ctx, const ProofJob& job, const uint32_
       unsigned timeouts = 0;
       ctx.to_host_many({{inner_up.data(), up.as<ef>(), sizeof(ef) * W}, {inner_down.data(), down.as<ef>(), sizeof(ef) * W},
                         {&timeouts, ctx.pipe_timeouts, sizeof(unsigned)}});
-      if (timeouts) throw std::runtime_error("inner sums: a bounded pipeline wait ran out on the device");
+      ctx.check_waits(timeouts);
     }
     cols.reset();
   }
@@ -1493,7 +1507,7 @@ std::vector<uint32_t> prove_air(Context& ctx, const ProofJob& job, const uint32_
     unsigned timeouts = 0;
     ctx.to_host_many({{gf.data(), g.as<ef>(), sizeof(ef) << m}, {wf.data(), w.as<ef>(), sizeof(ef) << m},
                       {&timeouts, ctx.pipe_timeouts, sizeof(unsigned)}});
-    if (timeouts) throw std::runtime_error("Merkle leaves: a bounded wait ran out on the device");
+    ctx.end_waits(timeouts);  // the last commitment's tree is done; what follows are grindings and copies
     ts.add_ext(gf.data(), gf.size());
     const WhirRound& cl = ws.c[ws.num_rounds];
     grind(ctx, ts, job.p16, cl.pow_bits);

@@ -52,9 +52,15 @@ struct Context {
   ef* partials(size_t n);
   // Second-level partial sums (launch_reduce_wide's output), fixed capacity.
   static constexpr int kWideBlocks = 512;
-  // Device counter of bounded pipeline waits that ran out (kernels with mbarrier pipelines);
-  // zero on a healthy device, checked after each such kernel's results are read.
+  // Device counter of bounded waits that ran out in the Merkle hashes, the opening checks and the
+  // inner sums (grinding has its own, beside its result); zero on a healthy device. A call that
+  // uses it begins with begin_waits and passes what it reads, once those kernels are done, to
+  // end_waits (check_waits in between). A failed call leaves it zero for the next one.
   unsigned* pipe_timeouts = nullptr;
+  bool waits_open = false;  // a call has begun and not got to its end_waits
+  void begin_waits();
+  void check_waits(unsigned ran_out);  // throws when not zero
+  void end_waits(unsigned ran_out);
   ef* part2 = nullptr;
   // Reduces nb interleaved rows of k partial sums to a few rows in part2 when nb is large
   // (returns part2 and sets nb to its row count), else returns partial unchanged.

@@ -160,7 +160,10 @@ wl_status wl_prove_batch(wl_ctx* ctx, const wl_air_settings* settings, const uin
 wl_status wl_sumcheck_abc_prove(wl_ctx* ctx, const uint32_t* p16_constants, int32_t log_n, int32_t skips,
                                 const uint32_t* a, const uint32_t* b, const uint32_t* c, uint32_t* proof_out,
                                 size_t* proof_len, float* round_ms);
-/* Same with device-resident inputs (canonical u32 device pointers, left unchanged). */
+/* Same with device-resident inputs (canonical u32 device pointers, left unchanged). Columns in the
+ * memory of the context's device are read where they lie, at any time until the call returns;
+ * columns elsewhere (another device, mapped or managed memory, an address that is no multiple of
+ * 4) are copied first. */
 wl_status wl_sumcheck_abc_prove_device(wl_ctx* ctx, const uint32_t* p16_constants, int32_t log_n, int32_t skips,
                                        const uint32_t* a_dev, const uint32_t* b_dev, const uint32_t* c_dev,
                                        uint32_t* proof_out, size_t* proof_len, float* round_ms);

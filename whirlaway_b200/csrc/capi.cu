@@ -9,6 +9,7 @@
 #include <new>
 
 #include "../../include/whirlaway_b200.h"
+#include "columns.h"
 #include "prover.h"
 #include "server.h"
 #include "verifier.h"
@@ -336,6 +337,32 @@ wl_status wl_prove_batch(wl_ctx* ctx, const wl_air_settings* s, const uint32_t* 
   return WL_OK;
 }
 
+// What CUDA knows of an address (nothing, for one that it does not).
+static wl::ColumnMemory column_memory(const void* p) {
+  using AddressRange = int (*)(unsigned long long* base, size_t* size, unsigned long long p);  // cuMemGetAddressRange
+  static const AddressRange range = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+    if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &f, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess)
+      f = nullptr;
+    cudaGetLastError();
+    return reinterpret_cast<AddressRange>(f);
+  }();
+  wl::ColumnMemory m;
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return m;
+  }
+  m.device_memory = at.type == cudaMemoryTypeDevice;
+  m.device = at.device;
+  unsigned long long base = 0;
+  size_t size = 0;
+  if (m.device_memory && range && range(&base, &size, reinterpret_cast<uintptr_t>(p)) == 0) m.base = base, m.size = size;
+  return m;
+}
+
 static wl_status abc_common(wl_ctx* ctx, const uint32_t* p16c, int32_t log_n, int32_t skips, const uint32_t* a,
                             const uint32_t* b, const uint32_t* c, bool device, uint32_t* proof_out, size_t* proof_len,
                             float* round_ms) {
@@ -345,14 +372,16 @@ static wl_status abc_common(wl_ctx* ctx, const uint32_t* p16c, int32_t log_n, in
   return guarded(ctx, [&] {
     cudaStream_t st = ctx->c->stream;
     const size_t N = size_t(1) << log_n;
-    wl::DBuf d(device ? 0 : N * 12, st);
-    if (!device) {
-      uint32_t* da = d.as<uint32_t>();
-      WL_CUDA(cudaMemcpyAsync(da, a, N * 4, cudaMemcpyHostToDevice, st));
-      WL_CUDA(cudaMemcpyAsync(da + N, b, N * 4, cudaMemcpyHostToDevice, st));
-      WL_CUDA(cudaMemcpyAsync(da + 2 * N, c, N * 4, cudaMemcpyHostToDevice, st));
-      a = da, b = da + N, c = da + 2 * N;
-    }
+    wl::DBuf staged[3];
+    auto column = [&](const uint32_t*& p, wl::DBuf& d) {
+      if (device && wl::read_in_place(column_memory(p), ctx->c->device, reinterpret_cast<uintptr_t>(p), N * 4)) return;
+      d = wl::DBuf(N * 4, st);
+      WL_CUDA(cudaMemcpyAsync(d.as<void>(), p, N * 4, device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, st));
+      p = d.as<uint32_t>();
+    };
+    column(a, staged[0]);
+    column(b, staged[1]);
+    column(c, staged[2]);
     kb::P16Consts p16 = wl::perm_consts_from<16>(p16c);
     std::vector<float> ms;
     std::vector<uint32_t> pr = wl::prove_abc(*ctx->c, p16, log_n, skips, a, b, c, &ms);

@@ -4,7 +4,8 @@
 // coordinate k: a product a b in F[X]/(X^8 - 3) is eight multiply-adds of a_t (in every lane) by
 // the vector whose lane k is b_(k-t) or 3 b_(k+8-t), four at a time below 2^64, and one
 // reduction of both halves. 15-25 ns a product against 110-135 ns for the scalar form. Without
-// AVX-512 the scalar loops run. All values Montgomery form.
+// AVX-512, or built with WL_HOST_VEC_SCALAR (the tests of these loops), the scalar loops run. All
+// values Montgomery form.
 #include <immintrin.h>
 
 #include <cstdint>
@@ -21,6 +22,9 @@ namespace {
 using kb::ef;
 
 bool have_avx512() {
+#ifdef WL_HOST_VEC_SCALAR
+  return false;
+#endif
   static const bool ok = __builtin_cpu_supports("avx512f") && __builtin_cpu_supports("avx512bw") &&
                          __builtin_cpu_supports("avx512dq") && __builtin_cpu_supports("avx512vl");
   return ok;
@@ -149,6 +153,7 @@ WL_AVX512 ef dot_base_v(const ef* a, const uint32_t* f, size_t stride, size_t n)
 
 }  // namespace
 
+bool hv_vectorised() { return have_avx512(); }
 void hv_scale(const ef* a, size_t n, const ef& s, ef* out) {
   if (have_avx512()) return scale_v(a, n, s, out);
   const ef c = s;

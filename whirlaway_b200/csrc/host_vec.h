@@ -6,6 +6,7 @@
 #include "kb.cuh"
 
 namespace wl {
+bool hv_vectorised();  // which of the two runs
 void hv_scale(const kb::ef* a, size_t n, const kb::ef& s, kb::ef* out);  // out[i] = a[i] s (out may be a)
 void hv_mac(const kb::ef* a, size_t n, const kb::ef& s, kb::ef* out);    // out[i] += a[i] s
 void hv_mac_base(const kb::ef& a, const uint32_t* f, size_t n, kb::ef* out);  // out[i] += a f[i]

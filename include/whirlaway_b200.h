@@ -156,7 +156,10 @@ wl_status wl_prove_batch(wl_ctx* ctx, const wl_air_settings* settings, const uin
  * eq(r, x) * (a(x) * b(x) - c(x)) with a univariate skip of `skips` variables; r is sampled
  * from a fresh challenger on Poseidon16 (p16_constants: 148 u32), the three final folded
  * values are appended. a, b, c: host arrays of 2^log_n. round_ms (may be NULL) receives
- * log_n - skips + 1 per-round device times. */
+ * log_n - skips + 1 device times in milliseconds, whose sum is the device time of the rounds. They
+ * are not all one round's own. The fold at round 0's challenge counts to round 1 where that round
+ * has more than 2048 points (one launch makes both), else to round 0. The rounds of 2048 points and
+ * fewer, up to 12 entries at the end, are one launch and each receive an equal share of its time. */
 wl_status wl_sumcheck_abc_prove(wl_ctx* ctx, const uint32_t* p16_constants, int32_t log_n, int32_t skips,
                                 const uint32_t* a, const uint32_t* b, const uint32_t* c, uint32_t* proof_out,
                                 size_t* proof_len, float* round_ms);

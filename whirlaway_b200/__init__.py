@@ -396,7 +396,12 @@ def verify_program(hash_constants: np.ndarray, program, log_n: int, proof: np.nd
 
 
 def sumcheck_abc_prove(ctx: Context, p16_constants: np.ndarray, log_n: int, skips: int, a, b, c, device=False):
-    """Zerocheck of eq(r, x) * (a*b - c) with a univariate skip; returns (proof, per-round ms)."""
+    """Zerocheck of eq(r, x) * (a*b - c) with a univariate skip; returns (proof, per-round ms).
+
+    With device, a, b, c are CUDA tensors (read in place when they are in the memory of ctx's
+    device, until the call returns). The times add up to the rounds' device time: round 1 holds the
+    fold at round 0's challenge where it has more than 2048 points, and the rounds of 2048 points and
+    fewer are one launch whose time they share evenly."""
     lib = ctx._lib
     cap = 8 * (3 * ((1 << skips) - 1) + 1 + 4 * (log_n - skips) + 3) + 64
     out = np.zeros(cap, np.uint32)

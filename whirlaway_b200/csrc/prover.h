@@ -155,8 +155,10 @@ std::vector<uint32_t> prove_air(Context& ctx, const ProofJob& job, const uint32_
 // present. Same proof as uploading first.
 std::vector<uint32_t> prove_air_host(Context& ctx, const ProofJob& job, const uint32_t* wit_host, Timings* t);
 
-// Standalone zerocheck of eq(r, x) * (a * b - c) with a univariate skip; a, b, c device
-// Montgomery arrays of 2^log_n. Returns the proof (canonical) and per-round device times.
+// Standalone zerocheck of eq(r, x) * (a * b - c) with a univariate skip; a, b, c device arrays of
+// 2^log_n words (any 32-bit words, taken for their residues). Returns the proof (canonical) and
+// the rounds' device times: round 1's holds round 0's fold when the two are one launch, and the
+// rounds of the last launch share its time evenly.
 std::vector<uint32_t> prove_abc(Context& ctx, const kb::P16Consts& p16, int log_n, int skips, const uint32_t* a,
                                 const uint32_t* b, const uint32_t* c, std::vector<float>* round_ms);
 

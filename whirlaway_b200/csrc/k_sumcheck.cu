@@ -2097,7 +2097,6 @@ void launch_zc0_fold(const uint32_t* src, int log_n, int k, int cb, int ce, cons
                                                                                  out);
   WL_LAUNCH_CHECK();
 }
-bool zc_eval_is_dense(int m) { return m - 1 >= 10; }
 // x blocks of 32, and the split of the columns that gives at least ZCS_FILL blocks.
 constexpr int ZCS_FILL = 2 * 2 * 148;
 static dim3 zcs_grid(int m) {
@@ -2107,6 +2106,7 @@ static dim3 zcs_grid(int m) {
   const int per = (most + want - 1) / want;
   return dim3((unsigned)bx, (unsigned)((most + per - 1) / per));
 }
+bool zc_eval_is_dense(int m) { return zcs_grid(m).y < unsigned(AIR_NC / ZCS_COLS); }
 int zc_ef_blocks(int m) {
   const dim3 g = zcs_grid(m);
   return (int)(g.x * g.y);

@@ -121,7 +121,8 @@ constexpr int ZC_COLS = AIR_NC + 1;  // the carried columns: 148 cube inputs and
 void launch_zc0_fold(const uint32_t* src, int log_n, int k, int cb, int ce, const ef* sel, const ef* arow, ef* out,
                      cudaStream_t s);
 int zc_ef_blocks(int m);
-// Rounds of at least 2^10 points per z (timed in a class of their own).
+// Whether the round over m variables has enough x blocks that a warp of k_zc_sbox sums several
+// columns (timed in a class of its own), rather than one each.
 bool zc_eval_is_dense(int m);
 // cols: the ZC_COLS carried columns, the ones from ZC0_NQ on at cols2 when it is given.
 // Writes zc_ef_blocks(m) partial sums for each of z = 0, 2, 3.

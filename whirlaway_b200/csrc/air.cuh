@@ -64,56 +64,6 @@ __host__ __device__ __forceinline__ void air_trace_row(const AirConsts& K, const
   }
 }
 
-// Base-field constraint evaluation. `get(c)` returns column c of the point, `acc(h, i)`
-// receives constraint i's value h; `flush()` is called after every 4 constraints.
-template <class Get, class Acc, class Flush>
-__device__ __forceinline__ void air_eval_f(const AirConsts& K, Get&& get, Acc&& acc, Flush&& flush) {
-  uint32_t s[16];
-#pragma unroll
-  for (int i = 0; i < 16; i++) s[i] = get(1 + i);
-  kb::mds_light<16>(s);
-  int col = 17;
-#pragma unroll 1
-  for (int r = 0; r < 4; r++) {
-#pragma unroll
-    for (int i = 0; i < 16; i++) s[i] = kb::cube(kb::add(s[i], K.begin[r][i]));
-    kb::mds_light<16>(s);
-#pragma unroll
-    for (int i = 0; i < 16; i++) {
-      uint32_t p = get(col + i);
-      acc(kb::sub(s[i], p), r * 16 + i);
-      s[i] = p;
-      if ((i & 3) == 3) flush();
-    }
-    col += 16;
-  }
-#pragma unroll 1
-  for (int r4 = 0; r4 < 20; r4 += 4) {
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const uint32_t x0 = kb::cube(kb::add(s[0], K.partial[r4 + q]));
-      const uint32_t p = get(col++);
-      acc(kb::sub(x0, p), 64 + r4 + q);
-      kb::internal_layer_with0<16>(s, p);
-    }
-    flush();
-  }
-#pragma unroll 1
-  for (int r = 0; r < 4; r++) {
-#pragma unroll
-    for (int i = 0; i < 16; i++) s[i] = kb::cube(kb::add(s[i], K.end[r][i]));
-    kb::mds_light<16>(s);
-#pragma unroll
-    for (int i = 0; i < 16; i++) {
-      uint32_t p = get(col + i);
-      acc(kb::sub(s[i], p), 84 + r * 16 + i);
-      s[i] = p;
-      if ((i & 3) == 3) flush();
-    }
-    col += 16;
-  }
-}
-
 // Extension-field constraint evaluation: returns sum_i alpha^i * h_i (device kernels and the
 // host verifier).
 template <class Get>

@@ -166,7 +166,6 @@ inline uint32_t fm(int64_t x) {  // Montgomery form of a small signed integer
   if (v < 0) v += kb::P;
   return kb::to_mont(uint32_t(v));
 }
-inline ef ef_scale(const ef& a, uint32_t f) { return kb::ef_mul_f(a, f); }
 
 // Basis polynomials (coefficients, base field) of Lagrange interpolation on nodes 0..n-1.
 inline std::vector<std::vector<uint32_t>> lagrange_basis(int n) {

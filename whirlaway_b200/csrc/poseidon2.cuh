@@ -219,11 +219,6 @@ KB_HD void internal_layer_with0(uint32_t* s, uint32_t x0) {
   for (int i = 1; i < W; i++) s[i] = p2_diag_mul_add<W>(i, s[i], sum);
 }
 template <int W>
-KB_HD void internal_layer(uint32_t* s) {
-  internal_layer_with0<W>(s, s[0]);
-}
-
-template <int W>
 KB_HD void p2_permute(uint32_t* s, const P2Consts<W>& c) {
   mds_light<W>(s);
 #pragma unroll 1
@@ -243,10 +238,13 @@ KB_HD void p2_permute(uint32_t* s, const P2Consts<W>& c) {
 }
 
 // ---------------------------------------------------------------- canonical-domain S-box
-// The Merkle hashes run in the canonical (non-Montgomery) domain with an S-box whose two
-// products take their quotients by p from the fp64 pipe, which the integer kernels leave
-// idle, instead of two Montgomery reductions (four high-word integer products) on the
-// integer multiply pipe. For a product t = a b with |a|, |b| < 2^32 and |t| < 2^64, the
+// From here to p2_permute_fd: a permutation in the canonical (non-Montgomery) domain, the whole state
+// in one thread. No kernel of the library runs it; it is what the tests compare the tensor-core
+// permutation (poseidon2_tc.cuh) with and what the benchmark's probe times beside it.
+//
+// The S-box's two products take their quotients by p from the fp64 pipe, which the integer
+// kernels leave idle, instead of two Montgomery reductions (four high-word integer products) on
+// the integer multiply pipe. For a product t = a b with |a|, |b| < 2^32 and |t| < 2^64, the
 // fp64 product fl(a b) is within 2^11 of t and fl(1/p) within 2^-84 of 1/p, so
 // fl(a b) fl(1/p) is within 2^-19 of t / p; one fused multiply-add that also adds
 // 1.5 * 2^52 rounds it to an integer held in the low mantissa bits: q = floor(t / p) or one
@@ -339,15 +337,6 @@ KB_HD void internal_lazy_finish(uint32_t* s) {
     if (!p2_diag_neg<W>(i) && p2_diag_k<W>(i) >= 8) x = umin(x, x - P);
     s[i] = x;
   }
-}
-
-// Canonical round constants (the canonical-domain S-box and lane kernels).
-template <int W>
-inline P2Consts<W> p2_consts_canonical(const P2Consts<W>& m) {
-  P2Consts<W> c;
-  for (int i = 0; i < 4 * W; i++) c.ext_init[i] = from_mont(m.ext_init[i]), c.ext_term[i] = from_mont(m.ext_term[i]);
-  for (int i = 0; i < P2Consts<W>::RP; i++) c.internal[i] = from_mont(m.internal[i]);
-  return c;
 }
 
 // ---------------------------------------------------------------- fp64 full rounds

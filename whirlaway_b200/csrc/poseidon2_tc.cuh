@@ -226,8 +226,7 @@ constexpr uint32_t PART_H = 1080000000u, PART_K = P + PART_H;
 // a with M a = v, M = (J + I) (x) M4 the external matrix: M^-1 = (I - J / (W/4 + 1)) (x) M4^-1.
 template <int W>
 inline void external_inverse(const uint32_t* v, uint32_t* a) {
-  // M4^-1 by Cramer's rule on [[2,3,1,1],[1,2,3,1],[1,1,2,3],[3,1,1,2]] (determinant -35),
-  // adjugate rows below
+  // M4^-1 by Gauss-Jordan elimination mod p
   struct Inv {
     uint64_t m[4][4];
     uint64_t q;
@@ -236,7 +235,7 @@ inline void external_inverse(const uint32_t* v, uint32_t* a) {
       uint64_t w[4][8];
       for (int i = 0; i < 4; i++)
         for (int j = 0; j < 8; j++) w[i][j] = j < 4 ? uint64_t(M[i][j]) : uint64_t(j - 4 == i);
-      for (int c = 0; c < 4; c++) {  // Gauss-Jordan mod p
+      for (int c = 0; c < 4; c++) {
         int p = c;
         while (w[p][c] == 0) p++;
         for (int j = 0; j < 8; j++) std::swap(w[p][j], w[c][j]);

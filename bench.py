@@ -262,7 +262,7 @@ def int_peaks(device, consts):
     return {"mul_lo_per_s": lo.value, "mul_hi_per_s": hi.value, "modmul_per_s": a.value, "p24_perms_per_s": b.value}
 
 
-LEAF_EXTRA_DRAM_BYTES = 22.5  # measured DRAM bytes per leaf row beyond the row itself
+LEAF_EXTRA_DRAM_BYTES = 26.1  # measured DRAM bytes per leaf row beyond the row itself (k_leaf_hash)
 
 
 def whir_rows_hashed(log_n):
@@ -311,14 +311,19 @@ def roofline(profile, breakdown, log_n, peaks, hbm_peak_gbs, steps, hbm_source):
         byts = (rows[0] * (88 * 4 + 64) + sum(r * (128 * 4 + 64) for r in rows[1:])) * steps
         achieved = perms * P24_MODMUL / (ms * 1e-3)
         # DRAM traffic per Merkle build: ncu's dram__bytes_read.sum + dram__bytes_write.sum of the
-        # leaf kernel at 2^17 rows was 374.5 B per 88-column row (the row once plus 22.5 B of digest
-        # and tree traffic); scaled by rows, with 128-column rows for the later commitments.
+        # leaf kernel is 378.1 B per row on 2^19 leaf rows of 88 columns, 184 MB (the row once plus
+        # 26.1 B, most of them the digest); scaled by rows, with 128-column rows for the later
+        # commitments. The compressions' own traffic is not in it.
         traffic = (rows[0] * (88 * 4 + LEAF_EXTRA_DRAM_BYTES)
                    + sum(r * (128 * 4 + LEAF_EXTRA_DRAM_BYTES) for r in rows[1:])) * steps / max(launches, 1)
         out.update({"bound": "int", "achieved": achieved / 1e12, "peak": modmul_peak / 1e12,
                     "unit": "T S-box products/s (430 per Poseidon2-24; the partial rounds' linear layers run on the tensor cores)",
                     "frac": achieved / modmul_peak, "traffic": traffic,
-                    "traffic_source": "ncu capture of the leaf kernel at 2^17 rows, scaled by rows",
+                    "traffic_source": "ncu counters of k_leaf_hash on 2^19 leaf rows of 88 columns (378.1 B a row), "
+                                      "scaled by rows",
+                    "frac_note": "the S-boxes are four low-word multiplies and four fp64 operations each, so this is "
+                                 "work done against the integer pipe's rate, not the distance from what binds the "
+                                 "kernel: its S-boxes' register reads, 14 to 15 clocks a warp and scheduler",
                     "peak_source": ("hardware: 32-bit multiplies measured in this run by dependency-free mul.lo / "
                                     "mul.hi probes, two of each per Montgomery product"),
                     "p24_per_s": perms / (ms * 1e-3),

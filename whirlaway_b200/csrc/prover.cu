@@ -530,8 +530,9 @@ void grind(Context& ctx, Transcript& ts, const kb::P16Consts& p16, int bits) {
   // round trip then); the search stops soon after the first witness, so a larger batch costs
   // no device work
   const uint32_t batch = 1u << std::min(24, bits + 3);
-  // the first witness lies near 2^bits: 2^(bits+1) threads find it in one pass of the grid
-  // almost always; 2^(bits-2) threads take a few passes and stop about 2^bits candidates in
+  // the first witness lies near 2^bits: the more candidates at a time (2^(bits+1), or as many as
+  // the resident blocks take), the sooner the search ends; with 2^(bits-2) it takes a few passes
+  // more and stops sooner after the first witness
   const uint32_t threads = ctx.grind_lean ? 1u << std::max(8, bits - 2) : 1u << std::min(20, bits + 1);
   for (uint64_t base = 0; base < kb::P; base += batch) {
     WL_CUDA(cudaMemsetAsync(res.as<void>(), 0xff, 8, ctx.stream));  // UINT32_MAX: none yet, no wait ran out
